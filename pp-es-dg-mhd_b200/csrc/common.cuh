@@ -287,86 +287,70 @@ __device__ __forceinline__ double ddot3(double a1, double b1, double a2, double 
   return dfma(a3, b3, dfma(a2, b2, dmul(a1, b1)));
 }
 
-// Entropy-conservative two-point flux, x (DIR=0, DG_solver.f90:1570-1609) or y (DIR=1,
-// DG_solver.f90:1611-1650).  a, b = (rho, vx, vy, vz, bx, by, bz, beta).
+// Four times the entropy-conservative two-point flux along the first direction (ec_flux_x,
+// DG_solver.f90:1570-1609; the y flux :1611-1650 is the same with the two directions exchanged).
+// a, b = (rho, vn, vt, vz, bn, bt, bz, beta); a_bsq, b_bsq = |B|^2 of each.
 //
 // The reference forms rho_hat = rho_bar / ff(rho) and beta_hat = beta_bar / ff(beta) with
 // ff = log_avg_divisor (zeta = a/b, f = (zeta-1)/(zeta+1), the series when f^2 < 1.4e-4, else
-// 0.5 log(zeta)/f), then divides by beta_bar three times and by beta_hat once.  The same values
-// with fewer FP64 divisions, by algebra only:
+// 0.5 log(zeta)/f).  Here everything is formed from the sums S = a + b instead of the means, the
+// factors 1/2 and 1/4 of the means going into the caller's coefficient (hence four times the flux):
 //   f = (a-b)/(a+b)                                  (= (zeta-1)/(zeta+1))
 //   series:  rho_hat = rho_bar / (1 + u/3 + u^2/5 + u^3/7),  u = f^2, formed as rho_bar times the
 //            inverse series (inv_series_divisor)
 //   log:     rho_hat = rho_bar / (0.5 log(zeta)/f) = (a-b) / log(a/b)
-//   1/beta_hat = ff(beta) / beta_bar = ff(beta) * inv_bb,  inv_bb = 1/beta_bar
-// and every "/ beta_bar" becomes "* inv_bb"; 1/(rho_a+rho_b) and 1/(beta_a+beta_b) both come from
-// the one reciprocal 1/((rho_a+rho_b)(beta_a+beta_b)), and "/ (gamma-1)" is a product with
-// igm1 = 1/(gamma-1), formed once by the caller.  Results agree with the reference's
-// expression order to a few ulp; the series/log branch is decided on the same u (to an ulp).
+//   1/rho_s and 1/beta_s come from one reciprocal; igm1 = 1/(gamma-1) from the caller.
+// The energy flux is the reference's sum with its exactly cancelling parts taken out: with
+// f_m = v_bar f_0 - bn_bar B_bar + n p_tot, v_bar.f_m = f_0 |v_bar|^2 - bn_bar (v_bar.B_bar) +
+// vn_bar p_tot, whose second part cancels the last term (v_bar.B_bar) bn_bar, and vn_bar p_tot -
+// vn_bar b_sq_bar / 2 = vn_bar rho_bar / (2 beta_bar); |v_bar|^2 - v_sq_bar / 2 = va.vb / 2.  So
+//   f_7 = f_0 (ff(beta)/((gamma-1) beta_bar) + va.vb)/2 + vn_bar rho_bar/(2 beta_bar) + B_bar.f_B.
+// 62 FP64 operations and a reciprocal against 107 for the expressions as the reference writes them
+// (the kernel that calls this is bound by its FP64 chains).
 __device__ __forceinline__ double series_divisor(double u) {
   return dfma(u, dfma(u, dfma(u, 1.0 / 7.0, 1.0 / 5.0), 1.0 / 3.0), 1.0);
 }
-// 1 / series_divisor(u) by its own series, 1 - u/3 - 4u^2/45 - 44u^3/945 + 1147u^4/14175 (the
+// half of 1 / series_divisor(u) by its own series, 1 - u/3 - 4u^2/45 - 44u^3/945 + 1147u^4/14175 (the
 // inverse of the power series; the truncation error is below 3e-22 relative for u < 1.4e-4),
 // so that the logarithmic mean of the common smooth case takes no division
-__device__ __forceinline__ double inv_series_divisor(double u) {
-  return dfma(u, dfma(u, dfma(u, dfma(u, 1147.0 / 14175.0, -44.0 / 945.0), -4.0 / 45.0), -1.0 / 3.0), 1.0);
+__device__ __forceinline__ double half_inv_series_divisor(double u) {
+  return dfma(u, dfma(u, dfma(u, dfma(u, 1147.0 / 28350.0, -22.0 / 945.0), -2.0 / 45.0), -1.0 / 6.0), 0.5);
 }
 
-template <int DIR>
-__device__ __forceinline__ void ec_flux(const double* a, const double* b, double igm1, double* f) {
+__device__ __forceinline__ void ec_flux4(const double* a, const double* b, double a_bsq, double b_bsq, double igm1,
+                                         double* f) {
   const double rho_s = dadd(a[0], b[0]), beta_s = dadd(a[7], b[7]);
-  const double rho_bar = dmul(0.5, rho_s);
-  const double vx_bar = dmul(0.5, dadd(a[1], b[1]));
-  const double vy_bar = dmul(0.5, dadd(a[2], b[2]));
-  const double vz_bar = dmul(0.5, dadd(a[3], b[3]));
-  const double bx_bar = dmul(0.5, dadd(a[4], b[4]));
-  const double by_bar = dmul(0.5, dadd(a[5], b[5]));
-  const double bz_bar = dmul(0.5, dadd(a[6], b[6]));
-  const double v_sq_bar = dmul(0.5, dadd(dsq3(a[1], a[2], a[3]), dsq3(b[1], b[2], b[3])));
-  const double b_sq_bar = dmul(0.5, dadd(dsq3(a[4], a[5], a[6]), dsq3(b[4], b[5], b[6])));
-  const double bvx = dmul(0.5, dfma(b[7], b[1], dmul(a[7], a[1])));
-  const double bvy = dmul(0.5, dfma(b[7], b[2], dmul(a[7], a[2])));
-  const double bvz = dmul(0.5, dfma(b[7], b[3], dmul(a[7], a[3])));
   const double rho_d = dsub(a[0], b[0]), beta_d = dsub(a[7], b[7]);
-  // 1/rho_s and 1/beta_s from one reciprocal
   const double r_rb = 1.0 / dmul(rho_s, beta_s);
-  const double inv_bb = dmul(2.0, dmul(rho_s, r_rb));  // 1 / beta_bar
+  const double ib = dmul(rho_s, r_rb);  // 1 / beta_s
   const double fr = dmul(rho_d, dmul(beta_s, r_rb)), ur = dmul(fr, fr);
-  const double fb = dmul(beta_d, dmul(0.5, inv_bb)), ub = dmul(fb, fb);
+  const double fb = dmul(beta_d, ib), ub = dmul(fb, fb);
   // logarithmic mean of rho and divisor of that of beta: the series forms, replaced by the
   // logarithmic forms in the uncommon case
-  double rho_hat = dmul(rho_bar, inv_series_divisor(ur));
+  double rho_hat = dmul(rho_s, half_inv_series_divisor(ur));
   double ffb = series_divisor(ub);
   if (ur >= 1.4e-4 || ub >= 1.4e-4) {
     if (ur >= 1.4e-4) rho_hat = rho_d / log(a[0] / b[0]);
     if (ub >= 1.4e-4) ffb = dmul(0.5, log(a[7] / b[7])) / fb;
   }
-  const double ptot = dmul(0.5, dfma(rho_bar, inv_bb, b_sq_bar));
-  const double ecoef = dmul(0.5, dfma(dmul(ffb, inv_bb), igm1, -v_sq_bar));
-  const double vb = ddot3(vx_bar, bx_bar, vy_bar, by_bar, vz_bar, bz_bar);
-  const double bn = DIR == 0 ? bx_bar : by_bar;  // the field component normal to the flux direction
-  const double vn = DIR == 0 ? vx_bar : vy_bar;
-  f[0] = dmul(rho_hat, vn);
-  f[1] = dfma(vx_bar, f[0], -dmul(bn, bx_bar));
-  f[2] = dfma(vy_bar, f[0], -dmul(bn, by_bar));
-  f[3] = dfma(vz_bar, f[0], -dmul(bn, bz_bar));
-  if (DIR == 0) {
-    f[1] = dadd(f[1], ptot);
-    f[4] = 0.0;
-    f[5] = dmul(dfma(bvx, by_bar, -dmul(bvy, bx_bar)), inv_bb);
-    f[6] = dmul(dfma(bvx, bz_bar, -dmul(bvz, bx_bar)), inv_bb);
-  } else {
-    f[2] = dadd(f[2], ptot);
-    f[4] = dmul(dfma(bvy, bx_bar, -dmul(bvx, by_bar)), inv_bb);
-    f[5] = 0.0;
-    f[6] = dmul(dfma(bvy, bz_bar, -dmul(bvz, by_bar)), inv_bb);
-  }
-  // ecoef f0 + (v . f[1..3]) + (b . f[4..6]) - 0.5 vn |b|^2 + (v . b) bn
-  double e = dfma(ecoef, f[0], ddot3(vx_bar, f[1], vy_bar, f[2], vz_bar, f[3]));
-  e = dadd(e, dfma(bz_bar, f[6], dfma(by_bar, f[5], dmul(bx_bar, f[4]))));
-  e = dfma(dmul(-0.5, vn), b_sq_bar, e);
-  f[7] = dfma(vb, bn, e);
+  const double vn = dadd(a[1], b[1]), vt = dadd(a[2], b[2]), vz = dadd(a[3], b[3]);
+  const double bn = dadd(a[4], b[4]), bt = dadd(a[5], b[5]), bz = dadd(a[6], b[6]);
+  const double h = dmul(rho_hat, vn);  // 2 f_0
+  const double q = dmul(rho_s, ib);    // rho_bar / beta_bar
+  const double i2 = dadd(ib, ib);      // 1 / beta_bar
+  const double p4 = dfma(2.0, q, dadd(a_bsq, b_bsq));  // 4 p_tot
+  f[0] = dadd(h, h);
+  f[1] = dfma(vn, h, dfma(-bn, bn, p4));
+  f[2] = dfma(vt, h, -dmul(bn, bt));
+  f[3] = dfma(vz, h, -dmul(bn, bz));
+  f[4] = 0.0;
+  const double gn = dfma(b[7], b[1], dmul(a[7], a[1]));
+  const double gt = dfma(b[7], b[2], dmul(a[7], a[2]));
+  const double gz = dfma(b[7], b[3], dmul(a[7], a[3]));
+  f[5] = dmul(dfma(gn, bt, -dmul(gt, bn)), i2);
+  f[6] = dmul(dfma(gn, bz, -dmul(gz, bn)), i2);
+  const double x = dfma(dmul(ffb, i2), igm1, ddot3(a[1], b[1], a[2], b[2], a[3], b[3]));
+  f[7] = dfma(0.5, dfma(bz, f[6], dmul(bt, f[5])), dfma(vn, q, dmul(h, x)));
 }
 
 // ESPP_HLL_flux_x (DG_solver.f90:894-1071).  wl, wr: conserved states already rotated into the

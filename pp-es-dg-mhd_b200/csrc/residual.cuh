@@ -284,6 +284,7 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
   const int gbase = (grp < G ? grp : 0) * NN;  // lanes beyond the groups mirror group 0
   const int k = node % N, l = node / N;
   const double sxh = 2.0 / g.hx, syh = 2.0 / g.hy;
+  const double sxq = 0.5 * sxh, syq = 0.5 * syh;  // 2 (2/h) / 4: the pair fluxes come as four times the flux
   double w[8];
   {
     const double* cw = s_cons + (act ? el : 0) * ES + node;
@@ -293,10 +294,10 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
   // (all arithmetic of the tile is exactly rounded as written: dmul/dadd/dsub/dfma of common.cuh)
   const double ir = 1.0 / w[0];
   const double vx = dmul(ir, w[1]), vy = dmul(ir, w[2]), vz = dmul(ir, w[3]);
-  double pt, sgx, sgy, pp[8];  // pp: (rho, vx, vy, vz, Bx, By, Bz, beta), the EC flux's inputs
+  double pt, sgx, sgy, bsq, pp[8];  // pp: (rho, vx, vy, vz, Bx, By, Bz, beta), the EC flux's inputs
   {
     const double ek = dmul(dmul(0.5, ir), dsq3(w[1], w[2], w[3]));
-    const double bsq = dsq3(w[4], w[5], w[6]);
+    bsq = dsq3(w[4], w[5], w[6]);
     const double pf = fmax(dmul(dsub(gamma, 1.0), dsub(w[7], dfma(0.5, bsq, ek))), PP_EPS);
     pp[0] = w[0];
     pp[1] = vx;
@@ -363,12 +364,13 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
 #pragma unroll
     for (int v = 0; v < 8; ++v) acc[v] = __fma_rn(-divB, GP[v], __fma_rn(-cll, Gf[v], -__dmul_rn(ckk, F[v])));
   }
-  // This lane's flux with the node in lane `src` (x frame, or y through swap_xy); the result F is
-  // in the global frame.  Every lane of the warp calls it (the shuffles need the full warp).
+  // Four times this lane's flux with the node in lane `src` (x frame, or y through swap_xy); the
+  // result F is in the global frame.  Every lane of the warp calls it (the shuffles need the full warp).
   auto pair_flux = [&](int src, bool ydir, double* F) {
     double A[8], B[8], Fx[8];
 #pragma unroll
     for (int v = 0; v < 8; ++v) B[v] = __shfl_sync(FULL, pp[v], src);
+    const double bsq_src = dsq3(B[4], B[5], B[6]);
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
       const int sv = swap_xy_var(v);
@@ -376,7 +378,7 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
       const double b = ydir ? B[sv] : B[v];
       Fx[v] = b;  // reuse as the rotated partner
     }
-    ec_flux<0>(A, Fx, igm1, B);
+    ec_flux4(A, Fx, bsq, bsq_src, igm1, B);
 #pragma unroll
     for (int v = 0; v < 8; ++v) F[v] = ydir ? B[swap_xy_var(v)] : B[v];
   };
@@ -384,9 +386,9 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
     const bool xb = (k == l);
     double F[8];
     pair_flux(xb ? lane_of(1 - k, l) : lane_of(k, 1 - l), !xb, F);
-    const double c1 = xb ? 2.0 * sxh * Dm(k + N * (1 - k)) : 2.0 * syh * Dm(l + N * (1 - l));
+    const double c1 = xb ? sxq * Dm(k + N * (1 - k)) : syq * Dm(l + N * (1 - l));
     const int src2 = xb ? lane_of(k, 1 - l) : lane_of(1 - k, l);
-    const double c2 = xb ? 2.0 * syh * Dm(l + N * (1 - l)) : 2.0 * sxh * Dm(k + N * (1 - k));
+    const double c2 = xb ? syq * Dm(l + N * (1 - l)) : sxq * Dm(k + N * (1 - k));
     // the reference's order: x partner below, y partner below, x above, y above
     const int rx = (1 - k) < k ? 0 : 2, ry = (1 - l) < l ? 1 : 3;
     const bool own_first = xb ? rx < ry : ry < rx;
@@ -402,7 +404,7 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
     for (int dir = 0; dir < 2; ++dir) {
       const int a = dir == 0 ? k : l;
       const int an = (a + 1) % N, ap = (a + N - 1) % N;
-      const double h2 = dir == 0 ? 2.0 * sxh : 2.0 * syh;
+      const double h2 = dir == 0 ? sxq : syq;
       double F[8];
       pair_flux(dir == 0 ? lane_of(an, l) : lane_of(k, an), dir == 1, F);
       const double c1 = h2 * Dm(a + N * an), c2 = h2 * Dm(a + N * ap);
@@ -420,7 +422,7 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
       const bool xb = ((k >> 1) ^ (l >> 1)) == 0;
       double F[8];
       pair_flux(xb ? lane_of(k ^ 2, l) : lane_of(k, l ^ 2), !xb, F);
-      const double cx = 2.0 * sxh * Dm(k + N * (k ^ 2)), cy = 2.0 * syh * Dm(l + N * (l ^ 2));
+      const double cx = sxq * Dm(k + N * (k ^ 2)), cy = syq * Dm(l + N * (l ^ 2));
       const int src2 = xb ? lane_of(k, l ^ 2) : lane_of(k ^ 2, l);
       // the reference's order: x partner below, y partner below, x above, y above
       const int rx = (k ^ 2) < k ? 0 : 2, ry = (l ^ 2) < l ? 1 : 3;
