@@ -305,7 +305,9 @@ __device__ __forceinline__ double ddot3(double a1, double b1, double a2, double 
 // vn_bar p_tot, whose second part cancels the last term (v_bar.B_bar) bn_bar, and vn_bar p_tot -
 // vn_bar b_sq_bar / 2 = vn_bar rho_bar / (2 beta_bar); |v_bar|^2 - v_sq_bar / 2 = va.vb / 2.  So
 //   f_7 = f_0 (ff(beta)/((gamma-1) beta_bar) + va.vb)/2 + vn_bar rho_bar/(2 beta_bar) + B_bar.f_B.
-// 62 FP64 operations and a reciprocal against 107 for the expressions as the reference writes them
+// pref4 = 4 p_ref, a constant pressure left out of the normal momentum flux (f[1] / 4 = f_1 - p_ref):
+// it drops out of a line's flux differences, and with it goes their largest rounding error.
+// 65 FP64 operations and a reciprocal against 107 for the expressions as the reference writes them
 // (the kernel that calls this is bound by its FP64 chains).
 __device__ __forceinline__ double series_divisor(double u) {
   return dfma(u, dfma(u, dfma(u, 1.0 / 7.0, 1.0 / 5.0), 1.0 / 3.0), 1.0);
@@ -318,7 +320,7 @@ __device__ __forceinline__ double half_inv_series_divisor(double u) {
 }
 
 __device__ __forceinline__ void ec_flux4(const double* a, const double* b, double a_bsq, double b_bsq, double igm1,
-                                         double* f) {
+                                         double pref4, double* f) {
   const double rho_s = dadd(a[0], b[0]), beta_s = dadd(a[7], b[7]);
   const double rho_d = dsub(a[0], b[0]), beta_d = dsub(a[7], b[7]);
   const double r_rb = 1.0 / dmul(rho_s, beta_s);
@@ -336,9 +338,11 @@ __device__ __forceinline__ void ec_flux4(const double* a, const double* b, doubl
   const double vn = dadd(a[1], b[1]), vt = dadd(a[2], b[2]), vz = dadd(a[3], b[3]);
   const double bn = dadd(a[4], b[4]), bt = dadd(a[5], b[5]), bz = dadd(a[6], b[6]);
   const double h = dmul(rho_hat, vn);  // 2 f_0
-  const double q = dmul(rho_s, ib);    // rho_bar / beta_bar
+  // rho_bar / beta_bar (twice the pressure of equal states) with one correction step, so that equal
+  // states give their pressure to the last bit and pref4 takes it out
+  const double q0 = dmul(rho_s, ib), q = dfma(ib, dfma(-q0, beta_s, rho_s), q0);
   const double i2 = dadd(ib, ib);      // 1 / beta_bar
-  const double p4 = dfma(2.0, q, dadd(a_bsq, b_bsq));  // 4 p_tot
+  const double p4 = dadd(dadd(a_bsq, b_bsq), dfma(2.0, q, -pref4));  // 4 (p_tot - p_ref)
   f[0] = dadd(h, h);
   f[1] = dfma(vn, h, dfma(-bn, bn, p4));
   f[2] = dfma(vt, h, -dmul(bn, bt));
@@ -355,7 +359,9 @@ __device__ __forceinline__ void ec_flux4(const double* a, const double* b, doubl
 
 // ESPP_HLL_flux_x (DG_solver.f90:894-1071).  wl, wr: conserved states already rotated into the
 // face normal frame (swap_xy for y faces).  out[0..7] = numerical flux, out[8] = nBn,
-// out[9] = sl, out[10] = sr.  igm1 = 1/(gamma-1).  Quotients are formed as products with shared
+// out[9] = sl, out[10] = sr, out[11] = the smaller of the two pressures, which is left out of the
+// normal momentum flux (the flux is out[1] + out[11]): the elements subtract their reference
+// pressure from it before it meets the rest of the flux (see ec_flux4).  igm1 = 1/(gamma-1).  Quotients are formed as products with shared
 // reciprocals: 1/rho_l and 1/rho_r from 1/(rho_l rho_r); 1/p_l and 1/p_r from 1/(p_l p_r); the Roe
 // weight 1/(sqrt(rho_l)+sqrt(rho_r)); 1/a_form; 1/(sr-sl).  The values agree with the reference's
 // expression order to a few ulp.
@@ -378,6 +384,7 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
   const double r_p = 1.0 / dmul(p_l, p_r);
   const double ip_l = dmul(p_r, r_p), ip_r = dmul(p_l, r_p);
   const double pt_l = dadd(p_l, pm_l), pt_r = dadd(p_r, pm_r);
+  const double pb = fmin(p_l, p_r);
   const double bu_l = ddot3(bx_l, vx_l, by_l, vy_l, bz_l, vz_l);
   const double bu_r = ddot3(bx_r, vx_r, by_r, vy_r, bz_r, vz_r);
   const double cs_l = dmul(dmul(gamma, p_l), ir_l), cs_r = dmul(dmul(gamma, p_r), ir_r);
@@ -392,7 +399,7 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
   const double ef_r = dmul(dmul(dmul(-rho_r, se_r), igm1), vx_r);
   double fl[8], fr[8];
   fl[0] = mx_l;
-  fl[1] = dadd(dfma(vx_l, mx_l, -dmul(bx_l, bx_l)), pt_l);
+  fl[1] = dadd(dfma(vx_l, mx_l, -dmul(bx_l, bx_l)), dadd(dsub(p_l, pb), pm_l));
   fl[2] = dfma(vx_l, my_l, -dmul(by_l, bx_l));
   fl[3] = dfma(vx_l, mz_l, -dmul(bz_l, bx_l));
   fl[4] = 0.0;
@@ -400,7 +407,7 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
   fl[6] = dfma(bz_l, vx_l, -dmul(bx_l, vz_l));
   fl[7] = dfma(vx_l, dadd(e_l, pt_l), -dmul(bx_l, bu_l));
   fr[0] = mx_r;
-  fr[1] = dadd(dfma(vx_r, mx_r, -dmul(bx_r, bx_r)), pt_r);
+  fr[1] = dadd(dfma(vx_r, mx_r, -dmul(bx_r, bx_r)), dadd(dsub(p_r, pb), pm_r));
   fr[2] = dfma(vx_r, my_r, -dmul(by_r, bx_r));
   fr[3] = dfma(vx_r, mz_r, -dmul(bz_r, bx_r));
   fr[4] = 0.0;
@@ -446,12 +453,17 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
   const double sl = fmin(fmin(-dadd(ar, aa), sl_pp), 0.0);
   const double sr = fmax(fmax(dadd(al, aa), sr_pp), 0.0);
   const double idsl = 1.0 / dsub(sr, sl);
-  const double wl_ = dmul(sr, idsl), wr_ = dmul(-sl, idsl), wd = dmul(dmul(sl, sr), idsl);
+  // (sr fl - sl fr)/(sr - sl) from the side with the larger weight, plus the other weight (at most
+  // 1/2) times the difference: equal states give exactly their flux, a supersonic face its upwind one
+  const bool left = sr >= -sl;
+  const double w = dmul(left ? -sl : -sr, idsl), wd = dmul(dmul(sl, sr), idsl);
 #pragma unroll
-  for (int s = 0; s < 8; ++s) out[s] = dfma(wd, dsub(wr[s], wl[s]), dfma(wr_, fr[s], dmul(wl_, fl[s])));
-  out[8] = dfma(wr_, bx_r, dmul(wl_, bx_l));
+  for (int s = 0; s < 8; ++s)
+    out[s] = dfma(wd, dsub(wr[s], wl[s]), dfma(w, dsub(fr[s], fl[s]), left ? fl[s] : fr[s]));
+  out[8] = dfma(w, jbx, left ? bx_l : bx_r);
   out[9] = sl;
   out[10] = sr;
+  out[11] = pb;
 }
 
 }  // namespace mhd

@@ -40,8 +40,10 @@ struct StageCombine {
 // so no pair flux goes through shared memory.  The tile's element blocks arrive in shared memory by
 // bulk asynchronous copies (one per contiguous run) completed on an mbarrier; the interface fluxes
 // are computed from there as in the shared-memory form (every face node once, y faces through
-// swap_xy), spread evenly over the warps.  Each lane then forms its node's residual and stores it
-// directly (a variable's nodes of one element are contiguous, so the stores coalesce).
+// swap_xy), spread evenly over the warps.  Each lane then adds the interface fluxes to its node's
+// sum and stores it directly (a variable's nodes of one element are contiguous, so the stores
+// coalesce).  The kernel is bound by the latency of its FP64 chains at 16 warps per SM, so terms
+// that cancel are left out (see phase 2); that took the 253 x 261 p = 3 residual from 147 to 135 us.
 // =============================================================================================
 #if __has_include("residual2_tuned.h")
 #include "residual2_tuned.h"
@@ -85,7 +87,7 @@ struct Res2Layout {
   static constexpr int NT = Res2Cfg<P>::NT, NW = NT / 32;
   static constexpr int NFX = (TX + 1) * TY * N;
   static constexpr int NFY = TX * (TY + 1) * N;
-  static constexpr int FW = 11;
+  static constexpr int FW = 12;
   static_assert(TE <= NW * G, "every element of the tile needs a lane group");
   static_assert(NT % 32 == 0 && NT <= 1024, "whole warps");
   static_assert((ES * 8) % 16 == 0, "bulk copies land on 16-byte boundaries");
@@ -263,7 +265,7 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
         ostride = L::NFY;
       }
       if (!live) continue;
-      double wl[8], wr[8], o[11];
+      double wl[8], wr[8], o[12];
 #pragma unroll
       for (int v = 0; v < 8; ++v) {
         const int sv = ydir ? swap_xy_var(v) : v;
@@ -294,7 +296,7 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
   // (all arithmetic of the tile is exactly rounded as written: dmul/dadd/dsub/dfma of common.cuh)
   const double ir = 1.0 / w[0];
   const double vx = dmul(ir, w[1]), vy = dmul(ir, w[2]), vz = dmul(ir, w[3]);
-  double pt, sgx, sgy, bsq, pp[8];  // pp: (rho, vx, vy, vz, Bx, By, Bz, beta), the EC flux's inputs
+  double sgx, sgy, bsq, pref, pp[8];  // pp: (rho, vx, vy, vz, Bx, By, Bz, beta), the EC flux's inputs
   {
     const double ek = dmul(dmul(0.5, ir), dsq3(w[1], w[2], w[3]));
     bsq = dsq3(w[4], w[5], w[6]);
@@ -307,8 +309,8 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
     pp[5] = w[5];
     pp[6] = w[6];
     pp[7] = dmul(0.5, w[0]) / pf;
+    pref = __shfl_sync(FULL, pf, gbase);  // the element's reference pressure (see ec_flux4)
     const double cs = dmul(dmul(gamma, pf), ir), ss = dfma(bsq, ir, cs), coef = dmul(dmul(4.0, cs), ir);
-    pt = dfma(0.5, bsq, pf);
     sgx = dadd(fabs(vx), sqrt(dmul(0.5, fmax(dadd(ss, sqrt(fmax(dfma(ss, ss, -dmul(coef, dmul(w[4], w[4]))), 0.0))), 0.0))));
     sgy = dadd(fabs(vy), sqrt(dmul(0.5, fmax(dadd(ss, sqrt(fmax(dfma(ss, ss, -dmul(coef, dmul(w[5], w[5]))), 0.0))), 0.0))));
   }
@@ -323,47 +325,11 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
   for (int r = 0; r < N; ++r) dbx = __fma_rn(Dm(k + N * r), __shfl_sync(FULL, w[4], lane_of(r, l)), dbx);
 #pragma unroll
   for (int m = 0; m < N; ++m) dby = __fma_rn(__shfl_sync(FULL, w[5], lane_of(k, m)), Dm(l + N * m), dby);
-  // node flux F, G and Godunov-Powell coefficients (DG_solver.f90:749-799), formed again for the
-  // surface terms after the barrier; the accumulation starts, as the reference's does
-  // (DG_solver.f90:833), with the diagonal and Godunov-Powell terms
-  auto node_fluxes = [&](double* F, double* Gf, double* GP) {
-    const double bx = w[4], by = w[5], bz = w[6];
-    const double bu = ddot3(bx, vx, by, vy, bz, vz);
-    const double ex = dfma(by, vz, -dmul(bz, vy)), ey = dfma(bz, vx, -dmul(bx, vz)), ez = dfma(bx, vy, -dmul(by, vx));
-    F[0] = w[1];
-    F[1] = dadd(dfma(vx, w[1], -dmul(bx, bx)), pt);
-    F[2] = dfma(vx, w[2], -dmul(by, bx));
-    F[3] = dfma(vx, w[3], -dmul(bz, bx));
-    F[4] = 0.0;
-    F[5] = -ez;
-    F[6] = ey;
-    F[7] = dfma(vx, dadd(w[7], pt), -dmul(bx, bu));
-    Gf[0] = w[2];
-    Gf[1] = dfma(vy, w[1], -dmul(bx, by));
-    Gf[2] = dadd(dfma(vy, w[2], -dmul(by, by)), pt);
-    Gf[3] = dfma(vy, w[3], -dmul(bz, by));
-    Gf[4] = ez;
-    Gf[5] = 0.0;
-    Gf[6] = -ex;
-    Gf[7] = dfma(vy, dadd(w[7], pt), -dmul(by, bu));
-    GP[0] = 0.0;
-    GP[1] = bx;
-    GP[2] = by;
-    GP[3] = bz;
-    GP[4] = vx;
-    GP[5] = vy;
-    GP[6] = vz;
-    GP[7] = bu;
-  };
-  double acc[8];
-  {
-    double F[8], Gf[8], GP[8];
-    node_fluxes(F, Gf, GP);
-    const double divB = dfma(syh, dby, dmul(sxh, dbx));
-    const double ckk = 2.0 * sxh * Dm(k + N * k), cll = 2.0 * syh * Dm(l + N * l);
-#pragma unroll
-    for (int v = 0; v < 8; ++v) acc[v] = __fma_rn(-divB, GP[v], __fma_rn(-cll, Gf[v], -__dmul_rn(ckk, F[v])));
-  }
+  // The node's own flux never appears: the diagonal of the flux differencing, -2 (2/h) D_kk F(u_k)
+  // (DG_solver.f90:833), is zero inside the element (D_kk = 0), and at an end node it is cancelled by
+  // the own-flux part of that face's surface term (DG_solver.f90:872-882), because 2 D_NN = 1/w_N =
+  // -2 D_00 (the summation-by-parts property of the GLL rule).  What remains of the surface term is
+  // the interface flux and a multiple of the Godunov-Powell vector, which joins the -div B one.
   // Four times this lane's flux with the node in lane `src` (x frame, or y through swap_xy); the
   // result F is in the global frame.  Every lane of the warp calls it (the shuffles need the full warp).
   auto pair_flux = [&](int src, bool ydir, double* F) {
@@ -378,89 +344,78 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
       const double b = ydir ? B[sv] : B[v];
       Fx[v] = b;  // reuse as the rotated partner
     }
-    ec_flux4(A, Fx, bsq, bsq_src, igm1, B);
+    ec_flux4(A, Fx, bsq, bsq_src, igm1, dmul(4.0, pref), B);
 #pragma unroll
     for (int v = 0; v < 8; ++v) F[v] = ydir ? B[swap_xy_var(v)] : B[v];
   };
+  double acc[8];
   if constexpr (P == 1) {
     const bool xb = (k == l);
     double F[8];
     pair_flux(xb ? lane_of(1 - k, l) : lane_of(k, 1 - l), !xb, F);
-    const double c1 = xb ? sxq * Dm(k + N * (1 - k)) : syq * Dm(l + N * (1 - l));
+    const double c1 = -(xb ? sxq * Dm(k + N * (1 - k)) : syq * Dm(l + N * (1 - l)));
     const int src2 = xb ? lane_of(k, 1 - l) : lane_of(1 - k, l);
-    const double c2 = xb ? syq * Dm(l + N * (1 - l)) : sxq * Dm(k + N * (1 - k));
-    // the reference's order: x partner below, y partner below, x above, y above
-    const int rx = (1 - k) < k ? 0 : 2, ry = (1 - l) < l ? 1 : 3;
-    const bool own_first = xb ? rx < ry : ry < rx;
+    const double c2 = -(xb ? syq * Dm(l + N * (1 - l)) : sxq * Dm(k + N * (1 - k)));
 #pragma unroll
-    for (int v = 0; v < 8; ++v) {
-      const double fr = __shfl_sync(FULL, F[v], src2);
-      acc[v] = __fma_rn(-(own_first ? c1 : c2), own_first ? F[v] : fr, acc[v]);
-      acc[v] = __fma_rn(-(own_first ? c2 : c1), own_first ? fr : F[v], acc[v]);
-    }
+    for (int v = 0; v < 8; ++v) acc[v] = dfma(c2, __shfl_sync(FULL, F[v], src2), dmul(c1, F[v]));
   } else {
     // rings along x and y: compute with the next node, receive from the previous one
 #pragma unroll
     for (int dir = 0; dir < 2; ++dir) {
       const int a = dir == 0 ? k : l;
       const int an = (a + 1) % N, ap = (a + N - 1) % N;
-      const double h2 = dir == 0 ? sxq : syq;
+      const double h2 = dir == 0 ? -sxq : -syq;
       double F[8];
       pair_flux(dir == 0 ? lane_of(an, l) : lane_of(k, an), dir == 1, F);
       const double c1 = h2 * Dm(a + N * an), c2 = h2 * Dm(a + N * ap);
       const int src2 = dir == 0 ? lane_of(ap, l) : lane_of(k, ap);
-      const bool next_first = an < ap;  // the two contributions in ascending partner order
 #pragma unroll
       for (int v = 0; v < 8; ++v) {
         if (v == (dir == 0 ? 4 : 5)) continue;  // that component of the flux is identically zero
         const double fr = __shfl_sync(FULL, F[v], src2);
-        acc[v] = __fma_rn(-(next_first ? c1 : c2), next_first ? F[v] : fr, acc[v]);
-        acc[v] = __fma_rn(-(next_first ? c2 : c1), next_first ? fr : F[v], acc[v]);
+        acc[v] = dfma(c2, fr, (dir == 0 || v == 4) ? dmul(c1, F[v]) : dfma(c1, F[v], acc[v]));
       }
     }
     if constexpr (P == 3) {  // the pairs (k, k^2) along x and (l, l^2) along y
       const bool xb = ((k >> 1) ^ (l >> 1)) == 0;
       double F[8];
       pair_flux(xb ? lane_of(k ^ 2, l) : lane_of(k, l ^ 2), !xb, F);
-      const double cx = sxq * Dm(k + N * (k ^ 2)), cy = syq * Dm(l + N * (l ^ 2));
+      const double cx = -(sxq * Dm(k + N * (k ^ 2))), cy = -(syq * Dm(l + N * (l ^ 2)));
       const int src2 = xb ? lane_of(k, l ^ 2) : lane_of(k ^ 2, l);
-      // the reference's order: x partner below, y partner below, x above, y above
-      const int rx = (k ^ 2) < k ? 0 : 2, ry = (l ^ 2) < l ? 1 : 3;
-      const bool own_first = xb ? rx < ry : ry < rx;
       const double c1 = xb ? cx : cy, c2 = xb ? cy : cx;
 #pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        const double fr = __shfl_sync(FULL, F[v], src2);
-        acc[v] = __fma_rn(-(own_first ? c1 : c2), own_first ? F[v] : fr, acc[v]);
-        acc[v] = __fma_rn(-(own_first ? c2 : c1), own_first ? fr : F[v], acc[v]);
-      }
+      for (int v = 0; v < 8; ++v) acc[v] = dfma(c2, __shfl_sync(FULL, F[v], src2), dfma(c1, F[v], acc[v]));
     }
   }
   __syncthreads();  // the interface fluxes of phase 1 are complete
 
-  // ---- phase 3: surface terms; dt_lim; store ----
+  // ---- phase 3: surface terms, Godunov-Powell terms; dt_lim; store ----
   {
-    const double bx = w[4], by = w[5];
-    double F[8], Gf[8], GP[8];
-    node_fluxes(F, Gf, GP);
-    // surface terms (DG_solver.f90:872-882): left face (k = 0) with -, right face (k = N-1) with +;
-    // likewise bottom/top in y
+    // (2/h)/w times the interface flux, + at the first node of a line and - at the last; `src`
+    // collects the factor of the Godunov-Powell vector (0, B, v, v.B) (DG_solver.f90:794-799)
+    double src = -dfma(syh, dby, dmul(sxh, dbx));
     if (k == 0 || k == N - 1) {
       const bool right = (k == N - 1);
       const double* fr = s_fx + (((ec + (right ? 1 : 0)) * TY + er) * N + l);
-      const double c = (right ? sxh : -sxh) * s_dm[NN + k];
-      const double jb = __dadd_rn(bx, -fr[8 * L::NFX]);
+      const double c = (right ? -sxh : sxh) * s_dm[NN + k];
+      src = dfma(-c, dsub(pp[4], fr[8 * L::NFX]), src);
 #pragma unroll
-      for (int v = 0; v < 8; ++v) acc[v] = __fma_rn(c, __fma_rn(GP[v], jb, __dadd_rn(F[v], -fr[v * L::NFX])), acc[v]);
+      for (int v = 0; v < 8; ++v)
+        acc[v] = dfma(c, v == 1 ? dadd(fr[L::NFX], dsub(fr[11 * L::NFX], pref)) : fr[v * L::NFX], acc[v]);
     }
     if (l == 0 || l == N - 1) {
       const bool top = (l == N - 1);
       const double* fr = s_fy + (((er + (top ? 1 : 0)) * TX + ec) * N + k);
-      const double c = (top ? syh : -syh) * s_dm[NN + l];
-      const double jb = __dadd_rn(by, -fr[8 * L::NFY]);
+      const double c = (top ? -syh : syh) * s_dm[NN + l];
+      src = dfma(-c, dsub(pp[5], fr[8 * L::NFY]), src);
 #pragma unroll
-      for (int v = 0; v < 8; ++v) acc[v] = __fma_rn(c, __fma_rn(GP[v], jb, __dadd_rn(Gf[v], -fr[v * L::NFY])), acc[v]);
+      for (int v = 0; v < 8; ++v)
+        acc[v] = dfma(c, v == 2 ? dadd(fr[2 * L::NFY], dsub(fr[11 * L::NFY], pref)) : fr[v * L::NFY], acc[v]);
     }
+    const double gp[8] = {0.0, pp[4], pp[5], pp[6], pp[1], pp[2], pp[3],
+                          ddot3(pp[4], pp[1], pp[5], pp[2], pp[6], pp[3])};
+#pragma unroll
+    for (int v = 1; v < 8; ++v) acc[v] = dfma(src, gp[v], acc[v]);
   }
   // dt_lim of the element: the largest node speed and interface speed per direction
   double my_dt = 1.0e300;
@@ -481,10 +436,11 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
       const long long e = ((long long)(j0 + er) * (nx + 2) + (i0 + ec)) * EB + node;
       const double dt = s_red[31];
       const double* u0n = s_u0 + el * ES + node;
+      const double* un = s_cons + el * ES + node;  // (read again: not held in registers meanwhile)
 #pragma unroll
       for (int v = 0; v < 8; ++v)
         sc.out[e + v * NN] = __dadd_rn(__dmul_rn(sc.ca, u0n[v * NN]),
-                                       __dmul_rn(sc.cb, __dadd_rn(w[v], __dmul_rn(dt, acc[v]))));
+                                       __dmul_rn(sc.cb, __dadd_rn(un[v * NN], __dmul_rn(dt, acc[v]))));
     } else {
       double* o = to.ut + ((long long)(j0 + er - 1) * nx + (i0 + ec - 1)) * EB + node;
 #pragma unroll
