@@ -613,6 +613,7 @@ int create_instance(int nx, int ny, int px, int py, int rknstg, double left, dou
   h->geo.bc_kind = bc_kind;
   for (int v = 0; v < 8; ++v) h->geo.bc_state[v] = h->bc_state[v];
   h->geo.ldfA = h->ldfA;
+  geo_constants(h->geo);
   if ((sync ? cudaStreamSynchronize(h->stream) : cudaGetLastError()) != cudaSuccess) {
     free_all(h);
     delete h;
@@ -1117,6 +1118,7 @@ extern "C" int mhd_gpu_semidiscretize_noalloc(int p, int nx, int ny, double hx, 
   g.hx = hx;
   g.hy = hy;
   g.gamma = gamma;
+  geo_constants(g);
   switch (p) {
     case 1: {
       using L = Res2Layout<1>;

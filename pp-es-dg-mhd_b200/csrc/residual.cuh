@@ -231,7 +231,7 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
     phase ^= 1u;
   }
 
-  const double igm1 = 1.0 / (gamma - 1.0);
+  const double igm1 = g.igm1;
   // ---- phase 1: interface fluxes, every face node of the tile once ----
   // Thread-major: the items fill whole warps first, so the fewest warps run this code (a warp
   // pays its issue slots whether or not all its lanes have an item); the others go on to phase 2.
@@ -285,7 +285,7 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
   const bool act = grp < G && el < TE && er < H && ec < W;
   const int gbase = (grp < G ? grp : 0) * NN;  // lanes beyond the groups mirror group 0
   const int k = node % N, l = node / N;
-  const double sxh = 2.0 / g.hx, syh = 2.0 / g.hy;
+  const double sxh = g.sxh, syh = g.syh;
   const double sxq = 0.5 * sxh, syq = 0.5 * syh;  // 2 (2/h) / 4: the pair fluxes come as four times the flux
   double w[8];
   {
@@ -294,7 +294,7 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
     for (int v = 0; v < 8; ++v) w[v] = cw[v * NN];
   }
   // (all arithmetic of the tile is exactly rounded as written: dmul/dadd/dsub/dfma of common.cuh)
-  const double ir = 1.0 / w[0];
+  const double ir = rcp_nr(w[0]);
   const double vx = dmul(ir, w[1]), vy = dmul(ir, w[2]), vz = dmul(ir, w[3]);
   double sgx, sgy, bsq, pref, pp[8];  // pp: (rho, vx, vy, vz, Bx, By, Bz, beta), the EC flux's inputs
   {
@@ -308,11 +308,11 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
     pp[4] = w[4];
     pp[5] = w[5];
     pp[6] = w[6];
-    pp[7] = dmul(0.5, w[0]) / pf;
+    pp[7] = dmul(dmul(0.5, w[0]), rcp_nr(pf));
     pref = __shfl_sync(FULL, pf, gbase);  // the element's reference pressure (see ec_flux4)
     const double cs = dmul(dmul(gamma, pf), ir), ss = dfma(bsq, ir, cs), coef = dmul(dmul(4.0, cs), ir);
-    sgx = dadd(fabs(vx), sqrt(dmul(0.5, fmax(dadd(ss, sqrt(fmax(dfma(ss, ss, -dmul(coef, dmul(w[4], w[4]))), 0.0))), 0.0))));
-    sgy = dadd(fabs(vy), sqrt(dmul(0.5, fmax(dadd(ss, sqrt(fmax(dfma(ss, ss, -dmul(coef, dmul(w[5], w[5]))), 0.0))), 0.0))));
+    sgx = dadd(fabs(vx), sqrt_nr(dmul(0.5, fmax(dadd(ss, sqrt_nr(fmax(dfma(ss, ss, -dmul(coef, dmul(w[4], w[4]))), TINY))), TINY))));
+    sgy = dadd(fabs(vy), sqrt_nr(dmul(0.5, fmax(dadd(ss, sqrt_nr(fmax(dfma(ss, ss, -dmul(coef, dmul(w[5], w[5]))), TINY))), TINY))));
   }
   auto Dm = [&](int i) { return s_dm[i]; };
   // the partner lane of node (kk, ll) of this lane's element
@@ -429,7 +429,7 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
     }
     ax = group_max<NN>(ax, gbase);
     ay = group_max<NN>(ay, gbase);
-    if (act && node == 0) my_dt = 1.0 / ((2 * P + 1) * ax / g.hx + (2 * P + 1) * ay / g.hy);
+    if (act && node == 0) my_dt = 1.0 / dmul(P + 0.5, dfma(ax, sxh, dmul(ay, syh)));
   }
   if (act) {
     if (sc.u0) {  // the next stage's state instead of L(u)
