@@ -392,6 +392,12 @@ __device__ __forceinline__ void ec_flux4(const double* a, const double* b, doubl
   f[7] = dfma(0.5, dfma(bz, f[6], dmul(bt, f[5])), dfma(vn, q, dmul(h, x)));
 }
 
+// The gas pressure, clamped (DG_solver.f90:779,951-954), from m.v, |B|^2 and the total energy: one
+// expression for nodes and interface states, so that the reference pressure cancels to the last bit.
+__device__ __forceinline__ double gas_pressure(double gm1, double mv, double bsq, double e) {
+  return fmax(dmul(gm1, dfma(-0.5, dadd(mv, bsq), e)), PP_EPS);
+}
+
 // ESPP_HLL_flux_x (DG_solver.f90:894-1071).  wl, wr: conserved states already rotated into the
 // face normal frame (swap_xy for y faces).  out[0..7] = numerical flux, out[8] = nBn,
 // out[9] = sl, out[10] = sr, out[11] = the smaller of the two pressures, which is left out of the
@@ -399,88 +405,90 @@ __device__ __forceinline__ void ec_flux4(const double* a, const double* b, doubl
 // pressure from it before it meets the rest of the flux (see ec_flux4).  igm1 = 1/(gamma-1).
 // Quotients are formed as products with reciprocals (rcp_nr); the values agree with the reference's
 // expression order to a few ulp.
+//
+// The entropy s = log p - gamma log rho enters only through its jump ds = s_r - s_l: with the entropy
+// flux q = -m s/(gamma-1) (m the normal momentum) and the first entropy variable
+// v_0 = (gamma - s)/(gamma-1) - k (k = the kinetic energy over p),
+//   q_r - q_l - v_0l (m_r - m_l) = -(m_r ds + gamma (m_r - m_l))/(gamma-1) + k_l (m_r - m_l),
+// likewise with v_0r and m_l ds, and v_0r - v_0l = -ds/(gamma-1) - (k_r - k_l).  So two logarithms
+// of ratios replace four, with the series log z = 2f (1 + u/3 + u^2/5 + ...), f = (z-1)/(z+1), u = f^2,
+// where both ratios are close to one (u < 1.4e-4, as in the two-point flux; truncation 5e-17
+// relative).  The sums over the entropy variables are taken as scalar products of the momentum and
+// field jumps.  Against four logarithms and component-by-component sums: 253 x 261 p = 3 residual
+// 105.2 -> 94.2 us, 301 x 199 p = 1 step 256 -> 242 us.
 __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, double gamma, double igm1, double* out) {
-  const double rho_l = wl[0], mx_l = wl[1], my_l = wl[2], mz_l = wl[3], bx_l = wl[4], by_l = wl[5], bz_l = wl[6], e_l = wl[7];
-  const double rho_r = wr[0], mx_r = wr[1], my_r = wr[2], mz_r = wr[3], bx_r = wr[4], by_r = wr[5], bz_r = wr[6], e_r = wr[7];
   const double gm1 = dsub(gamma, 1.0);
-  const double ir_l = rcp_nr(rho_l), ir_r = rcp_nr(rho_r);
-  const double vx_l = dmul(ir_l, mx_l), vx_r = dmul(ir_r, mx_r);
-  const double vy_l = dmul(ir_l, my_l), vy_r = dmul(ir_r, my_r);
-  const double vz_l = dmul(ir_l, mz_l), vz_r = dmul(ir_r, mz_r);
-  const double ek_l = dmul(dmul(0.5, ir_l), dsq3(mx_l, my_l, mz_l));
-  const double ek_r = dmul(dmul(0.5, ir_r), dsq3(mx_r, my_r, mz_r));
-  const double bsq_l = dsq3(bx_l, by_l, bz_l);
-  const double bsq_r = dsq3(bx_r, by_r, bz_r);
-  const double pm_l = dmul(0.5, bsq_l), pm_r = dmul(0.5, bsq_r);
-  const double p_l = fmax(dmul(gm1, dsub(e_l, dadd(ek_l, pm_l))), PP_EPS);
-  const double p_r = fmax(dmul(gm1, dsub(e_r, dadd(ek_r, pm_r))), PP_EPS);
-  const double ip_l = rcp_nr(p_l), ip_r = rcp_nr(p_r);
-  const double pt_l = dadd(p_l, pm_l), pt_r = dadd(p_r, pm_r);
-  const double pb = fmin(p_l, p_r);
-  const double bu_l = ddot3(bx_l, vx_l, by_l, vy_l, bz_l, vz_l);
-  const double bu_r = ddot3(bx_r, vx_r, by_r, vy_r, bz_r, vz_r);
-  const double cs_l = dmul(dmul(gamma, p_l), ir_l), cs_r = dmul(dmul(gamma, p_r), ir_r);
-  const double ss_l = dfma(bsq_l, ir_l, cs_l), ss_r = dfma(bsq_r, ir_r, cs_r);
-  const double cf_l = sqrt_nr(dmul(0.5, dadd(ss_l, sqrt_nr(fmax(dfma(ss_l, ss_l, -dmul(dmul(dmul(4.0, cs_l), ir_l), dmul(bx_l, bx_l))), TINY)))));
-  const double cf_r = sqrt_nr(dmul(0.5, dadd(ss_r, sqrt_nr(fmax(dfma(ss_r, ss_r, -dmul(dmul(dmul(4.0, cs_r), ir_r), dmul(bx_r, bx_r))), TINY)))));
-  const double ith_l = dmul(rho_l, ip_l), ith_r = dmul(rho_r, ip_r);
-  const double phi_l = dmul(ith_l, bu_l), phi_r = dmul(ith_r, bu_r);
-  const double se_l = dfma(-gamma, log(rho_l), log(p_l));
-  const double se_r = dfma(-gamma, log(rho_r), log(p_r));
-  const double ef_l = dmul(dmul(dmul(-rho_l, se_l), igm1), vx_l);
-  const double ef_r = dmul(dmul(dmul(-rho_r, se_r), igm1), vx_r);
-  double fl[8], fr[8];
-  fl[0] = mx_l;
-  fl[1] = dadd(dfma(vx_l, mx_l, -dmul(bx_l, bx_l)), dadd(dsub(p_l, pb), pm_l));
-  fl[2] = dfma(vx_l, my_l, -dmul(by_l, bx_l));
-  fl[3] = dfma(vx_l, mz_l, -dmul(bz_l, bx_l));
-  fl[4] = 0.0;
-  fl[5] = -dfma(bx_l, vy_l, -dmul(by_l, vx_l));
-  fl[6] = dfma(bz_l, vx_l, -dmul(bx_l, vz_l));
-  fl[7] = dfma(vx_l, dadd(e_l, pt_l), -dmul(bx_l, bu_l));
-  fr[0] = mx_r;
-  fr[1] = dadd(dfma(vx_r, mx_r, -dmul(bx_r, bx_r)), dadd(dsub(p_r, pb), pm_r));
-  fr[2] = dfma(vx_r, my_r, -dmul(by_r, bx_r));
-  fr[3] = dfma(vx_r, mz_r, -dmul(bz_r, bx_r));
-  fr[4] = 0.0;
-  fr[5] = -dfma(bx_r, vy_r, -dmul(by_r, vx_r));
-  fr[6] = dfma(bz_r, vx_r, -dmul(bx_r, vz_r));
-  fr[7] = dfma(vx_r, dadd(e_r, pt_r), -dmul(bx_r, bu_r));
-  const double sq_l = sqrt_nr(rho_l), sq_r = sqrt_nr(rho_r);
-  const double isum = rcp_nr(dadd(sq_l, sq_r));
-  const double vx_roe = dmul(dfma(vx_r, sq_r, dmul(vx_l, sq_l)), isum);
-  const double db = dmul(sqrt_nr(dadd(dsq3(dsub(bx_l, bx_r), dsub(by_l, by_r), dsub(bz_l, bz_r)), TINY)), isum);
-  const double sl_pp = dsub(dsub(fmin(vx_l, vx_roe), cf_l), db);
-  const double sr_pp = dadd(dadd(fmax(vx_r, vx_roe), cf_r), db);
-  // entropy variables (DG_solver.f90:1003-1019) formed component by component, not kept
-  double da = 0.0, dbl = 0.0, dbr = 0.0;
+  double ir[2], v[2][3], mv[2], bsq[2], prs[2], ip[2], ith[2], bu[2], cf[2], sq[2], f[2][8];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {  // the two sides
+    const double* w = h ? wr : wl;
+    ir[h] = rcp_nr(w[0]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) v[h][q] = dmul(ir[h], w[1 + q]);
+    mv[h] = ddot3(w[1], v[h][0], w[2], v[h][1], w[3], v[h][2]);
+    bsq[h] = dsq3(w[4], w[5], w[6]);
+    prs[h] = gas_pressure(gm1, mv[h], bsq[h], w[7]);
+    ip[h] = rcp_nr(prs[h]);
+    ith[h] = dmul(w[0], ip[h]);
+    bu[h] = ddot3(w[4], v[h][0], w[5], v[h][1], w[6], v[h][2]);
+    const double bn2 = dmul(w[4], w[4]);
+    const double cs = dmul(dmul(gamma, prs[h]), ir[h]), ss = dfma(bsq[h], ir[h], cs);
+    const double disc = fmax(dfma(ss, ss, -dmul(dmul(dmul(4.0, cs), ir[h]), bn2)), TINY);
+    cf[h] = sqrt_nr(dmul(0.5, dadd(ss, sqrt_nr(disc))));
+    sq[h] = sqrt_nr(w[0]);
+    f[h][0] = w[1];
+    f[h][1] = dfma(v[h][0], w[1], -bn2);  // the pressures follow below
+    f[h][2] = dfma(v[h][0], w[2], -dmul(w[5], w[4]));
+    f[h][3] = dfma(v[h][0], w[3], -dmul(w[6], w[4]));
+    f[h][4] = 0.0;
+    f[h][5] = dfma(w[5], v[h][0], -dmul(w[4], v[h][1]));
+    f[h][6] = dfma(w[6], v[h][0], -dmul(w[4], v[h][2]));
+    f[h][7] = dfma(v[h][0], dadd(w[7], dfma(0.5, bsq[h], prs[h])), -dmul(w[4], bu[h]));
+  }
+  const double pb = fmin(prs[0], prs[1]);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) f[h][1] = dadd(f[h][1], dfma(0.5, bsq[h], dsub(prs[h], pb)));
+  double ds;
+  {
+    const double fp = dmul(dsub(prs[1], prs[0]), rcp_nr(dadd(prs[0], prs[1]))), up = dmul(fp, fp);
+    const double fd = dmul(dsub(wr[0], wl[0]), rcp_nr(dadd(wl[0], wr[0]))), ud = dmul(fd, fd);
+    double lp = dmul(dadd(fp, fp), series_divisor(up)), ld = dmul(dadd(fd, fd), series_divisor(ud));
+    if (up >= 1.4e-4 || ud >= 1.4e-4) {
+      if (up >= 1.4e-4) lp = log(dmul(prs[1], ip[0]));
+      if (ud >= 1.4e-4) ld = log(dmul(wr[0], ir[0]));
+    }
+    ds = dmul(dfma(-gamma, ld, lp), igm1);  // (s_r - s_l)/(gamma-1)
+  }
+  double j[8], d[8];
 #pragma unroll
   for (int s = 0; s < 8; ++s) {
-    double vls, vrs;
-    if (s == 0) {
-      vls = dfma(-ek_l, ip_l, dmul(dsub(gamma, se_l), igm1));
-      vrs = dfma(-ek_r, ip_r, dmul(dsub(gamma, se_r), igm1));
-    } else if (s < 4) {
-      vls = dmul(wl[s], ip_l);
-      vrs = dmul(wr[s], ip_r);
-    } else if (s < 7) {
-      vls = dmul(ith_l, wl[s]);
-      vrs = dmul(ith_r, wr[s]);
-    } else {
-      vls = -ith_l;
-      vrs = -ith_r;
-    }
-    const double dfs = dsub(fr[s], fl[s]);
-    da = dfma(dsub(vrs, vls), dsub(wr[s], wl[s]), da);
-    dbl = dfma(vls, dfs, dbl);
-    dbr = dfma(vrs, dfs, dbr);
+    j[s] = dsub(wr[s], wl[s]);
+    if (s != 4) d[s] = dsub(f[1][s], f[0][s]);
   }
+  d[4] = 0.0;
+  const double isum = rcp_nr(dadd(sq[0], sq[1]));
+  const double vx_roe = dmul(dfma(v[1][0], sq[1], dmul(v[0][0], sq[0])), isum);
+  const double db = dmul(sqrt_nr(dadd(dsq3(j[4], j[5], j[6]), TINY)), isum);
+  const double sl_pp = dsub(dsub(fmin(v[0][0], vx_roe), cf[0]), db);
+  const double sr_pp = dadd(dadd(fmax(v[1][0], vx_roe), cf[1]), db);
+  // a = sum (v_r - v_l)(w_r - w_l); b = q_r - q_l - sum v (f_r - f_l) - phi (B_r - B_l)_n per side
+  const double gg = dmul(gamma, igm1);
+  double k[2], b[2], mj[2], bj[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const double* w = h ? wr : wl;
+    k[h] = dmul(dmul(0.5, mv[h]), ip[h]);
+    mj[h] = dmul(ip[h], ddot3(w[1], j[1], w[2], j[2], w[3], j[3]));
+    bj[h] = dmul(ith[h], ddot3(w[4], j[4], w[5], j[5], w[6], j[6]));
+    const double md = dmul(ip[h], ddot3(w[1], d[1], w[2], d[2], w[3], d[3]));
+    const double vd = dfma(ith[h], dfma(w[6], d[6], dfma(w[5], d[5], -d[7])), md);
+    b[h] = -dfma(dmul(ith[h], bu[h]), j[4], dfma(dsub(gg, k[h]), d[0], dfma(h ? wl[1] : wr[1], ds, vd)));
+  }
+  const double da = dadd(dfma(dsub(ith[0], ith[1]), j[7], -dmul(dadd(ds, dsub(k[1], k[0])), j[0])),
+                         dadd(dsub(mj[1], mj[0]), dsub(bj[1], bj[0])));
   const double ia = rcp_nr(dadd(fmax(da, 0.0), 1e-8));
-  const double def = dsub(ef_r, ef_l), jbx = dsub(bx_r, bx_l);
-  const double bl_form = dfma(-phi_l, jbx, dsub(def, dbl));
-  const double br_form = dfma(-phi_r, jbx, dsub(def, dbr));
-  const double al = fmax(dmul(bl_form, ia), 0.0);
-  const double ar = fmax(dmul(br_form, ia), 0.0);
+  const double al = fmax(dmul(b[0], ia), 0.0);
+  const double ar = fmax(dmul(b[1], ia), 0.0);
   const double aa = sqrt_nr(dfma(al, ar, TINY));
   const double sl = fmin(fmin(-dadd(ar, aa), sl_pp), 0.0);
   const double sr = fmax(fmax(dadd(al, aa), sr_pp), 0.0);
@@ -490,9 +498,8 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
   const bool left = sr >= -sl;
   const double w = dmul(left ? -sl : -sr, idsl), wd = dmul(dmul(sl, sr), idsl);
 #pragma unroll
-  for (int s = 0; s < 8; ++s)
-    out[s] = dfma(wd, dsub(wr[s], wl[s]), dfma(w, dsub(fr[s], fl[s]), left ? fl[s] : fr[s]));
-  out[8] = dfma(w, jbx, left ? bx_l : bx_r);
+  for (int s = 0; s < 8; ++s) out[s] = dfma(wd, j[s], dfma(w, d[s], left ? f[0][s] : f[1][s]));
+  out[8] = dfma(w, j[4], left ? wl[4] : wr[4]);
   out[9] = sl;
   out[10] = sr;
   out[11] = pb;

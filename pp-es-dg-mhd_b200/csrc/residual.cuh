@@ -298,9 +298,8 @@ __device__ __forceinline__ bool residual_tile2(const double* __restrict__ u, con
   const double vx = dmul(ir, w[1]), vy = dmul(ir, w[2]), vz = dmul(ir, w[3]);
   double sgx, sgy, bsq, pref, pp[8];  // pp: (rho, vx, vy, vz, Bx, By, Bz, beta), the EC flux's inputs
   {
-    const double ek = dmul(dmul(0.5, ir), dsq3(w[1], w[2], w[3]));
     bsq = dsq3(w[4], w[5], w[6]);
-    const double pf = fmax(dmul(dsub(gamma, 1.0), dsub(w[7], dfma(0.5, bsq, ek))), PP_EPS);
+    const double pf = gas_pressure(dsub(gamma, 1.0), ddot3(w[1], vx, w[2], vy, w[3], vz), bsq, w[7]);
     pp[0] = w[0];
     pp[1] = vx;
     pp[2] = vy;
