@@ -4,8 +4,9 @@
 
 Two groups of build-time knobs, each a macro per degree p = 1, 2, 3:
 
-  residual  MHD_RES2_CFG<p> = TX, TY, threads, CTAs per SM of the residual tile (csrc/residual.cuh;
-            a tile holds at most (threads / 32) * (32 / (p+1)^2) elements, one lane per node).
+  residual  MHD_RES2_CFG<p> = TX, TY, threads, CTAs per SM of the residual (csrc/residual.cuh: each
+            warp takes one item of a CTA's TX x TY elements, 4 x 2, 3 x 1 or 2 x 1 of them at
+            p = 1, 2, 3, one lane per node).
             Timed: the residual alone, CUDA events over 20 launches.  Written to
             csrc/residual2_tuned.h.
   post      MHD_PP_CFG<p> = threads, CTAs per SM of the loop-1 and loop-3 kernels, and
@@ -35,10 +36,10 @@ import build as B  # noqa: E402
 # group -> macro(s) -> per degree the candidates; set i takes candidate i of every degree
 GROUPS = {
     "residual": {
-        "MHD_RES2_CFG": {  # 128 threads at 4, 5 and 6 CTAs per SM (128, 102, 85 registers), 256 at 3
-            1: [(8, 4, 128, 4), (8, 4, 128, 5), (8, 4, 128, 6), (8, 8, 256, 3)],
-            2: [(4, 3, 128, 4), (4, 3, 128, 5), (4, 3, 128, 6), (6, 4, 256, 3)],
-            3: [(4, 2, 128, 4), (4, 2, 128, 5), (4, 2, 128, 6), (8, 2, 256, 3)],
+        "MHD_RES2_CFG": {  # one warp a CTA at 16 per SM (128 registers), two at 8, four at 4, one at 18 (112)
+            1: [(4, 2, 32, 16), (4, 4, 64, 8), (8, 4, 128, 4), (4, 2, 32, 18)],
+            2: [(3, 1, 32, 16), (3, 2, 64, 8), (6, 2, 128, 4), (3, 1, 32, 18)],
+            3: [(2, 1, 32, 16), (2, 2, 64, 8), (4, 2, 128, 4), (2, 1, 32, 17)],
         },
     },
     "post": {  # sets 1 and 2 vary the indicator kernel, set 3 loops 1 and 3, against set 0

@@ -95,10 +95,9 @@ InstDesc make_desc(const mhd_gpu* h) {
 // items of each kind one member contributes (the same decomposition as its single-instance launches)
 template <int P>
 void member_work(const mhd_gpu* h, long long* cnt, InstDesc& d) {
-  using RL = Res2Layout<P>;
   constexpr int EB = 8 * (P + 1) * (P + 1), TE = PPCfg<P>::TE;
   const long long nx = h->nx, ny = h->ny;
-  cnt[WK_RES] = ((nx + RL::TX - 1) / RL::TX) * ((ny + RL::TY - 1) / RL::TY);
+  cnt[WK_RES] = (long long)res2_item_cols<P>(h->nx) * res2_item_rows<P>(h->ny);
   const long long nelg = (nx + 2) * (ny + 2);
   d.nblk_avg = (int)((nelg + TE - 1) / TE);
   cnt[WK_AVG] = d.nblk_avg;

@@ -30,6 +30,14 @@ struct DegConst {
 };
 // Defined here: the device code of the library is one translation unit (mhd_gpu.cu).
 __constant__ DegConst c_deg[MAXP + 1];
+// The rows of D for lanes that each want their own (a constant-memory read is replayed once per
+// distinct address): row k starting at its diagonal, row[k][r] = D(k, (k + r) mod n), 16-byte aligned,
+// and 1/w_k.  In global memory, read through L1.
+struct DegRows {
+  double row[MAXN][4];
+  double iqw[MAXN];
+};
+__device__ DegRows d_rows[MAXP + 1];
 
 // Status flag bits of the control block (the MHD_FLAG_* values of mhd_gpu.h).  FLAGS_FATAL: the
 // bits that end a run (every bit but the per-stage inadmissible average).
@@ -153,16 +161,18 @@ __device__ __forceinline__ int batch_member(const int* __restrict__ pref, int n,
   return lo;
 }
 
-// The items a CTA of a batched kernel takes: one contiguous share [b*nw/G, (b+1)*nw/G) of the
-// group's nw items (CTA b of G), visited in order.  The member is found by binary search once and
+// The items a worker of a batched kernel (a CTA, or a warp of the residual) takes: one contiguous
+// share [b*nw/G, (b+1)*nw/G) of the group's nw items (worker b of G), visited in order.  The member is found by binary search once and
 // then walked forward, so consecutive items of one member reuse its descriptor (and whatever the
 // kernel staged for it), and neighbouring tiles of a member are processed close in time.
 // pref == nullptr: a single instance owns all nw items.
 struct BatchWalk {
   const int* pref;
   int w, last, m, mstart, mend;
-  __device__ __forceinline__ BatchWalk(const int* __restrict__ pref_, int n, int nw) : pref(pref_) {
-    const long long b = blockIdx.x, G = gridDim.x;
+  __device__ __forceinline__ BatchWalk(const int* __restrict__ pref_, int n, int nw)
+      : BatchWalk(pref_, n, nw, blockIdx.x, gridDim.x) {}
+  __device__ __forceinline__ BatchWalk(const int* __restrict__ pref_, int n, int nw, long long b, long long G)
+      : pref(pref_) {
     w = (int)(b * nw / G);
     last = (int)((b + 1) * nw / G);
     m = mstart = 0;
@@ -186,11 +196,14 @@ struct BatchWalk {
 };
 
 // BatchWalk's order of items with the walker's state in shared memory, for kernels whose items need
-// every register: thread 0 starts and advances it, between barriers of the whole CTA.
+// every register: one thread starts and advances it, between barriers of the worker (CTA or warp).
 struct SharedWalk {
   int w, last, m, mstart, mend;
   __device__ __forceinline__ void start(const int* __restrict__ pref, int n, int nw) {
-    const BatchWalk it(pref, n, nw);
+    start(pref, n, nw, blockIdx.x, gridDim.x);
+  }
+  __device__ __forceinline__ void start(const int* __restrict__ pref, int n, int nw, long long b, long long G) {
+    const BatchWalk it(pref, n, nw, b, G);
     w = it.w;
     last = it.last;
     m = it.m;
@@ -230,7 +243,7 @@ __device__ __forceinline__ bool gate_open(const Ctrl* c, int gate) {
 }
 
 // ---- asynchronous bulk copies global -> shared (sm_90+ cp.async.bulk, completed on an mbarrier) ---
-// Used for tile rows, which are contiguous runs of 16-byte aligned element blocks.  The source is
+// Used for element blocks, which are contiguous and 16-byte aligned.  The source is
 // always this GPU's own memory; no multicast.
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
@@ -288,6 +301,10 @@ __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a,
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double dfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+// x, or the clamp c where x is smaller (larger) or NaN: the result of fmax (fmin) for a clamp that is
+// not NaN, as one comparison and a select
+__device__ __forceinline__ double at_least(double x, double c) { return x > c ? x : c; }
+__device__ __forceinline__ double at_most(double x, double c) { return x < c ? x : c; }
 // a*a + b*b + c*c, left to right with fused multiply-adds
 __device__ __forceinline__ double dsq3(double a, double b, double c) { return dfma(c, c, dfma(b, b, dmul(a, a))); }
 // a1*b1 + a2*b2 + a3*b3, likewise
@@ -395,7 +412,7 @@ __device__ __forceinline__ void ec_flux4(const double* a, const double* b, doubl
 // The gas pressure, clamped (DG_solver.f90:779,951-954), from m.v, |B|^2 and the total energy: one
 // expression for nodes and interface states, so that the reference pressure cancels to the last bit.
 __device__ __forceinline__ double gas_pressure(double gm1, double mv, double bsq, double e) {
-  return fmax(dmul(gm1, dfma(-0.5, dadd(mv, bsq), e)), PP_EPS);
+  return at_least(dmul(gm1, dfma(-0.5, dadd(mv, bsq), e)), PP_EPS);
 }
 
 // ESPP_HLL_flux_x (DG_solver.f90:894-1071).  wl, wr: conserved states already rotated into the
@@ -418,7 +435,7 @@ __device__ __forceinline__ double gas_pressure(double gm1, double mv, double bsq
 // 105.2 -> 94.2 us, 301 x 199 p = 1 step 256 -> 242 us.
 __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, double gamma, double igm1, double* out) {
   const double gm1 = dsub(gamma, 1.0);
-  double ir[2], v[2][3], mv[2], bsq[2], prs[2], ip[2], ith[2], bu[2], cf[2], sq[2], f[2][8];
+  double ir[2], v[2][3], mv[2], bsq[2], prs[2], ip[2], ith[2], bu[2], cf[2], f[2][8];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {  // the two sides
     const double* w = h ? wr : wl;
@@ -433,9 +450,8 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
     bu[h] = ddot3(w[4], v[h][0], w[5], v[h][1], w[6], v[h][2]);
     const double bn2 = dmul(w[4], w[4]);
     const double cs = dmul(dmul(gamma, prs[h]), ir[h]), ss = dfma(bsq[h], ir[h], cs);
-    const double disc = fmax(dfma(ss, ss, -dmul(dmul(dmul(4.0, cs), ir[h]), bn2)), TINY);
+    const double disc = at_least(dfma(ss, ss, -dmul(dmul(dmul(4.0, cs), ir[h]), bn2)), TINY);
     cf[h] = sqrt_nr(dmul(0.5, dadd(ss, sqrt_nr(disc))));
-    sq[h] = sqrt_nr(w[0]);
     f[h][0] = w[1];
     f[h][1] = dfma(v[h][0], w[1], -bn2);  // the pressures follow below
     f[h][2] = dfma(v[h][0], w[2], -dmul(w[5], w[4]));
@@ -445,13 +461,14 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
     f[h][6] = dfma(w[6], v[h][0], -dmul(w[4], v[h][2]));
     f[h][7] = dfma(v[h][0], dadd(w[7], dfma(0.5, bsq[h], prs[h])), -dmul(w[4], bu[h]));
   }
-  const double pb = fmin(prs[0], prs[1]);
+  const double pb = at_most(prs[0], prs[1]);
 #pragma unroll
   for (int h = 0; h < 2; ++h) f[h][1] = dadd(f[h][1], dfma(0.5, bsq[h], dsub(prs[h], pb)));
+  const double rho_s = dadd(wl[0], wr[0]);
   double ds;
   {
     const double fp = dmul(dsub(prs[1], prs[0]), rcp_nr(dadd(prs[0], prs[1]))), up = dmul(fp, fp);
-    const double fd = dmul(dsub(wr[0], wl[0]), rcp_nr(dadd(wl[0], wr[0]))), ud = dmul(fd, fd);
+    const double fd = dmul(dsub(wr[0], wl[0]), rcp_nr(rho_s)), ud = dmul(fd, fd);
     double lp = dmul(dadd(fp, fp), series_divisor(up)), ld = dmul(dadd(fd, fd), series_divisor(ud));
     if (up >= 1.4e-4 || ud >= 1.4e-4) {
       if (up >= 1.4e-4) lp = log(dmul(prs[1], ip[0]));
@@ -466,11 +483,12 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
     if (s != 4) d[s] = dsub(f[1][s], f[0][s]);
   }
   d[4] = 0.0;
-  const double isum = rcp_nr(dadd(sq[0], sq[1]));
-  const double vx_roe = dmul(dfma(v[1][0], sq[1], dmul(v[0][0], sq[0])), isum);
-  const double db = dmul(sqrt_nr(dadd(dsq3(j[4], j[5], j[6]), TINY)), isum);
-  const double sl_pp = dsub(dsub(fmin(v[0][0], vx_roe), cf[0]), db);
-  const double sr_pp = dadd(dadd(fmax(v[1][0], vx_roe), cf[1]), db);
+  // Roe's weights with one root, s = sqrt(rho_l rho_r): both quotients over (sqrt rho_l + sqrt rho_r)^2
+  const double s_rho = sqrt_nr(dmul(wl[0], wr[0])), irs = rcp_nr(dfma(2.0, s_rho, rho_s));
+  const double vx_roe = dmul(dfma(s_rho, dadd(v[0][0], v[1][0]), dadd(wl[1], wr[1])), irs);
+  const double db = sqrt_nr(dfma(dsq3(j[4], j[5], j[6]), irs, TINY));
+  const double sl_pp = dsub(dsub(at_most(vx_roe, v[0][0]), cf[0]), db);
+  const double sr_pp = dadd(dadd(at_least(vx_roe, v[1][0]), cf[1]), db);
   // a = sum (v_r - v_l)(w_r - w_l); b = q_r - q_l - sum v (f_r - f_l) - phi (B_r - B_l)_n per side
   const double gg = dmul(gamma, igm1);
   double k[2], b[2], mj[2], bj[2];
@@ -486,12 +504,12 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
   }
   const double da = dadd(dfma(dsub(ith[0], ith[1]), j[7], -dmul(dadd(ds, dsub(k[1], k[0])), j[0])),
                          dadd(dsub(mj[1], mj[0]), dsub(bj[1], bj[0])));
-  const double ia = rcp_nr(dadd(fmax(da, 0.0), 1e-8));
-  const double al = fmax(dmul(b[0], ia), 0.0);
-  const double ar = fmax(dmul(b[1], ia), 0.0);
+  const double ia = rcp_nr(dadd(at_least(da, 0.0), 1e-8));
+  const double al = at_least(dmul(b[0], ia), 0.0);
+  const double ar = at_least(dmul(b[1], ia), 0.0);
   const double aa = sqrt_nr(dfma(al, ar, TINY));
-  const double sl = fmin(fmin(-dadd(ar, aa), sl_pp), 0.0);
-  const double sr = fmax(fmax(dadd(al, aa), sr_pp), 0.0);
+  const double sl = at_most(sl_pp, -dadd(ar, aa));  // (never above zero: ar, aa >= 0)
+  const double sr = at_least(sr_pp, dadd(al, aa));
   const double idsl = rcp_nr(dsub(sr, sl));
   // (sr fl - sl fr)/(sr - sl) from the side with the larger weight, plus the other weight (at most
   // 1/2) times the difference: equal states give exactly their flux, a supersonic face its upwind one

@@ -166,6 +166,14 @@ int init_device_tables(int dev) {
       }
   }
   CK(cudaMemcpyToSymbol(c_deg, tabs, sizeof(tabs)));
+  DegRows rows[MAXP + 1];
+  std::memset(rows, 0, sizeof(rows));
+  for (int p = 1; p <= MAXP; ++p)
+    for (int k = 0, n = p + 1; k < n; ++k) {
+      for (int r = 0; r < n; ++r) rows[p].row[k][r] = tabs[p].D[k + n * ((k + r) % n)];
+      rows[p].iqw[k] = tabs[p].iqw[k];
+    }
+  CK(cudaMemcpyToSymbol(d_rows, rows, sizeof(rows)));
   CK(cudaFuncSetAttribute(residual2_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
   CK(cudaFuncSetAttribute(residual2_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
   CK(cudaFuncSetAttribute(residual2_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
@@ -243,9 +251,9 @@ int res_resident_ctas(int dev) {
 template <int P>
 void launch_residual_retry(mhd_gpu* h, const double* u, double* ut) {
   using L = Res2Layout<P>;
-  const int ntx = (h->nx + L::TX - 1) / L::TX, ntiles = ntx * ((h->ny + L::TY - 1) / L::TY);
-  residual2_persistent<P><<<std::min(ntiles, res_resident_ctas<P>(h->device)), L::NT, L::BYTES, h->stream>>>(
-      u, ut, h->geo, h->ctrl, ST_RECOMPUTE, ntx, ntiles);
+  const int ncol = res2_item_cols<P>(h->nx), nitems = ncol * res2_item_rows<P>(h->ny);
+  residual2_persistent<P><<<std::min(grid1d(nitems, L::NW), res_resident_ctas<P>(h->device)), L::NT, L::BYTES,
+                            h->stream>>>(u, ut, h->geo, h->ctrl, ST_RECOMPUTE, ncol, nitems);
 }
 
 template <int P>
