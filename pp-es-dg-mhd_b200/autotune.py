@@ -49,9 +49,9 @@ GROUPS = {
             3: [(256, 4), (256, 4), (256, 4), (128, 8)],
         },
         "MHD_SIG_CFG": {
-            1: [(8, 8, 3), (8, 8, 4), (8, 4, 4), (8, 8, 3)],
-            2: [(8, 4, 3), (8, 4, 4), (4, 4, 4), (8, 4, 3)],
-            3: [(4, 4, 2), (4, 4, 4), (4, 4, 3), (4, 4, 2)],
+            1: [(16, 4, 4), (8, 8, 4), (8, 8, 5), (16, 4, 4)],
+            2: [(8, 4, 5), (8, 4, 4), (4, 4, 6), (8, 4, 5)],
+            3: [(4, 4, 4), (4, 4, 3), (2, 8, 4), (4, 4, 4)],
         },
     },
 }

@@ -56,13 +56,13 @@ constexpr unsigned FULL_MASK = 0xffffffffu;
 #define MHD_PP_CFG3 256, 4
 #endif
 #ifndef MHD_SIG_CFG1
-#define MHD_SIG_CFG1 8, 8, 3
+#define MHD_SIG_CFG1 16, 4, 4
 #endif
 #ifndef MHD_SIG_CFG2
-#define MHD_SIG_CFG2 8, 4, 3
+#define MHD_SIG_CFG2 8, 4, 5
 #endif
 #ifndef MHD_SIG_CFG3
-#define MHD_SIG_CFG3 4, 4, 2
+#define MHD_SIG_CFG3 4, 4, 4
 #endif
 struct PPParams {
   int NT, MINB;
@@ -743,164 +743,114 @@ __global__ void __launch_bounds__(256) pp_reduce_batched(const InstDesc* __restr
 // face of each (plus the right/top boundary faces on the last tile of a row/column).  The tile
 // and its left/bottom neighbours (and the ghost column/row on the last tiles) are staged in
 // shared memory with coalesced loads; each (face, variable) item then reads two variable blocks.
-// Shared records are padded (NN+1 doubles per variable) against bank conflicts.
+// Shared records take an odd number of doubles per variable (padded where (p+1)^2 is even), so that the
+// eight variables of two neighbouring elements fall in 16 different bank pairs.
 // ---------------------------------------------------------------------------------------------
+// Derivatives along the face of a polynomial given by its values f at the N GLL nodes, in units of the
+// reference coordinate, by the closed form of the interpolant (N = 4: its even part alpha + beta x^2 and
+// odd part gamma x + delta x^3 at +-1, +-1/sqrt 5; 27 operations for the three derivatives against
+// 48 for three products with D).  d1, d2: nodal values of the first and second derivative; d3: the
+// third, a constant (as are d2 at N = 3 and d1 at N = 2, which then stand at index 0 alone).
+template <int N>
+__device__ __forceinline__ void face_derivs(const double* f, double* d1, double* d2, double& d3) {
+  if constexpr (N == 4) {
+    constexpr double R5 = 2.2360679774997896964, I5 = 1.0 / R5;  // sqrt 5 and 1/sqrt 5
+    const double b2 = 1.25 * ((f[0] + f[3]) - (f[1] + f[2]));    // 2 beta
+    const double o = f[3] - f[0], dl = o - R5 * (f[2] - f[1]);   // delta = 0.625 dl
+    const double e1 = I5 * b2;
+    const double q3 = 0.5 * o + 1.25 * dl, q2 = 0.5 * o - 0.25 * dl;  // gamma + 3 delta x^2
+    d1[0] = q3 - b2;
+    d1[1] = q2 - e1;
+    d1[2] = q2 + e1;
+    d1[3] = q3 + b2;
+    d2[0] = b2 - 3.75 * dl;
+    d2[1] = b2 - (3.75 * I5) * dl;
+    d2[2] = b2 + (3.75 * I5) * dl;
+    d2[3] = b2 + 3.75 * dl;
+    d3 = 3.75 * dl;
+  } else if constexpr (N == 3) {
+    d2[0] = (f[0] + f[2]) - 2.0 * f[1];
+    d1[1] = 0.5 * (f[2] - f[0]);
+    d1[0] = d1[1] - d2[0];
+    d1[2] = d1[1] + d2[0];
+  } else {
+    d1[0] = 0.5 * (f[1] - f[0]);
+  }
+}
+// <w/2, |f|> at the N GLL nodes
+template <int N>
+__device__ __forceinline__ double face_l1(const double* f) {
+  if constexpr (N == 4) return (1.0 / 12.0) * (fabs(f[0]) + fabs(f[3])) + (5.0 / 12.0) * (fabs(f[1]) + fabs(f[2]));
+  else if constexpr (N == 3) return (1.0 / 6.0) * (fabs(f[0]) + fabs(f[2])) + (2.0 / 3.0) * fabs(f[1]);
+  else return 0.5 * (fabs(f[0]) + fabs(f[1]));
+}
+
 // One face, either direction.  Rp, Lm = the variable's nodes of the element after and before the
-// face (its first trace, R0, and last trace, RN, along the normal); node (a along the normal, b
-// along the face) sits at a*sn + b*st (x face: sn = 1, st = N; y face: sn = N, st = 1).  sn_h,
-// st_h = 2/h along the normal and along the face; coef[n][t] = (2(n+t)+1) h^(n+t) / (2 max(2p-1,1)
-// n! t!) with h the element size along the normal.  The x face of the reference (DG_solver.f90:
-// 296-343) is this with (R, L, hx, hy); its y face (:360-407) with (T, B, hy, hx): the two loops
-// are the same arithmetic with the roles of the directions exchanged.
+// face; node (a along the normal, b along the face) sits at a*sn + b*st (x face: sn = 1, st = N; y
+// face: sn = N, st = 1).  coef[n][t] = (2(n+t)+1) h^(n+t) / (2 max(2p-1,1) n! t!) with h the element
+// size along the normal, times (2/h)^n (2/h_t)^t, the scales of the derivatives.  The x face of the
+// reference (DG_solver.f90:296-343) is this with (R, L, hx, hy); its y face (:360-407) with (T, B,
+// hy, hx): the two loops are the same arithmetic with the roles of the directions exchanged.
+//
+// The n-th normal derivative is R0[n] . R at the first node of R and RN[n] . L at the last of L, with
+// RN[n][a] = (-1)^n R0[n][N-1-a] (the nodes are symmetric): the jump of an odd (even) order is R0[n]
+// times the sums (differences) R[a] +- L[N-1-a].  Scales applied to the sums of magnitudes, the
+// derivatives along the face in closed form: about 185 operations a face and variable at p = 3
+// (295 as products with the scaled D), in 64 registers, so that one thread takes a whole face where
+// two warps shared it.  With the faces ordered along rows (16 different bank pairs per half-warp):
+// 400 x 400, p = 3 135 -> 75 us, p = 2 63 -> 40, 500 x 500 p = 1 48 -> 34.  Bound by the
+// shared-memory pipe (each node value is read by four faces) and its staging.
 template <int P>
-__device__ __forceinline__ double sigsum_face(const double* Rp, const double* Lm, int sn, int st, double sn_h,
-                                              double st_h, const double* coef) {
+__device__ __forceinline__ double sigsum_face(const double* Rp, const double* Lm, int sn, int st, const double* coef) {
   constexpr int N = P + 1;
   const DegConst& dc = c_deg[P];
-  // J[kk][b] = the jump of the kk-th normal derivative at face node b, formed column by column
-  // (each column of the two variable blocks is read from shared memory once)
-  double sk[N], J[N][N];
-  double snk = 1.0;
-#pragma unroll
-  for (int kk = 0; kk <= P; ++kk) {
-    sk[kk] = snk;
-    snk *= sn_h;
-  }
+  double J[N][N];  // J[n][b] = the jump of the n-th normal derivative at face node b
 #pragma unroll
   for (int b = 0; b < N; ++b) {
-    double cr[N], cl[N];
+    double sum[N], dif[N];
 #pragma unroll
     for (int a = 0; a < N; ++a) {
-      cr[a] = Rp[a * sn + b * st];
-      cl[a] = Lm[a * sn + b * st];
+      const double r = Rp[a * sn + b * st], l = Lm[(N - 1 - a) * sn + b * st];
+      sum[a] = r + l;
+      dif[a] = r - l;
     }
-    // order 0: the rows of D^0 = I pick the end nodes (the sums below give exactly these values)
-    J[0][b] = cr[0] - cl[N - 1];
+    J[0][b] = dif[0];
 #pragma unroll
-    for (int kk = 1; kk <= P; ++kk) {
-      double tr = 0.0, tl = 0.0;
+    for (int n = 1; n <= P; ++n) {
+      const double* x = (n & 1) ? sum : dif;
+      double t = dc.R0[n][0] * x[0];
 #pragma unroll
-      for (int a = 0; a < N; ++a) {
-        tr += dc.R0[kk][a] * cr[a];
-        tl += dc.RN[kk][a] * cl[a];
-      }
-      J[kk][b] = sk[kk] * tr - sk[kk] * tl;
+      for (int a = 1; a < N; ++a) t += dc.R0[n][a] * x[a];
+      J[n][b] = t;
     }
   }
-  double total = 0.0;
+  double total = 0.0, d1[N], d2[N], d3 = 0.0;
 #pragma unroll
-  for (int kk = 0; kk <= P; ++kk) {
-    double jump[N];
-#pragma unroll
-    for (int b = 0; b < N; ++b) jump[b] = J[kk][b];
-#pragma unroll
-    for (int ll = 0; ll <= P; ++ll) {
-      if (ll > P - kk) break;
-      double L1 = 0.0;
-#pragma unroll
-      for (int b = 0; b < N; ++b) L1 += (0.5 * dc.qw[b]) * fabs(jump[b]);
-      total = total + coef[kk * N + ll] * L1;
-      if (ll < P - kk) {  // tangential derivative for the next order
-        double nj[N];
-#pragma unroll
-        for (int a = 0; a < N; ++a) {
-          double acc = 0.0;
-#pragma unroll
-          for (int b = 0; b < N; ++b) acc += (st_h * dc.D[a + N * b]) * jump[b];
-          nj[a] = acc;
-        }
-#pragma unroll
-        for (int a = 0; a < N; ++a) jump[a] = nj[a];
-      }
+  for (int n = 0; n <= P; ++n) {
+    total += coef[n * N] * face_l1<N>(J[n]);
+    if (n < P) {  // orders along the face up to P - n; the last of a degree-P polynomial is a constant
+      face_derivs<N>(J[n], d1, d2, d3);
+      total += coef[n * N + 1] * (N == 2 ? fabs(d1[0]) : face_l1<N>(d1));
+      if (P >= 2 && n + 2 <= P) total += coef[n * N + 2] * (N == 3 ? fabs(d2[0]) : face_l1<N>(d2));
+      if (P == 3 && n == 0) total += coef[3] * fabs(d3);
     }
   }
   return total;
 }
 
-// The part of sigsum_face from the normal-derivative orders KA and KB only (in that order): the two
-// halves {0, P} and {1, P-1} of a face at P = 3, each computed by its own warp (fewer registers,
-// half the dependent chain); the face's value is the sum of the two halves.
-template <int P, int KA, int KB>
-__device__ __forceinline__ double sigsum_face_pair(const double* Rp, const double* Lm, int sn, int st, double sn_h,
-                                                   double st_h, const double* coef) {
-  constexpr int N = P + 1;
-  const DegConst& dc = c_deg[P];
-  constexpr int KS[2] = {KA, KB};
-  double sk[2], J[2][N];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    double snk = 1.0;
-#pragma unroll
-    for (int i = 0; i < KS[h]; ++i) snk *= sn_h;  // sn_h^kk, the running product of sigsum_face
-    sk[h] = snk;
-  }
-#pragma unroll
-  for (int b = 0; b < N; ++b) {
-    double cr[N], cl[N];
-#pragma unroll
-    for (int a = 0; a < N; ++a) {
-      cr[a] = Rp[a * sn + b * st];
-      cl[a] = Lm[a * sn + b * st];
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int kk = KS[h];
-      if (kk == 0) {
-        J[h][b] = cr[0] - cl[N - 1];
-      } else {
-        double tr = 0.0, tl = 0.0;
-#pragma unroll
-        for (int a = 0; a < N; ++a) {
-          tr += dc.R0[kk][a] * cr[a];
-          tl += dc.RN[kk][a] * cl[a];
-        }
-        J[h][b] = sk[h] * tr - sk[h] * tl;
-      }
-    }
-  }
-  double total = 0.0;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int kk = KS[h];
-    double jump[N];
-#pragma unroll
-    for (int b = 0; b < N; ++b) jump[b] = J[h][b];
-#pragma unroll
-    for (int ll = 0; ll <= P; ++ll) {
-      if (ll > P - kk) break;
-      double L1 = 0.0;
-#pragma unroll
-      for (int b = 0; b < N; ++b) L1 += (0.5 * dc.qw[b]) * fabs(jump[b]);
-      total = total + coef[kk * N + ll] * L1;
-      if (ll < P - kk) {  // tangential derivative for the next order (D from the constant bank,
-        double nj[N];     // the scale applied after the sum: no scaled copy of D held in registers)
-#pragma unroll
-        for (int a = 0; a < N; ++a) {
-          double acc = 0.0;
-#pragma unroll
-          for (int b = 0; b < N; ++b) acc += dc.D[a + N * b] * jump[b];
-          nj[a] = st_h * acc;
-        }
-#pragma unroll
-        for (int a = 0; a < N; ++a) jump[a] = nj[a];
-      }
-    }
-  }
-  return total;
-}
-
-// coef[n][t] of sigsum_face for element size h (the reference's running products h^(n+t), n! t!)
+// coef[n][t] of sigsum_face for element size h along the normal (the reference's running products
+// h^(n+t), n! t!) and the derivative scales sn = 2/h, st = 2/h_t
 template <int P>
-__device__ __forceinline__ double sigsum_coef(int n, int t, double h) {
+__device__ __forceinline__ double sigsum_coef(int n, int t, double h, double sn, double st) {
   const int denom_base = 2 * max(2 * P - 1, 1);
   double hp = 1.0;
   int fn = 1, ft = 1;
   for (int i = 0; i < n; ++i) {
-    hp *= h;
+    hp *= h * sn;
     fn *= (i + 1);
   }
   for (int i = 0; i < t; ++i) {
-    hp *= h;
+    hp *= h * st;
     ft *= (i + 1);
   }
   return ((2 * (n + t) + 1) * hp) / (double)(denom_base * fn * ft);
@@ -915,10 +865,9 @@ template <int P>
 struct SigLayout {
   static constexpr int N = P + 1, NN = N * N, EB = 8 * NN;
   static constexpr int TX = SigCfg<P>::TX, TY = SigCfg<P>::TY;
-  static constexpr int VS = NN + 1, ES = 8 * VS;   // padded variable / element record
+  static constexpr int VS = NN | 1, ES = 8 * VS;   // variable / element record: an odd variable stride
   static constexpr int RW = TX + 2, RH = TY + 2;   // staged rectangle (max)
   static constexpr int DOUBLES = RW * RH * ES;
-  static constexpr int NQ = 8 * ((TX + 1) * TY + TX * (TY + 1));  // face-variable items of a tile, at most
 };
 
 
@@ -943,7 +892,6 @@ __device__ __forceinline__ void pp_sigsum_tile(const double* __restrict__ u, con
   __shared__ double s_e[L::DOUBLES];  // face math reads its two variable blocks from here
   __shared__ double s_coef[2 * (P + 1) * (P + 1)];  // x faces (h = hx), then y faces (h = hy)
   __shared__ double s_mm[2][NT / 32][8];              // per warp: max, min of each variable
-  __shared__ double s_part[P == 3 ? 2 * L::NQ : 1];   // P = 3: the two halves of every item
   const int tid = threadIdx.x;
   const int nx = g.nx, ny = g.ny;
   const int i0 = 1 + tile_x * TX, j0 = 1 + tile_y * TY;
@@ -968,7 +916,7 @@ __device__ __forceinline__ void pp_sigsum_tile(const double* __restrict__ u, con
   }
   if (tid < 2 * (P + 1) * (P + 1)) {
     const int d = tid / ((P + 1) * (P + 1)), r = tid - d * (P + 1) * (P + 1), n = r / (P + 1), t = r - n * (P + 1);
-    s_coef[tid] = (n + t <= P) ? sigsum_coef<P>(n, t, d == 0 ? g.hx : g.hy) : 0.0;
+    s_coef[tid] = (n + t <= P) ? sigsum_coef<P>(n, t, d == 0 ? g.hx : g.hy, d == 0 ? g.sxh : g.syh, d == 0 ? g.syh : g.sxh) : 0.0;
   }
   cp_async_wait_all();
   __syncthreads();
@@ -980,8 +928,8 @@ __device__ __forceinline__ void pp_sigsum_tile(const double* __restrict__ u, con
       const double* src = s_e + ((r + 1) * RW + c + 1) * ES + v * VS;
 #pragma unroll
       for (int q = 0; q < NN; ++q) {
-        mx = fmax(mx, src[q]);
-        mn = fmin(mn, src[q]);
+        mx = at_least(src[q], mx);
+        mn = at_most(src[q], mn);
       }
     }
 #pragma unroll
@@ -994,63 +942,22 @@ __device__ __forceinline__ void pp_sigsum_tile(const double* __restrict__ u, con
       s_mm[1][tid >> 5][v] = mn;
     }
   }
-  const double sxh = 2.0 / g.hx, syh = 2.0 / g.hy;
   const int wr = W + right, ht = H + top;  // TX and TY on interior tiles
   const int nfx = H * wr, nfy = W * ht;
-  // face-variable item q: the variable's block of the element before the face, and the output
-  auto item = [&](int q, bool& xf, const double*& lo, double*& dst) {
+  // face-variable items: 8 variables of a face in consecutive threads, faces along a row, so that
+  // 16 threads (2 faces x 8 variables) read 16 different bank pairs
+  for (int q = tid; q < 8 * (nfx + nfy); q += NT) {
     const int v = q & 7, f = q >> 3;
-    xf = f < nfx;
-    if (xf) {  // x face: row r, face c between columns c-1 and c of the tile
-      const int r = (wr == TX) ? f / TX : f / wr, c = f - r * wr;
-      lo = s_e + ((r + 1) * RW + c) * ES + v * VS;
-      dst = so.sig_x + (((long long)(j0 + r - 1) * (nx + 1)) + (i0 + c - 1)) * 8 + v;
-    } else {  // y face: column c, face r between rows r-1 and r of the tile
-      const int f2 = f - nfx;
-      const int c = (ht == TY) ? f2 / TY : f2 / ht, r = f2 - c * ht;
-      lo = s_e + (r * RW + c + 1) * ES + v * VS;
-      dst = so.sig_y + (((long long)(j0 + r - 1) * nx) + (i0 + c - 1)) * 8 + v;
-    }
-  };
-  const int nq = 8 * (nfx + nfy);
-  if constexpr (P == 3) {
-    // two warps per 32 items: the even warps take the orders {0, 3}, the odd ones {1, 2}
-    // (sigsum_face_pair; the warp's half is uniform, so neither diverges); the halves meet in
-    // shared memory and are added in that order
-    static_assert(((NT / 32) & 1) == 0, "warps pair up");
-    for (int it = tid; it < 2 * ((nq + 31) & ~31); it += NT) {
-      const int half = (it >> 5) & 1, q = ((it >> 6) << 5) + (it & 31);
-      if (q < nq) {
-        bool xf;
-        const double* lo;
-        double* dst;
-        item(q, xf, lo, dst);
-        const double* rp = lo + (xf ? ES : RW * ES);
-        const int sn = xf ? 1 : P + 1, st = xf ? P + 1 : 1;
-        const double snh = xf ? sxh : syh, sth = xf ? syh : sxh;
-        const double* cf = s_coef + (xf ? 0 : (P + 1) * (P + 1));
-        s_part[half * L::NQ + q] = half == 0 ? sigsum_face_pair<P, 0, 3>(rp, lo, sn, st, snh, sth, cf)
-                                             : sigsum_face_pair<P, 1, 2>(rp, lo, sn, st, snh, sth, cf);
-      }
-    }
-    __syncthreads();
-    for (int q = tid; q < nq; q += NT) {
-      bool xf;
-      const double* lo;
-      double* dst;
-      item(q, xf, lo, dst);
-      *dst = s_part[q] + s_part[L::NQ + q];
-    }
-  } else {
-    for (int q = tid; q < nq; q += NT) {
-      bool xf;
-      const double* lo;
-      double* dst;
-      item(q, xf, lo, dst);
-      // one call site for both directions (the strides and scales select the direction)
-      *dst = sigsum_face<P>(lo + (xf ? ES : RW * ES), lo, xf ? 1 : P + 1, xf ? P + 1 : 1, xf ? sxh : syh,
-                            xf ? syh : sxh, s_coef + (xf ? 0 : (P + 1) * (P + 1)));
-    }
+    const bool xf = f < nfx;
+    const int f2 = xf ? f : f - nfx, n = xf ? wr : W;
+    const int r = (n == TX) ? f2 / TX : f2 / n, c = f2 - r * n;
+    // the block of the element before the face: left of x face (r, c), below y face (r, c)
+    const double* lo = s_e + ((xf ? (r + 1) * RW + c : r * RW + c + 1)) * ES + v * VS;
+    double* dst = xf ? so.sig_x + (((long long)(j0 + r - 1) * (nx + 1)) + (i0 + c - 1)) * 8 + v
+                     : so.sig_y + (((long long)(j0 + r - 1) * nx) + (i0 + c - 1)) * 8 + v;
+    // one call site for both directions (the strides select the direction)
+    *dst = sigsum_face<P>(lo + (xf ? ES : RW * ES), lo, xf ? 1 : P + 1, xf ? P + 1 : 1,
+                          s_coef + (xf ? 0 : (P + 1) * (P + 1)));
   }
   __syncthreads();
   if (tid < 16) {  // threads 0-7: max of variable tid; 8-15: min of variable tid - 8

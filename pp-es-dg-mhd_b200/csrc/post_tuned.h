@@ -9,7 +9,7 @@
 #define MHD_PP_CFG1 256, 4
 #endif
 #ifndef MHD_SIG_CFG1
-#define MHD_SIG_CFG1 8, 8, 3
+#define MHD_SIG_CFG1 16, 4, 4
 #endif
 //   p=2 MHD_PP_CFG (256, 4); MHD_SIG_CFG (8, 4, 3): 1.6700 ms  <- chosen
 //   p=2 MHD_PP_CFG (256, 4); MHD_SIG_CFG (8, 4, 4): 1.6682 ms
@@ -19,7 +19,7 @@
 #define MHD_PP_CFG2 256, 4
 #endif
 #ifndef MHD_SIG_CFG2
-#define MHD_SIG_CFG2 8, 4, 3
+#define MHD_SIG_CFG2 8, 4, 5
 #endif
 //   p=3 MHD_PP_CFG (256, 4); MHD_SIG_CFG (4, 4, 2): 2.6317 ms
 //   p=3 MHD_PP_CFG (256, 4); MHD_SIG_CFG (4, 4, 4): 2.5707 ms  <- chosen
