@@ -116,11 +116,16 @@ struct Geo {
   int bc_kind;
   int pad_;
   double bc_state[8];
-  const double* ldfA;  // dense LDF nodal operator (2n^2 x 2n^2, column-major), device memory
+  const double* ldfA;  // the LDF operator as loop 1 applies it (tables.h, ldf_table), device memory
   double sxh, syh, igm1;  // 2/hx, 2/hy, 1/(gamma-1) (geo_constants)
 };
 
-// the quotients every thread of the residual would form again
+// doubles of the LDF table of degree p: 2 per node and input slot
+__host__ __device__ constexpr int ldf_table_doubles(int p) {
+  return 2 * (p + 1) * (p + 1) * 2 * ((p + 2) / 2) * ((p + 2) / 2);
+}
+
+// the quotients every thread would form again
 inline void geo_constants(Geo& g) {
   g.sxh = 2.0 / g.hx;
   g.syh = 2.0 / g.hy;
@@ -283,16 +288,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsig
 
 // ---- physics (MHD_PDE.f90 formulas as inlined in DG_solver.f90) -------------------------------
 
-// _macro_prs_ (DG_solver.f90:125)
-__device__ __forceinline__ double prs_of(double rho, double mx, double my, double mz, double bx,
-                                         double by, double bz, double e, double gamma) {
-  return (gamma - 1.0) * (e - 0.5 * ((mx * mx + my * my + mz * mz) / rho + (bx * bx + by * by + bz * bz)));
-}
-// _macro_ent_ (DG_solver.f90:126)
-__device__ __forceinline__ double ent_of(double rho, double prs, double gamma) {
-  return -(rho * (log(prs) - gamma * log(rho)) / (gamma - 1.0));
-}
-
 // Exactly rounded arithmetic for the residual's flux functions: every product, sum and fused
 // multiply-add is written out, so the compiler has no freedom to contract or re-use products
 // differently in different kernels, and every kernel that inlines these functions (single
@@ -331,6 +326,16 @@ __device__ __forceinline__ double sqrt_nr(double x) {
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double h = dmul(x, y), e = dfma(-h, y, 1.0);
   return dfma(h, dmul(e, dfma(0.375, e, 0.5)), h);
+}
+
+// _macro_prs_ (DG_solver.f90:125), its quotient as a product with rcp_nr
+__device__ __forceinline__ double prs_of(double rho, double mx, double my, double mz, double bx,
+                                         double by, double bz, double e, double gamma) {
+  return (gamma - 1.0) * (e - 0.5 * ((mx * mx + my * my + mz * mz) * rcp_nr(rho) + (bx * bx + by * by + bz * bz)));
+}
+// _macro_ent_ (DG_solver.f90:126); igm1 = 1/(gamma-1)
+__device__ __forceinline__ double ent_of(double rho, double prs, double gamma, double igm1) {
+  return -(rho * (log(prs) - gamma * log(rho)) * igm1);
 }
 
 // Four times the entropy-conservative two-point flux along the first direction (ec_flux_x,

@@ -104,8 +104,7 @@ InstLayout inst_layout(int nx, int ny, int p, int R) {
   for (int s = 1; s <= R; ++s) L.ut[s] = take(tb);
   L.u_avg = take(sizeof(double) * 8 * nelg);
   L.staging = take(sb);
-  const size_t n2 = 2 * (size_t)(p + 1) * (p + 1);
-  L.ldfA = take(sizeof(double) * n2 * n2);
+  L.ldfA = take(sizeof(double) * ldf_table_doubles(p));
   L.sig_x = take(sizeof(double) * 8 * (size_t)(nx + 1) * ny);
   L.sig_y = take(sizeof(double) * 8 * (size_t)nx * (ny + 1));
   const size_t te_min = pp_min_chunk();  // the smallest elements-per-CTA of the post-process kernels
@@ -596,7 +595,6 @@ int create_instance(int nx, int ny, int px, int py, int rknstg, double left, dou
   h->ctrl = reinterpret_cast<Ctrl*>(base + L.ctrl);
   const size_t sb = sizeof(double) * (size_t)n_state(h), tb = sizeof(double) * (size_t)n_ut(h);
   const long long nelg = (long long)(nx + 2) * (ny + 2);
-  const int n2 = 2 * h->nn;
   h->ctrl_host = static_cast<Ctrl*>(std::calloc(1, sizeof(Ctrl)));
   if (!h->ctrl_host) {
     free_all(h);
@@ -604,9 +602,9 @@ int create_instance(int nx, int ny, int px, int py, int rknstg, double left, dou
     return MHD_ERR_CUDA;
   }
   if (u0) cudaMemcpyAsync(h->staging, u0, sb, cudaMemcpyHostToDevice, h->stream);
-  double A[32 * 32];
-  tables::ldf_nodal_operator(px, h->hx, h->hy, A);
-  cudaMemcpyAsync(h->ldfA, A, sizeof(double) * n2 * n2, cudaMemcpyHostToDevice, h->stream);
+  double A[ldf_table_doubles(MAXP)];
+  tables::ldf_table(px, h->hx, h->hy, A);
+  cudaMemcpyAsync(h->ldfA, A, sizeof(double) * ldf_table_doubles(px), cudaMemcpyHostToDevice, h->stream);
   // NaN-filled state, as the reference allocates with ieee_signaling_nan (DG_solver.f90:56,68-71)
   for (int s = 0; s <= rknstg; ++s) cudaMemsetAsync(h->u[s], 0xFF, sb, h->stream);
   for (int s = 1; s <= rknstg; ++s) cudaMemsetAsync(h->ut[s], 0xFF, tb, h->stream);

@@ -178,10 +178,31 @@ __device__ __forceinline__ double grp_min(double v) { return grp_reduce<GS>(v, O
 template <int GS>
 __device__ __forceinline__ double grp_max(double v) { return grp_reduce<GS>(v, OpMax{}); }
 
+// Maximum over a group of values that are not negative (NaN counts as zero).  Such doubles order as
+// their bit patterns do, so groups of more than four lanes take the maximum of the upper words and then
+// of the lower words among the lanes that hold it, by the warp's integer reduction (two instead of
+// four exchanges of a double with a comparison each).
+template <int GS>
+__device__ __forceinline__ double grp_max_nonneg(double v) {
+  v = at_least(v, 0.0);
+  if constexpr (GS <= 4) {
+    return grp_max<GS>(v);
+  } else {
+    const GrpLane<GS> gl = grp_lane<GS>();
+    const unsigned all = (0xffffffffu >> (32 - GS)) << (gl.grp * GS);
+    const unsigned mask = gl.idle ? 0xffffffffu << (32 / GS * GS & 31) : all;  // idle lanes among themselves
+    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+    const unsigned mh = __reduce_max_sync(mask, hi);
+    const unsigned ml = __reduce_max_sync(mask, hi == mh ? lo : 0u);
+    return __hiloint2double((int)mh, (int)ml);
+  }
+}
+
 // All eight sums of a[0..7] over each group of GS lanes, in every lane of the group, by a
 // reduce-scatter (each exchange halves the values a lane carries, one lane bit per level: 8
 // exchanges at GS = 16 instead of 8 butterflies of 4) and an all-gather through the group's
-// shared row `row` (8 doubles).  Deterministic, and every lane of a group ends with the same sums
+// shared row `row` (8 doubles, 16-byte aligned; they stay there: the caller's __syncwarp comes before
+// the row is rewritten).  Deterministic, and every lane of a group ends with the same sums
 // (each final sum is formed in one lane pair as x + y and y + x, which IEEE addition makes equal,
 // and read from the one copy in `row`).
 template <int GS>
@@ -217,16 +238,11 @@ __device__ __forceinline__ void grp_sum8(double* a, double* row) {
     for (int i = 0; i < CNT; ++i) row[vb + i] = a[i];
   __syncwarp();
 #pragma unroll
-  for (int v = 0; v < 8; ++v) a[v] = row[v];
-  __syncwarp();  // the row is rewritten next
-}
-
-// a[v] for a lane-dependent v in 0..7, by selects (an indexed read would put a[] in local memory)
-__device__ __forceinline__ double pick8(const double* a, int v) {
-  double r = a[0];
-#pragma unroll
-  for (int q = 1; q < 8; ++q) r = (v == q) ? a[q] : r;
-  return r;
+  for (int v = 0; v < 8; v += 2) {
+    const double2 t = *reinterpret_cast<const double2*>(row + v);
+    a[v] = t.x;
+    a[v + 1] = t.y;
+  }
 }
 
 __device__ __forceinline__ double node_prs(const double* x, double gamma) {
@@ -299,7 +315,7 @@ __device__ __forceinline__ double limit_group(double* x, const double* avg, bool
   // entropy-offset limiter (DG_solver.f90:606-633)
   if (ent_offset) {
     const bool use = active && !cell_ent_nan[ce];
-    const double nw = grp_sum<GS>(use ? wq * ent_of(x[0], fmax(node_prs(x, gamma), PP_EPS), gamma) : 0.0);
+    const double nw = grp_sum<GS>(use ? wq * ent_of(x[0], at_least(node_prs(x, gamma), PP_EPS), gamma, g.igm1) : 0.0);
     if (use) {
       const double old = cell_ent_DG[ce], eavg = cell_ent_FV[ce];
       if (nw > old) {
@@ -311,13 +327,13 @@ __device__ __forceinline__ double limit_group(double* x, const double* avg, bool
     }
   }
   // cell entropy (DG_solver.f90:635-649)
-  if (comput_ent) return grp_sum<GS>(active ? wq * ent_of(x[0], fmax(node_prs(x, gamma), PP_EPS), gamma) : 0.0);
+  if (comput_ent) return grp_sum<GS>(active ? wq * ent_of(x[0], at_least(node_prs(x, gamma), PP_EPS), gamma, g.igm1) : 0.0);
   return 0.0;
 }
 
 // ---------------------------------------------------------------------------------------------
 // loop 1 for one chunk of TE consecutive element blocks of the ghosted grid (one contiguous run of
-// memory).  s_A = the LDF operator in shared memory, in output-row pairs (load_ldf); s_red = CTA
+// memory).  s_A = the LDF table in shared memory (load_ldf); s_red = CTA
 // scratch of TE * 8 doubles for the chunk sums, which a caller either alternates between two such
 // buffers from chunk to chunk or protects with a barrier after the call (one barrier per chunk
 // here, between the writes of s_red and the reads).
@@ -496,7 +512,13 @@ __device__ __forceinline__ void pp_avg_ldf_chunk(double* __restrict__ u, double*
   double avg[8];
 #pragma unroll
   for (int v = 0; v < 8; ++v) avg[v] = w * x[v];
-  grp_sum8<GS>(avg, s_ldf + (warp * G + grp) * (N2 + 2));
+  double* row = s_ldf + (warp * G + grp) * (N2 + 2);
+  grp_sum8<GS>(avg, row);
+  // the averages this lane stores below: variables node, node + GS, ...
+  double mine[GS >= 8 ? 1 : 8 / GS];
+#pragma unroll
+  for (int v0 = 0; v0 < 8; v0 += GS) mine[v0 / GS] = row[(node + v0) & 7];
+  __syncwarp();  // the row is rewritten next
   // admissibility of the average (DG_solver.f90:186-193): an inadmissible element is left unwritten
   if (valid) {
     const double prs = prs_of(avg[0], avg[1], avg[2], avg[3], avg[4], avg[5], avg[6], avg[7], gamma);
@@ -505,59 +527,78 @@ __device__ __forceinline__ void pp_avg_ldf_chunk(double* __restrict__ u, double*
       valid = inner = false;
     }
   }
-  // cell entropies for the entropy-offset limiter (DG_solver.f90:195-224)
-  if (ent_offset) {
-    const double pq = act ? node_prs(x, gamma) : 0.0;
-    const bool okq = !act || (x[0] >= PP_EPS && pq >= PP_EPS);
-    const double okall = grp_min<GS>(okq ? 1.0 : 0.0);
-    const double ce = grp_sum<GS>((act && okall > 0.5) ? 0.25 * g.hx * g.hy * dc.qw[k] * dc.qw[l] * ent_of(x[0], pq, gamma) : 0.0);
-    if (valid && node == 0) {
-      const double prs = prs_of(avg[0], avg[1], avg[2], avg[3], avg[4], avg[5], avg[6], avg[7], gamma);
-      cell_ent_FV[e] = ent_of(avg[0], prs, gamma);
-      cell_ent_DG[e] = okall > 0.5 ? ce : 0.0;
-      cell_ent_nan[e] = okall > 0.5 ? 0 : 1;
-    }
-  }
-  // LDF projection of (Bx - avg, By - avg) with the dense nodal operator: this lane forms the
-  // outputs at its node (rows `node` and NN + node); the inputs come from the group's lanes
-  if (apply_ldf) {  // the group's (Bx, By) - avg pass through a padded per-group shared row
-    double* sb = s_ldf + (warp * G + grp) * (N2 + 2);
-    if (nd) {
-      sb[node] = x[4] - avg[4];
-      sb[NN + node] = x[5] - avg[5];
-    }
-    __syncwarp();
-    double ox = 0.0, oy = 0.0;
-    if (nd) {
-      // s_A holds (row node, row NN + node) of column m as one pair at m * NN + node (load_ldf),
-      // and the input row is read two entries at a time; the sums run over m in order
-      const double2* a2 = reinterpret_cast<const double2*>(s_A) + node;
-      const double2* b2 = reinterpret_cast<const double2*>(sb);
+  if (valid)
 #pragma unroll
-      for (int m = 0; m < N2; m += 2) {
-        const double2 b = b2[m >> 1];
-        const double2 a0 = a2[m * NN], a1 = a2[(m + 1) * NN];
-        ox += a0.x * b.x;
-        oy += a0.y * b.x;
-        ox += a1.x * b.y;
-        oy += a1.y * b.y;
-      }
-    }
-    __syncwarp();  // the row is rewritten by the next chunk
-    if (valid) {
-      x[4] = ox + avg[4];
-      x[5] = oy + avg[5];
-    }
-  }
+    for (int v0 = 0; v0 < 8; v0 += GS)
+      if (node + v0 < 8) u_avg[e * 8 + node + v0] = mine[v0 / GS];
   if (NEEDG && need_global) {
     // chunk sum of (hx*hy)*avg over interior elements in element order (DG_solver.f90:227-229)
     if (el < TE)
 #pragma unroll
       for (int v0 = 0; v0 < 8; v0 += GS)
-        if (node + v0 < 8) s_red[el * 8 + node + v0] = inner ? (g.hx * g.hy) * pick8(avg, node + v0) : 0.0;
+        if (node + v0 < 8) s_red[el * 8 + node + v0] = inner ? (g.hx * g.hy) * mine[v0 / GS] : 0.0;
+  }
+  // cell entropies for the entropy-offset limiter (DG_solver.f90:195-224)
+  if (ent_offset) {
+    const double pq = act ? node_prs(x, gamma) : 0.0;
+    const bool okq = !act || (x[0] >= PP_EPS && pq >= PP_EPS);
+    const double okall = grp_min<GS>(okq ? 1.0 : 0.0);
+    const double ce = grp_sum<GS>((act && okall > 0.5) ? 0.25 * g.hx * g.hy * dc.qw[k] * dc.qw[l] * ent_of(x[0], pq, gamma, g.igm1) : 0.0);
+    if (valid && node == 0) {
+      const double prs = prs_of(avg[0], avg[1], avg[2], avg[3], avg[4], avg[5], avg[6], avg[7], gamma);
+      cell_ent_FV[e] = ent_of(avg[0], prs, gamma, g.igm1);
+      cell_ent_DG[e] = okall > 0.5 ? ce : 0.0;
+      cell_ent_nan[e] = okall > 0.5 ? 0 : 1;
+    }
+  }
+  // LDF projection of (Bx - avg, By - avg), on the sums and differences of mirror nodes (tables.h,
+  // ldf_table): butterflies along x and y, this lane's output place from at most 2 M^2 input places
+  // through the group's row, butterflies back.  The shared-memory pipe bounds this kernel, and the
+  // dense operator (2n^2 products an output) read its rows from there: 400^2 without / with the OEDG
+  // sums, p = 3: 92 -> 75 / 90 -> 61 us, p = 2: 77 -> 70 / 70 -> 61 us; p = 1, 500^2: 38.5 -> 37.7 us.
+  if (apply_ldf) {
+    constexpr int M = (N + 1) / 2;
+    const int gb = lane - node;  // the group's first lane
+    const int mx = nd ? gb + (N - 1 - k) + N * l : lane, my = nd ? gb + k + N * (N - 1 - l) : lane;
+    const double sx = 2 * k < N - 1 ? 1.0 : (2 * k == N - 1 ? 0.0 : -1.0);
+    const double sy = 2 * l < N - 1 ? 1.0 : (2 * l == N - 1 ? 0.0 : -1.0);
+    double bx = x[4] - avg[4], by = x[5] - avg[5];
+    bx = __fma_rn(sx, __shfl_sync(FULL_MASK, bx, mx), bx);
+    by = __fma_rn(sx, __shfl_sync(FULL_MASK, by, mx), by);
+    bx = __fma_rn(sy, __shfl_sync(FULL_MASK, bx, my), bx);
+    by = __fma_rn(sy, __shfl_sync(FULL_MASK, by, my), by);
+    double2* in = reinterpret_cast<double2*>(row);
+    if (nd) in[node] = make_double2(bx, by);
+    __syncwarp();
+    double ox = 0.0, oy = 0.0;
+    if (nd) {
+      const double2* w = reinterpret_cast<const double2*>(s_A) + node;
+      const bool px = 2 * k > N - 1, py = 2 * l > N - 1;  // the parity of this lane's place
+#pragma unroll
+      for (int jy = 0; jy < M; ++jy)
+#pragma unroll
+        for (int jx = 0; jx < M; ++jx) {
+          const int s = jx + M * jy;
+          const double2 c = w[s * NN], f = in[(px ? N - 1 - jx : jx) + N * (py ? N - 1 - jy : jy)];
+          ox = __fma_rn(c.x, f.x, ox);
+          oy = __fma_rn(c.y, f.y, oy);
+          const double2 d = w[(s + M * M) * NN], h = in[(px ? jx : N - 1 - jx) + N * (py ? jy : N - 1 - jy)];
+          ox = __fma_rn(d.x, h.y, ox);
+          oy = __fma_rn(d.y, h.x, oy);
+        }
+    }
+    __syncwarp();  // the row is rewritten by the next chunk
+    ox = __fma_rn(-sy, __shfl_sync(FULL_MASK, ox, my), ox);
+    oy = __fma_rn(-sy, __shfl_sync(FULL_MASK, oy, my), oy);
+    ox = __fma_rn(-sx, __shfl_sync(FULL_MASK, ox, mx), ox);
+    oy = __fma_rn(-sx, __shfl_sync(FULL_MASK, oy, mx), oy);
+    if (valid) {
+      x[4] = ox + avg[4];
+      x[5] = oy + avg[5];
+    }
   }
   bool neg = false, scaled = false;
-  if (limit) {
+  if (!NEEDG && limit) {  // (the OEDG form is never fused: its damping comes first)
     __syncwarp();  // the group's lane 0 wrote the cell entropies limit_group reads
     limit_group<P>(x, avg, inner && nd, inner && node == 0, node, e, g, ctrl, ent_offset, 0, cell_ent_DG, cell_ent_FV,
                    cell_ent_nan, &neg, &scaled);
@@ -577,14 +618,11 @@ __device__ __forceinline__ void pp_avg_ldf_chunk(double* __restrict__ u, double*
       u[e * EB + 5 * NN + node] = x[5];
     }
   }
-  if (valid)
-#pragma unroll
-    for (int v0 = 0; v0 < 8; v0 += GS)
-      if (node + v0 < 8) u_avg[e * 8 + node + v0] = pick8(avg, node + v0);
   if (NEEDG && need_global) {
     __syncthreads();
     if (tid < 8) {
       double sacc = 0.0;
+#pragma unroll 4
       for (int q = 0; q < ne; ++q) sacc = sacc + s_red[q * 8 + tid];
       partial_out[tid] = sacc;
     }
@@ -594,14 +632,7 @@ __device__ __forceinline__ void pp_avg_ldf_chunk(double* __restrict__ u, double*
 
 template <int P>
 __device__ __forceinline__ void load_ldf(const double* __restrict__ A, double* s_A) {
-  constexpr int N2 = PPCfg<P>::N2;
-  constexpr int NN = PPCfg<P>::NN;
-  // pair (A[node][m], A[NN + node][m]) at m * NN + node; A is stored column-major (row + N2 * m)
-  for (int it = threadIdx.x; it < N2 * NN; it += PPCfg<P>::NT) {
-    const int m = it / NN, node = it - m * NN;
-    s_A[2 * it] = __ldg(A + node + N2 * m);
-    s_A[2 * it + 1] = __ldg(A + NN + node + N2 * m);
-  }
+  for (int it = threadIdx.x; it < ldf_table_doubles(P); it += PPCfg<P>::NT) s_A[it] = __ldg(A + it);
 }
 
 // one CTA walks chunks blockIdx.x, blockIdx.x + gridDim.x, ... (the LDF operator is loaded once).
@@ -614,7 +645,7 @@ __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB)
                       double* __restrict__ cell_ent_DG, double* __restrict__ cell_ent_FV,
                       unsigned char* __restrict__ cell_ent_nan, int limit, int nchunks, Stage1Src s1) {
   using C = PPCfg<P>;
-  __shared__ __align__(16) double s_A[C::N2 * C::N2];
+  __shared__ __align__(16) double s_A[ldf_table_doubles(P)];
   __shared__ __align__(16) double s_ldf[C::TE * (C::N2 + 2)];
   __shared__ double s_red[2 * C::TE * 8];  // chunk sums, two buffers used in turn
   __shared__ __align__(16) double s_pf[(C::NT / 32) * 2 * C::G * C::EB];  // per warp: u (or u_con), k1
@@ -662,7 +693,7 @@ __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB > 3 ? 3 : PPCfg<P
                        const int* __restrict__ nwork, const int* __restrict__ ninst, int slot, int gate,
                        int stage1) {
   using C = PPCfg<P>;
-  __shared__ __align__(16) double s_A[C::N2 * C::N2];
+  __shared__ __align__(16) double s_A[ldf_table_doubles(P)];
   __shared__ __align__(16) double s_ldf[C::TE * (C::N2 + 2)];
   __shared__ double s_red[C::TE * 8];  // chunk sums (the loop's barriers protect it)
   __shared__ int s_cnt;
@@ -1050,27 +1081,33 @@ __device__ __forceinline__ void pp_limit_segment(const LimitIO& io, const Geo& g
   const double gamma = g.gamma;
   double x[8], avg[8];
 #pragma unroll
-  for (int v = 0; v < 8; ++v) {
-    x[v] = act ? io.u[e * EB + v * NN + node] : 0.0;
-    avg[v] = inside ? io.u_avg[e * 8 + v] : 1.0;
+  for (int v = 0; v < 8; ++v) x[v] = act ? io.u[e * EB + v * NN + node] : 0.0;
+#pragma unroll
+  for (int v = 0; v < 8; v += 2) {
+    const double2 t = inside ? *reinterpret_cast<const double2*>(io.u_avg + e * 8 + v) : make_double2(1.0, 1.0);
+    avg[v] = t.x;
+    avg[v + 1] = t.y;
   }
+  // Instructions bound this kernel (most of them 64-bit), so quotients are products with rcp_nr, roots are
+  // sqrt_nr, and a maximum of values that are not negative goes through the integer reduction: 98 -> 88 us
+  // at p = 3, 76 -> 67 us at p = 2 (400^2), 48 -> 41 us at p = 1 (500^2).
   if (io.apply_oedg) {  // DG_solver.f90:448-524
     double sx = 0.0, sy = 0.0;
     if (act) {
-      const double rho = fmax(x[0], PP_EPS);
-      const double ir = 1.0 / rho;
+      const double rho = at_least(x[0], PP_EPS);
+      const double ir = rcp_nr(rho);
       const double vx = ir * x[1], vy = ir * x[2];
       const double ek = 0.5 * ir * (x[1] * x[1] + x[2] * x[2] + x[3] * x[3]);
       const double bx = x[4], by = x[5], bz = x[6];
       const double bsq = bx * bx + by * by + bz * bz;
-      const double pf = fmax((gamma - 1.0) * (x[7] - (ek + 0.5 * bsq)), PP_EPS);
+      const double pf = at_least((gamma - 1.0) * (x[7] - (ek + 0.5 * bsq)), PP_EPS);
       const double cs = gamma * pf * ir, ss = cs + bsq * ir, sqsq = ss * ss, coef = 4.0 * cs * ir;
-      sx = fabs(vx) + sqrt(0.5 * fmax(ss + sqrt(fmax(sqsq - coef * (bx * bx), 0.0)), 0.0));
-      sy = fabs(vy) + sqrt(0.5 * fmax(ss + sqrt(fmax(sqsq - coef * (by * by), 0.0)), 0.0));
+      sx = fabs(vx) + sqrt_nr(0.5 * at_least(ss + sqrt_nr(at_least(sqsq - coef * (bx * bx), TINY)), TINY));
+      sy = fabs(vy) + sqrt_nr(0.5 * at_least(ss + sqrt_nr(at_least(sqsq - coef * (by * by), TINY)), TINY));
     }
-    const double mx = grp_max<GS>(sx), my = grp_max<GS>(sy);
+    const double mx = grp_max_nonneg<GS>(sx), my = grp_max_nonneg<GS>(sy);
     // lane `node` of the group forms delta_v for v = node, node + GS, ... from the element's four faces
-    double d = -1.0e308;
+    double d = 0.0;
     if (inside) {
       const int i = i0 + el;
       const long long fxl = ((long long)(j - 1) * (nx + 1) + (i - 1)) * 8;
@@ -1079,16 +1116,15 @@ __device__ __forceinline__ void pp_limit_segment(const LimitIO& io, const Geo& g
       const Ctrl* ctrl = io.ctrl;
       const double* sig_x = io.sig_x;
       const double* sig_y = io.sig_y;
+      const double wx = 0.5 * g.sxh * mx, wy = 0.5 * g.syh * my;
       for (int v = node; v < 8; v += GS) {
         const double gs = ctrl->u_avg_global[v];
-        const double uv = fmax(0.0, fmax(ord_dec(ctrl->umax_bits[v]) - gs, gs - ord_dec(ctrl->umin_bits[v])));
-        double dv = 0.0;
+        const double uv = at_least(fmax(ord_dec(ctrl->umax_bits[v]) - gs, gs - ord_dec(ctrl->umin_bits[v])), 0.0);
         if (uv > OEDG_EPS)
-          dv = ((mx / g.hx) * (sig_x[fxl + v] + sig_x[fxl + 8 + v]) + (my / g.hy) * (sig_y[fyb + v] + sig_y[fyt + v])) / uv;
-        d = fmax(d, dv);
+          d = at_least((wx * (sig_x[fxl + v] + sig_x[fxl + 8 + v]) + wy * (sig_y[fyb + v] + sig_y[fyt + v])) * rcp_nr(uv), d);
       }
     }
-    const double dmax = grp_max<GS>(d);
+    const double dmax = grp_max_nonneg<GS>(d);
     const double theta = exp(-io.oedg_dt * dmax);
     if (act)
 #pragma unroll
@@ -1105,13 +1141,15 @@ __device__ __forceinline__ void pp_limit_segment(const LimitIO& io, const Geo& g
       if (!io.accept_only) io.u[e * EB + v * NN + node] = x[v];
       if (io.accept_dst) io.accept_dst[e * EB + v * NN + node] = x[v];
     }
-  if (io.comput_ent) {  // chunk partial in element order
+  if (io.comput_ent) {  // chunk partial in a fixed order
     if (inside && node == 0) s_ent[el] = ce;
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0) {
       double tot = 0.0;
-      for (int q = 0; q < ne; ++q) tot = tot + s_ent[q];
-      *io.ent_out = tot;
+      for (int q = lane; q < ne; q += 32) tot = tot + s_ent[q];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) tot = tot + __shfl_xor_sync(FULL_MASK, tot, o);
+      if (lane == 0) *io.ent_out = tot;
     }
   }
 }

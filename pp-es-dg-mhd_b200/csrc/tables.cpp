@@ -311,5 +311,41 @@ int ldf_nodal_operator(int p, double hx, double hy, double* A) {
   return 0;
 }
 
+int ldf_table(int p, double hx, double hy, double* out) {
+  if (p < 1 || p > 3) return -1;
+  double A[32 * 32];
+  if (ldf_nodal_operator(p, hx, hy, A)) return -1;
+  const int n = p + 1, nn = n * n, n2 = 2 * nn, M = (n + 1) / 2;
+  // y, the sums and differences: y_k = f_k + f_{p-k} at k < p-k, f_k - f_{p-k} at k > p-k, f_k in the
+  // middle; back: f_k = (y_k - y_{p-k})/2, (y_k + y_{p-k})/2, y_k.  The output's forward map and the
+  // input's way back each touch a place and its mirror image in either direction.
+  auto half = [&](int k) { return 2 * k == p ? 1.0L : 0.5L; };
+  auto fwd = [&](int k, int m) { return m == 0 || 2 * k < p ? 1.0L : (2 * k == p ? 0.0L : -1.0L); };  // of f_k (m = 0), f_{p-k}
+  auto back = [&](int k, int m) { return m == 0 || 2 * k < p ? half(k) : (2 * k == p ? 0.0L : -half(k)); };  // y_k in f_k, f_{p-k}
+  // weight of input place (field b, node kj, lj) for output place (field c, node k, l)
+  auto weight = [&](int c, int k, int l, int b, int kj, int lj) {
+    ld w = 0.0L;
+    for (int m = 0; m < 16; ++m) {
+      const int a = m & 1, d = m >> 1 & 1, e = m >> 2 & 1, f = m >> 3;
+      const int r = (a ? p - k : k) + n * (d ? p - l : l), t = (e ? p - kj : kj) + n * (f ? p - lj : lj);
+      w += fwd(k, a) * fwd(l, d) * back(kj, e) * back(lj, f) * (ld)A[(c * nn + r) + (size_t)n2 * (b * nn + t)];
+    }
+    return (double)(half(k) * half(l) * w);
+  };
+  for (int q = 0; q < nn; ++q) {
+    const int k = q % n, l = q / n;
+    const bool ox = 2 * k > p, oy = 2 * l > p;  // the place holds an odd part
+    for (int s = 0; s < 2 * M * M; ++s) {
+      const bool other = s >= M * M, px = ox != other, py = oy != other;  // parity of the input places
+      const int jx = (s % (M * M)) % M, jy = (s % (M * M)) / M;
+      const int kj = px ? p - jx : jx, lj = py ? p - jy : jy;
+      const bool there = (2 * kj > p) == px && (2 * lj > p) == py;  // (an odd part has one place fewer at p = 2)
+      for (int c = 0; c < 2; ++c)
+        out[2 * (s * nn + q) + c] = there ? weight(c, k, l, other ? 1 - c : c, kj, lj) : 0.0;
+    }
+  }
+  return 0;
+}
+
 }  // namespace tables
 }  // namespace mhd
