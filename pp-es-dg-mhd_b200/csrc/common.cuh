@@ -125,6 +125,23 @@ __host__ __device__ constexpr int ldf_table_doubles(int p) {
   return 2 * (p + 1) * (p + 1) * 2 * ((p + 2) / 2) * ((p + 2) / 2);
 }
 
+// Launch of a kernel of a chain, each of which waits by grid_begin.  `early`: its CTAs may start while
+// its predecessor in the stream still runs.
+template <typename... K, typename... A>
+void launch_next(cudaStream_t st, bool early, dim3 grid, int block, size_t smem, void (*kernel)(K...), A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+
 // the quotients every thread would form again
 inline void geo_constants(Geo& g) {
   g.sxh = 2.0 / g.hx;
@@ -245,6 +262,15 @@ inline double ord_dec_host(unsigned long long e) {
 
 __device__ __forceinline__ bool gate_open(const Ctrl* c, int gate) {
   return gate < 0 || c->state == gate;
+}
+
+// In every kernel that launch_next may launch, before its first read of anything a kernel writes: wait
+// until the kernels before it in the stream have completed and their writes are visible, then let the next
+// one's CTAs take their places as this kernel's leave theirs.  Every thread of every CTA waits, also
+// those with nothing to do, so that a kernel's completion implies that of all before it.
+__device__ __forceinline__ void grid_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // ---- asynchronous bulk copies global -> shared (sm_90+ cp.async.bulk, completed on an mbarrier) ---

@@ -216,11 +216,19 @@ int enter(const mhd_gpu* h) {
 }
 
 // ---- launchers ---------------------------------------------------------------------------
+// Kernels of a small state are over in a few microseconds each, a large part of which is the start of their
+// CTAs: there each kernel is launched while its predecessor runs.  On a large state the early CTAs take
+// slots and shared memory from the predecessor's last wave instead.  A step of Orszag-Tang, SSP-RK(3,3),
+// without -> with (us): p = 1, 256^2 (0.26 million nodes): 218 -> 205; p = 3, 140^2 (0.31): 219 -> 210; p = 3,
+// 200^2 (0.64): 338 -> 332; p = 2, 320^2 (0.92): 526 -> 528; p = 1, 512^2 (1.05): 539 -> 547; p = 2, 400^2 (1.44):
+// 749 -> 774.
+bool early_launch(const mhd_gpu* h) { return (long long)h->nx * h->ny * h->nn <= 3LL << 18; }
+
 template <int P>
 void launch_bc(mhd_gpu* h, double* u, int gate) {
   constexpr int EB = 8 * (P + 1) * (P + 1);
   const long long n = 2LL * (h->nx + h->ny) * EB;
-  bc_kernel<P><<<grid1d(n, 256), 256, 0, h->stream>>>(u, h->geo, h->ctrl, gate);
+  launch_next(h->stream, early_launch(h), grid1d(n, 256), 256, 0, bc_kernel<P>, u, h->geo, h->ctrl, gate);
 }
 
 // ug: the array whose ghost ring the boundary halos come from (nullptr: u's own)
@@ -229,7 +237,7 @@ void launch_residual(mhd_gpu* h, const double* u, double* ut, int gate, StageCom
                      const double* ug = nullptr) {
   using L = Res2Layout<P>;
   dim3 grid((h->nx + L::TX - 1) / L::TX, (h->ny + L::TY - 1) / L::TY);
-  residual2_kernel<P><<<grid, L::NT, L::BYTES, h->stream>>>(u, ug ? ug : u, ut, h->geo, h->ctrl, gate, sc);
+  launch_next(h->stream, early_launch(h), grid, L::NT, L::BYTES, residual2_kernel<P>, u, ug ? ug : u, ut, h->geo, h->ctrl, gate, sc);
 }
 
 // the re-try residual of a try (gate ST_RECOMPUTE, usually closed): a persistent grid of the CTAs
@@ -251,18 +259,18 @@ template <int P>
 void launch_residual_retry(mhd_gpu* h, const double* u, double* ut) {
   using L = Res2Layout<P>;
   const int ncol = res2_item_cols<P>(h->nx), nitems = ncol * res2_item_rows<P>(h->ny);
-  residual2_persistent<P><<<std::min(grid1d(nitems, L::NW), res_resident_ctas<P>(h->device)), L::NT, L::BYTES,
-                            h->stream>>>(u, ut, h->geo, h->ctrl, ST_RECOMPUTE, ncol, nitems);
+  launch_next(h->stream, early_launch(h), std::min(grid1d(nitems, L::NW), res_resident_ctas<P>(h->device)), L::NT, L::BYTES,
+              residual2_persistent<P>, u, ut, h->geo, h->ctrl, ST_RECOMPUTE, ncol, nitems);
 }
 
 template <int P>
 void launch_combine(mhd_gpu* h, int stage, const double* dt_ptr, double dt, int gate) {
   constexpr int EB = 8 * (P + 1) * (P + 1);
   const long long n = (long long)h->nx * h->ny * EB;
-  combine_kernel<EB><<<grid1d(n, 256), 256, 0, h->stream>>>(
-      h->u[0], h->u[1], h->R >= 2 ? h->u[2] : nullptr, h->R >= 3 ? h->u[3] : nullptr, h->R >= 4 ? h->u[4] : nullptr,
-      h->ut[1], h->R >= 2 ? h->ut[2] : nullptr, h->R >= 3 ? h->ut[3] : nullptr, h->R >= 4 ? h->ut[4] : nullptr,
-      h->R >= 5 ? h->ut[5] : nullptr, h->u[stage], h->nx, h->ny, h->R, stage, dt_ptr, dt, h->ctrl, gate);
+  launch_next(h->stream, early_launch(h), grid1d(n, 256), 256, 0, combine_kernel<EB>,
+              h->u[0], h->u[1], h->R >= 2 ? h->u[2] : nullptr, h->R >= 3 ? h->u[3] : nullptr, h->R >= 4 ? h->u[4] : nullptr,
+              h->ut[1], h->R >= 2 ? h->ut[2] : nullptr, h->R >= 3 ? h->ut[3] : nullptr, h->R >= 4 ? h->ut[4] : nullptr,
+              h->R >= 5 ? h->ut[5] : nullptr, h->u[stage], h->nx, h->ny, h->R, stage, dt_ptr, dt, h->ctrl, gate);
 }
 
 // post_process on slot `slot` (everything but the control-block reset and the host read-back)
@@ -281,14 +289,14 @@ void launch_post(mhd_gpu* h, int slot, int apply_oedg, int apply_ldf, const doub
   const int limit_in_loop1 = fuse && !apply_oedg && !comput_ent && !accept_dst;
   if (apply_oedg) {
     const int grid1 = std::min(nb1, pp_resident_ctas<P, true>(h->device));
-    pp_avg_ldf_kernel<P, true><<<grid1, PPCfg<P>::NT, 0, h->stream>>>(h->u[slot], h->u_avg, h->geo, h->ctrl, gate, apply_ldf,
-                                                                1, ent_offset, h->partial, h->cell_ent_DG,
-                                                                h->cell_ent_FV, h->cell_ent_nan, limit_in_loop1, nb1, s1);
+    launch_next(h->stream, early_launch(h), grid1, PPCfg<P>::NT, 0, pp_avg_ldf_kernel<P, true>, h->u[slot],
+                h->u_avg, h->geo, h->ctrl, gate, apply_ldf, 1, ent_offset, h->partial, h->cell_ent_DG, h->cell_ent_FV, h->cell_ent_nan, limit_in_loop1,
+                nb1, s1);
   } else {
     const int grid1 = std::min(nb1, pp_resident_ctas<P, false>(h->device));
-    pp_avg_ldf_kernel<P, false><<<grid1, PPCfg<P>::NT, 0, h->stream>>>(h->u[slot], h->u_avg, h->geo, h->ctrl, gate, apply_ldf,
-                                                                 0, ent_offset, h->partial, h->cell_ent_DG,
-                                                                 h->cell_ent_FV, h->cell_ent_nan, limit_in_loop1, nb1, s1);
+    launch_next(h->stream, early_launch(h), grid1, PPCfg<P>::NT, 0, pp_avg_ldf_kernel<P, false>, h->u[slot],
+                h->u_avg, h->geo, h->ctrl, gate, apply_ldf, 0, ent_offset, h->partial, h->cell_ent_DG, h->cell_ent_FV, h->cell_ent_nan, limit_in_loop1,
+                nb1, s1);
   }
   if (limit_in_loop1) return;
   if (apply_oedg) {  // the global sums (one CTA) and the face indicators are independent: fork/join
@@ -297,16 +305,20 @@ void launch_post(mhd_gpu* h, int slot, int apply_oedg, int apply_ldf, const doub
     pp_reduce_kernel<<<1, 256, 0, h->side_stream>>>(h->partial, nb1, h->ctrl, gate);
     cudaEventRecord(h->ev_join, h->side_stream);
     const dim3 gs((h->nx + SigCfg<P>::TX - 1) / SigCfg<P>::TX, (h->ny + SigCfg<P>::TY - 1) / SigCfg<P>::TY);
-    pp_sigsum_kernel<P><<<gs, 256, 0, h->stream>>>(h->u[slot], h->geo, h->ctrl, gate, h->sig_x, h->sig_y);
+    launch_next(h->stream, early_launch(h), gs, 256, 0, pp_sigsum_kernel<P>, h->u[slot], h->geo, h->ctrl, gate, h->sig_x, h->sig_y);
     cudaStreamWaitEvent(h->stream, h->ev_join, 0);
   }
   dim3 g3 = pp_grid_limit<P>(h);
-  pp_limit_kernel<P><<<g3, PPCfg<P>::NT, 0, h->stream>>>(h->u[slot], h->u_avg, h->geo, h->ctrl, gate, apply_oedg, dt_ptr,
-                                                   oedg_dt, ent_offset, comput_ent, h->sig_x, h->sig_y,
-                                                   h->cell_ent_DG, h->cell_ent_FV, h->cell_ent_nan,
-                                                   h->ent_partial, accept_dst, accept_only);
+  const auto limit = [&](auto... args) {
+    if (apply_oedg)  // after the join: a plain launch, which waits for both
+      pp_limit_kernel<P><<<g3, PPCfg<P>::NT, 0, h->stream>>>(args...);
+    else
+      launch_next(h->stream, early_launch(h), g3, PPCfg<P>::NT, 0, pp_limit_kernel<P>, args...);
+  };
+  limit(h->u[slot], h->u_avg, h->geo, h->ctrl, gate, apply_oedg, dt_ptr, oedg_dt, ent_offset, comput_ent, h->sig_x,
+        h->sig_y, h->cell_ent_DG, h->cell_ent_FV, h->cell_ent_nan, h->ent_partial, accept_dst, accept_only);
   if (comput_ent && !entsum_later)
-    pp_entsum_kernel<<<1, 256, 0, h->stream>>>(h->ent_partial, (int)(g3.x * g3.y), h->ctrl, gate);
+    launch_next(h->stream, early_launch(h), 1, 256, 0, pp_entsum_kernel, h->ent_partial, (int)(g3.x * g3.y), h->ctrl, gate);
 }
 
 // stage diagnostics of state u into the newest log record
@@ -314,9 +326,9 @@ template <int P>
 void launch_diag(mhd_gpu* h, const double* u, int gate) {
   const long long E = (long long)h->nx * h->ny;
   const int nb = (int)std::min<long long>(DIAG_MAX_BLOCKS, std::max<long long>(1, E / 16));
-  stage_diag_kernel<P><<<nb, 256, 0, h->stream>>>(u, h->geo, h->ctrl, gate, h->diag_part,
-                                                   reinterpret_cast<unsigned int*>(h->diag_part + DIAG_VALS * DIAG_MAX_BLOCKS),
-                                                   h->log, h->log_cap);
+  launch_next(h->stream, early_launch(h), nb, 256, 0, stage_diag_kernel<P>, u, h->geo, h->ctrl, gate,
+              h->diag_part, reinterpret_cast<unsigned int*>(h->diag_part + DIAG_VALS * DIAG_MAX_BLOCKS), h->log,
+              h->log_cap);
 }
 
 #define DISPATCH_P(h, fn, ...)              \
@@ -395,7 +407,7 @@ void enqueue_try(mhd_gpu* h) {
   const int R = h->R;
   ctl_step_begin<<<1, 1, 0, h->stream>>>(h->ctrl);
   launch_residual_retry<P>(h, h->u[0], h->ut[1]);
-  ctl_dt_stage1<<<1, 1, 0, h->stream>>>(h->ctrl, R);  // dt, and the pseudo-time of stage 1
+  launch_next(h->stream, early_launch(h), 1, 1, 0, ctl_dt_stage1, h->ctrl, R);  // dt, and the pseudo-time of stage 1
   // SSP-RK(2,2) and (3,3): stages after the first take their combination from the previous
   // stage's residual (next_stage_combine); SSP-RK(1,1) and (5,4) keep the separate combine
   constexpr int EB = 8 * (P + 1) * (P + 1);
@@ -415,14 +427,14 @@ void enqueue_try(mhd_gpu* h) {
                    fin ? h->u[0] : nullptr, ST_RUN, 1, s1, /*entsum_later=*/true, /*accept_only=*/fin);
     const double* cur = fin ? h->u[0] : h->u[s];  // the stage result's interior
     // entropy sum (final stage), stage-end decision, next stage's pseudo-time and the ghost ring
-    stage_end_bc_kernel<P><<<grid1d(nghost, 256), 256, 0, h->stream>>>(
-        cur, h->u[s], h->geo, h->ctrl, R, s, fin ? 0 : s + 1, fin ? h->ent_partial : nullptr, nseg, h->log,
-        h->log_cap);
+    launch_next(h->stream, early_launch(h), grid1d(nghost, 256), 256, 0, stage_end_bc_kernel<P>,
+                cur, h->u[s], h->geo, h->ctrl, R, s, fin ? 0 : s + 1, fin ? h->ent_partial : nullptr, nseg, h->log,
+                h->log_cap);
     if (h->diag) launch_diag<P>(h, cur, ST_RUN);
     launch_residual<P>(h, cur, h->ut[(s % R) + 1], ST_RUN, fin ? StageCombine{} : next_stage_combine(h, s + 1),
                        h->u[s]);
   }
-  ctl_step_end<<<1, 1, 0, h->stream>>>(h->ctrl, R, h->log, h->log_cap);
+  launch_next(h->stream, early_launch(h), 1, 1, 0, ctl_step_end, h->ctrl, R, h->log, h->log_cap);
 }
 
 // kernel nodes of a graph (every launch of the captured try, gated ones included)

@@ -83,6 +83,7 @@ __device__ __forceinline__ void bc_value(const double* src, double* dst_u, const
 
 template <int P>
 __global__ void __launch_bounds__(256) bc_kernel(double* __restrict__ u, Geo g, const Ctrl* ctrl, int gate) {
+  grid_begin();
   if (!gate_open(ctrl, gate)) return;
   bc_value<P>(u, u, g, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -156,6 +157,7 @@ __global__ void __launch_bounds__(256)
                    const double* __restrict__ k4, const double* __restrict__ k5, double* __restrict__ out,
                    int nx, int ny, int R, int stage, const double* __restrict__ dt_ptr, double dt_arg,
                    const Ctrl* ctrl, int gate) {
+  grid_begin();
   if (!gate_open(ctrl, gate)) return;
   const double dt = dt_ptr ? *dt_ptr : dt_arg;
   combine_value<EB>(u0, r1, r2, r3, r4, k1, k2, k3, k4, k5, out, nx, ny, R, stage, dt,
@@ -407,9 +409,13 @@ __global__ void ctl_log_initial(Ctrl* c, LogEntry* log, int log_cap) {
 }
 
 __global__ void ctl_step_begin(Ctrl* c) { ctl_step_begin_body(c); }
-__global__ void ctl_step_end(Ctrl* c, int R, LogEntry* log, int log_cap) { ctl_step_end_body(c, R, log, log_cap); }
+__global__ void ctl_step_end(Ctrl* c, int R, LogEntry* log, int log_cap) {
+  grid_begin();
+  ctl_step_end_body(c, R, log, log_cap);
+}
 // the dt of the try and the pseudo-time of its first stage, in one launch
 __global__ void ctl_dt_stage1(Ctrl* c, int R) {
+  grid_begin();
   ctl_dt_body(c);
   ctl_stage_time_body(c, R, 1);
 }

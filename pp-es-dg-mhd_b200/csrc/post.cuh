@@ -650,9 +650,10 @@ __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB)
   __shared__ double s_red[2 * C::TE * 8];  // chunk sums, two buffers used in turn
   __shared__ __align__(16) double s_pf[(C::NT / 32) * 2 * C::G * C::EB];  // per warp: u (or u_con), k1
   __shared__ int s_cnt;
-  if (!gate_open(ctrl, gate)) return;
   if (threadIdx.x == 0) s_cnt = 0;
-  if (apply_ldf) load_ldf<P>(g.ldfA, s_A);
+  if (apply_ldf) load_ldf<P>(g.ldfA, s_A);  // (written when the instance was created)
+  grid_begin();
+  if (!gate_open(ctrl, gate)) return;
   __syncthreads();
   // the copies of a warp's next chunk are in flight while it works on this one
   double* bu = s_pf + (threadIdx.x >> 5) * 2 * C::G * C::EB;
@@ -1008,6 +1009,7 @@ template <int P>
 __global__ void __launch_bounds__(256, SigCfg<P>::MINB)
     pp_sigsum_kernel(const double* __restrict__ u, Geo g, Ctrl* ctrl, int gate,
                      double* __restrict__ sig_x, double* __restrict__ sig_y) {
+  grid_begin();
   if (!gate_open(ctrl, gate)) return;
   pp_sigsum_tile<P>(u, g, SigOut{sig_x, sig_y, ctrl}, blockIdx.x, blockIdx.y);
 }
@@ -1162,6 +1164,7 @@ __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB)
                     const double* __restrict__ sig_y, const double* __restrict__ cell_ent_DG,
                     const double* __restrict__ cell_ent_FV, const unsigned char* __restrict__ cell_ent_nan,
                     double* __restrict__ ent_partial, double* __restrict__ accept_dst, int accept_only) {
+  grid_begin();
   __shared__ double s_ent[PPCfg<P>::TEL];
   __shared__ int s_cnt;
   if (!gate_open(ctrl, gate)) return;
@@ -1241,6 +1244,7 @@ __global__ void __launch_bounds__(256) stage_end_bc_kernel(const double* src, do
                                                           int stage, int next_stage,
                                                           const double* __restrict__ ent_partial, int ent_nblk,
                                                           LogEntry* log, int log_cap) {
+  grid_begin();
   __shared__ int s_run, s_ent;
   bool run;
   if (blockIdx.x == 0) {  // one read of the state for the whole block, before thread 0 updates it
@@ -1264,6 +1268,7 @@ __global__ void __launch_bounds__(256) stage_end_bc_kernel(const double* src, do
 
 __global__ void __launch_bounds__(256) pp_entsum_kernel(const double* __restrict__ partial, int nblk,
                                                         Ctrl* ctrl, int gate) {
+  grid_begin();
   if (!gate_open(ctrl, gate)) return;
   if (ctrl->neg_avg) return;
   pp_entsum_body(partial, nblk, ctrl);
@@ -1330,6 +1335,7 @@ template <int P>
 __global__ void __launch_bounds__(256) stage_diag_kernel(const double* __restrict__ u, Geo g, Ctrl* ctrl, int gate,
                                                         double* __restrict__ part, unsigned int* ticket,
                                                         LogEntry* log, int log_cap) {
+  grid_begin();
   constexpr int N = P + 1, NN = N * N, EB = 8 * NN;
   __shared__ double s[DIAG_VALS][256];
   __shared__ bool s_last;

@@ -499,13 +499,13 @@ __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
     residual2_kernel(const double* __restrict__ u, const double* __restrict__ ug, double* __restrict__ ut, Geo g,
                      Ctrl* ctrl, int gate, StageCombine sc) {
   using L = Res2Layout<P>;
-  if (!gate_open(ctrl, gate)) return;
   extern __shared__ __align__(16) double sm[];
   const int warp = threadIdx.x >> 5;
   const int ix = blockIdx.x * L::IX + warp % L::IX, iy = blockIdx.y * L::IY + warp / L::IX;
-  if (ix * L::EX >= g.nx || iy * L::EY >= g.ny) return;
   double* wsm = sm + warp * L::WARP;
   res2_prologue<P>(wsm);
+  grid_begin();
+  if (!gate_open(ctrl, gate) || ix * L::EX >= g.nx || iy * L::EY >= g.ny) return;
   unsigned phase = 0;
   residual_item<P>(u, ug, TileOut{ut, ctrl}, g, ix, iy, wsm, phase, sc);
 }
@@ -517,6 +517,7 @@ template <int P>
 __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
     residual2_persistent(const double* __restrict__ u, double* __restrict__ ut, Geo g, Ctrl* ctrl, int gate,
                          int ncol, int nitems) {
+  grid_begin();
   using L = Res2Layout<P>;
   if (!gate_open(ctrl, gate)) return;
   extern __shared__ __align__(16) double sm[];
