@@ -49,6 +49,8 @@ enum GateState : int { GATE_ALWAYS = -1, ST_IDLE = 0, ST_RUN = 1, ST_RECOMPUTE =
 
 // Device-resident control block: the scalars of solve_execute (drive.f90:39-48) and the global
 // reductions of post_process / DG_semidiscretize.
+constexpr long long NO_STEP_LIMIT = 0x7fffffffffffffffLL;
+
 struct Ctrl {
   double t, dt, dt_lim, final_T, cfl_total, tot_ent;
   double t_rk[6];
@@ -59,6 +61,7 @@ struct Ctrl {
   unsigned long long umin_bits[8];
   long long steps, retries, num_negcell_total;
   long long step_limit;  // ctl_step_begin idles once steps >= step_limit
+  long long steps_from;  // steps when the budget was last set (ctl_step_budget)
   int state;
   int try_num;
   int last_step;     // flag == .false. in drive.f90:115-120

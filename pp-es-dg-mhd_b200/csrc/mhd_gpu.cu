@@ -48,7 +48,7 @@ struct mhd_gpu {
   double* cell_ent_FV;
   unsigned char* cell_ent_nan;
   Ctrl* ctrl;
-  Ctrl* ctrl_host;  // pinned mirror
+  Ctrl* ctrl_host;  // host mirror (a slot of g_host_slots while one is free)
   size_t bytes;
   void* block;      // the one device allocation every buffer above is carved from
   bool owns_block;  // false: the block was lent by a server and goes back to it
@@ -141,6 +141,58 @@ int pp_resident_ctas(int dev) {
   return cached[dev];
 }
 
+// Page-locked slots, each the size of a control block, for what a call reads back and waits for: such a copy is
+// one DMA, a pageable one is staged by the driver (a residual with its dt_lim, 33 x 31, p = 1: 34.3 -> 32.4 us).  One
+// fixed array per process, made with the first device's tables; who finds no slot free uses pageable
+// memory.  Slots are taken and given back under a lock, by instances (for life) and by single calls.
+class HostSlots {
+ public:
+  void init() {  // once, under g_init_mutex
+    if (slots_) return;
+    void* m = nullptr;
+    if (cudaHostAlloc(&m, kSlots * sizeof(Ctrl), cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    std::lock_guard<std::mutex> lk(m_);
+    slots_ = static_cast<Ctrl*>(m);
+    for (int i = kSlots - 1; i >= 0; --i) free_.push_back(i);
+  }
+  Ctrl* take() {
+    std::lock_guard<std::mutex> lk(m_);
+    if (free_.empty()) return nullptr;
+    const int i = free_.back();
+    free_.pop_back();
+    return slots_ + i;
+  }
+  bool give(Ctrl* c) {  // false: not a slot
+    std::lock_guard<std::mutex> lk(m_);
+    if (!slots_ || c < slots_ || c >= slots_ + kSlots) return false;
+    free_.push_back((int)(c - slots_));
+    return true;
+  }
+
+ private:
+  static constexpr int kSlots = 128;
+  std::mutex m_;
+  Ctrl* slots_ = nullptr;
+  std::vector<int> free_;
+};
+HostSlots g_host_slots;
+
+// a double that a kernel left on the device as its bit pattern: copy it back and wait for it
+int read_double(const unsigned long long* src, double* out, cudaStream_t st) {
+  unsigned long long local = 0;
+  Ctrl* slot = g_host_slots.take();
+  unsigned long long* bits = slot ? &slot->dt_lim_bits : &local;
+  cudaError_t e = cudaMemcpyAsync(bits, src, sizeof(*bits), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) std::memcpy(out, bits, sizeof(*out));
+  if (slot) g_host_slots.give(slot);
+  CK(e);
+  return MHD_OK;
+}
+
 int init_device_tables(int dev) {
   std::lock_guard<std::mutex> lk(g_init_mutex);
   if (dev < 0 || dev >= kMaxDevices) return MHD_ERR_INVALID;
@@ -182,6 +234,7 @@ int init_device_tables(int dev) {
   CK(cudaFuncSetAttribute(residual2_persistent<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
   CK(cudaFuncSetAttribute(residual2_persistent<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
   CK(cudaFuncSetAttribute(residual2_persistent<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
+  g_host_slots.init();
   g_dev_init[dev] = true;
   return MHD_OK;
 }
@@ -486,7 +539,7 @@ void free_all(mhd_gpu* h) {
     cudaStreamSynchronize(fs);
     cudaStreamDestroy(fs);
   }
-  std::free(h->ctrl_host);
+  if (!g_host_slots.give(h->ctrl_host)) std::free(h->ctrl_host);
 }
 
 }  // namespace
@@ -607,12 +660,14 @@ int create_instance(int nx, int ny, int px, int py, int rknstg, double left, dou
   h->ctrl = reinterpret_cast<Ctrl*>(base + L.ctrl);
   const size_t sb = sizeof(double) * (size_t)n_state(h), tb = sizeof(double) * (size_t)n_ut(h);
   const long long nelg = (long long)(nx + 2) * (ny + 2);
-  h->ctrl_host = static_cast<Ctrl*>(std::calloc(1, sizeof(Ctrl)));
+  h->ctrl_host = g_host_slots.take();
+  if (!h->ctrl_host) h->ctrl_host = static_cast<Ctrl*>(std::malloc(sizeof(Ctrl)));
   if (!h->ctrl_host) {
     free_all(h);
     delete h;
     return MHD_ERR_CUDA;
   }
+  std::memset(h->ctrl_host, 0, sizeof(Ctrl));
   if (u0) cudaMemcpyAsync(h->staging, u0, sb, cudaMemcpyHostToDevice, h->stream);
   double A[ldf_table_doubles(MAXP)];
   tables::ldf_table(px, h->hx, h->hy, A);
@@ -855,15 +910,7 @@ int mhd_gpu_semidiscretize(mhd_gpu_t* h, int ut_stage, int slot, double* dt_lim)
   CK(cudaMemsetAsync(&h->ctrl->dt_lim_bits, 0xFF, sizeof(unsigned long long), h->stream));
   DISPATCH_P(h, launch_residual, h, h->u[slot], h->ut[ut_stage], GATE_ALWAYS);
   CK(cudaGetLastError());
-  if (dt_lim) {
-    unsigned long long bits;
-    CK(cudaMemcpyAsync(&bits, &h->ctrl->dt_lim_bits, sizeof(bits), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    double d;
-    std::memcpy(&d, &bits, sizeof(d));
-    *dt_lim = d;
-  }
-  return MHD_OK;
+  return dt_lim ? read_double(&h->ctrl->dt_lim_bits, dt_lim, h->stream) : MHD_OK;
 }
 
 int mhd_gpu_rk_combine(mhd_gpu_t* h, int stage, double dt) {
@@ -920,7 +967,7 @@ int mhd_gpu_solve_begin(mhd_gpu_t* h, double final_T, double cfl, int use_oedg, 
   c.cfl_total = ((h->R <= 3) ? 1.0 : 1.508) * cfl;  // CFL_RK * CFL (drive.f90:57-63,109)
   c.tot_ent = te;
   c.state = ST_IDLE;
-  c.step_limit = 0x7fffffffffffffffLL;
+  c.step_limit = NO_STEP_LIMIT;
   *h->ctrl_host = c;
   CK(cudaMemcpyAsync(h->ctrl, h->ctrl_host, sizeof(Ctrl), cudaMemcpyHostToDevice, h->stream));
   if (h->log) {  // a new run starts a new log: its first record is the initial state (drive.f90:74)
@@ -940,11 +987,6 @@ int mhd_gpu_solve_begin(mhd_gpu_t* h, double final_T, double cfl, int use_oedg, 
   return MHD_OK;
 }
 
-static int set_step_limit(mhd_gpu* h, long long limit) {
-  CK(cudaMemcpyAsync(&h->ctrl->step_limit, &limit, sizeof(limit), cudaMemcpyHostToDevice, h->stream));
-  return MHD_OK;
-}
-
 int mhd_gpu_get_status(mhd_gpu_t* h, mhd_gpu_status* st) {
   int rc = enter(h);
   if (rc) return rc;
@@ -959,33 +1001,38 @@ int mhd_gpu_advance(mhd_gpu_t* h, long long max_steps, int check_every, mhd_gpu_
   if (rc) return rc;
   if (!h->solve_ready) return MHD_ERR_STATE;
   if (check_every <= 0) check_every = 16;
-  rc = read_ctrl(h);
-  if (rc) return rc;
+  if (h->ctrl_host->done || h->ctrl_host->flags) {  // by the last status read: nothing will run
+    rc = read_ctrl(h);
+    if (rc) return rc;
+    if (h->ctrl_host->done || h->ctrl_host->flags) {
+      fill_status(h, st);
+      return h->ctrl_host->flags;
+    }
+  }
   if (!h->step_exec) {
     rc = build_step_graph(h);
     if (rc) return rc;
   }
-  const long long start = h->ctrl_host->steps;
-  const long long target = (max_steps > 0) ? start + max_steps : 0x7fffffffffffffffLL;
-  rc = set_step_limit(h, target);
-  if (rc) return rc;
-  for (;;) {
-    const Ctrl* c = h->ctrl_host;
-    if (c->done || c->flags || c->steps >= target) break;
-    // tries left before the target: retries need extra launches, so never queue more than
-    // the remaining steps plus a small slack; extra launches past the target are idle.
-    long long left = target - c->steps;
-    int batch = (int)((left < check_every) ? left : check_every);
-    if (batch < 1) batch = 1;
+  // The step budget lives on the device and is set and lifted by kernels around each round of tries, so
+  // that a round waits for the device once, when it reads the status (before: a read, two writes of the
+  // budget and three waits a call; one step of Orszag-Tang 64^2, p = 2: 117 -> 102 us).
+  const Ctrl* c = h->ctrl_host;
+  long long left = (max_steps > 0) ? max_steps : NO_STEP_LIMIT;
+  do {
+    // tries of this round: retries need extra launches, so never queue more than the remaining
+    // steps; launches past the budget are idle
+    const int batch = (int)std::min<long long>(left, check_every);
+    ctl_step_budget<<<1, 1, 0, h->stream>>>(h->ctrl, left);
     for (int b = 0; b < batch; ++b) CK(cudaGraphLaunch(h->step_exec, h->stream));
+    ctl_step_budget<<<1, 1, 0, h->stream>>>(h->ctrl, -1);
+    CK(cudaGetLastError());
     rc = read_ctrl(h);
     if (rc) return rc;
     rc = drain_log(h);
     if (rc) return rc;
-  }
+    if (max_steps > 0) left -= c->steps - c->steps_from;
+  } while (!c->done && !c->flags && left > 0);
   fill_status(h, st);
-  set_step_limit(h, 0x7fffffffffffffffLL);
-  CK(cudaStreamSynchronize(h->stream));
   return h->ctrl_host->flags;
 }
 
@@ -1127,8 +1174,8 @@ extern "C" int mhd_gpu_semidiscretize_noalloc(int p, int nx, int ny, double hx, 
   if (rc) return rc;
   Ctrl* ctrl = static_cast<Ctrl*>(addr);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // the reduction cell must start "empty" (all ones: above every positive double's bit pattern)
-  CK(cudaMemsetAsync(&ctrl->dt_lim_bits, 0xFF, sizeof(unsigned long long), s));
+  // a reduction cell that is read must start "empty" (all ones: above every positive double's bit pattern)
+  if (dt_lim) CK(cudaMemsetAsync(&ctrl->dt_lim_bits, 0xFF, sizeof(unsigned long long), s));
   Geo g;
   std::memset(&g, 0, sizeof(g));
   g.nx = nx;
@@ -1155,15 +1202,7 @@ extern "C" int mhd_gpu_semidiscretize_noalloc(int p, int nx, int ny, double hx, 
     }
   }
   CK(cudaGetLastError());
-  if (dt_lim) {
-    unsigned long long bits = 0;
-    CK(cudaMemcpyAsync(&bits, &ctrl->dt_lim_bits, sizeof(bits), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    double d;
-    std::memcpy(&d, &bits, sizeof(d));
-    *dt_lim = d;
-  }
-  return MHD_OK;
+  return dt_lim ? read_double(&ctrl->dt_lim_bits, dt_lim, s) : MHD_OK;
 }
 
 #include "batch_impl.cuh"

@@ -409,6 +409,18 @@ __global__ void ctl_log_initial(Ctrl* c, LogEntry* log, int log_cap) {
 }
 
 __global__ void ctl_step_begin(Ctrl* c) { ctl_step_begin_body(c); }
+
+// The step budget of a round of tries: `more` steps from here (none for a run that has ended or raised a
+// flag; NO_STEP_LIMIT: as many as it takes), or no limit any more (more < 0).
+__global__ void ctl_step_budget(Ctrl* c, long long more) {
+  if (more < 0) {
+    c->step_limit = NO_STEP_LIMIT;
+    return;
+  }
+  c->steps_from = c->steps;
+  c->step_limit = (c->done || c->flags) ? c->steps : (more > NO_STEP_LIMIT - c->steps ? NO_STEP_LIMIT : c->steps + more);
+}
+
 __global__ void ctl_step_end(Ctrl* c, int R, LogEntry* log, int log_cap) {
   grid_begin();
   ctl_step_end_body(c, R, log, log_cap);
@@ -433,7 +445,7 @@ __global__ void ctl_solve_begin(Ctrl* c, double final_T, double cfl_total) {
   z.final_T = final_T;
   z.cfl_total = cfl_total;
   z.state = ST_IDLE;
-  z.step_limit = 0x7fffffffffffffffLL;
+  z.step_limit = NO_STEP_LIMIT;
   if (neg) {
     z.flags = 8;  // MHD_FLAG_INIT_NEG_AVG
   } else {

@@ -120,7 +120,7 @@ int solve_begin_async(mhd_gpu* h, double final_T, double cfl, int use_oedg, int 
   std::memset(h->ctrl_host, 0, sizeof(Ctrl));
   h->ctrl_host->final_T = final_T;
   h->ctrl_host->cfl_total = cfl_total;
-  h->ctrl_host->step_limit = 0x7fffffffffffffffLL;
+  h->ctrl_host->step_limit = NO_STEP_LIMIT;
   if (h->step_exec) {
     cudaGraphExecDestroy(h->step_exec);
     h->step_exec = nullptr;
