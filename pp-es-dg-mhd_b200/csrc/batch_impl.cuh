@@ -15,7 +15,7 @@
 
 namespace {
 
-enum WorkKind { WK_RES = 0, WK_AVG, WK_SIG, WK_LIM, WK_CMB, WK_BC, WK_COUNT };
+enum WorkKind { WK_RES = 0, WK_AVG, WK_SUM, WK_SIG, WK_LIM, WK_CMB, WK_BC, WK_COUNT };
 
 // One group's device table, one allocation, uploaded with one copy:
 //   InstDesc insts[cap] | int total[WK_COUNT] | int ninst | int pref[WK_COUNT][cap + 1]
@@ -99,8 +99,8 @@ void member_work(const mhd_gpu* h, long long* cnt, InstDesc& d) {
   const long long nx = h->nx, ny = h->ny;
   cnt[WK_RES] = (long long)res2_item_cols<P>(h->nx) * res2_item_rows<P>(h->ny);
   const long long nelg = (nx + 2) * (ny + 2);
-  d.nblk_avg = (int)((nelg + TE - 1) / TE);
-  cnt[WK_AVG] = d.nblk_avg;
+  cnt[WK_AVG] = (nelg + TE - 1) / TE;
+  cnt[WK_SUM] = pp_sum_chunks(h->nx, h->ny);
   cnt[WK_SIG] = ((nx + SigCfg<P>::TX - 1) / SigCfg<P>::TX) * ((ny + SigCfg<P>::TY - 1) / SigCfg<P>::TY);
   constexpr int TEL = PPCfg<P>::TEL;  // the limiter's row segments
   d.nseg_limit = (int)(((nx + TEL - 1) / TEL) * ny);
@@ -146,7 +146,7 @@ int refresh_batch(mhd_batch* b) {
     InstDesc* hi = reinterpret_cast<InstDesc*>(hs);
     int* htot = reinterpret_cast<int*>(hs + sizeof(InstDesc) * g.cap);
     int* hpref = htot + WK_COUNT + 1;
-    long long run[WK_COUNT] = {0, 0, 0, 0, 0, 0};
+    long long run[WK_COUNT] = {};
     for (int k = 0; k < WK_COUNT; ++k) hpref[k * (g.cap + 1)] = 0;
     for (int m = 0; m < n; ++m) {
       InstDesc d = make_desc(g.members[m]);
@@ -190,7 +190,7 @@ int full_grid(K kernel, int threads, size_t smem, int nsm) {
 }
 
 struct BatchGrids {
-  int res, cmb, bc, avg, avg_final, sig, lim, seb;
+  int res, res_post, cmb, bc, avg, avg_final, sum, sig, lim, seb;
 };
 
 // queried before a capture begins (the occupancy calculator is host-only work)
@@ -198,11 +198,13 @@ template <int P>
 BatchGrids batch_grids(int nsm) {
   constexpr int EB = 8 * (P + 1) * (P + 1);
   BatchGrids gr;
-  gr.res = full_grid(residual2_batched<P>, Res2Layout<P>::NT, Res2Layout<P>::BYTES, nsm);
+  gr.res = full_grid(residual2_batched<P, RES_UT>, Res2Layout<P>::NT, Res2Layout<P>::BYTES, nsm);
+  gr.res_post = full_grid(residual2_batched<P, RES_POST>, Res2Layout<P>::NT, Res2Layout<P>::BYTES, nsm);
   gr.cmb = full_grid(combine_batched<EB>, 256, 0, nsm);
   gr.bc = full_grid(bc_batched<P>, 256, 0, nsm);
-  gr.avg = full_grid(pp_avg_ldf_batched<P, false>, PPCfg<P>::NT, 0, nsm);
-  gr.avg_final = full_grid(pp_avg_ldf_batched<P, true>, PPCfg<P>::NT, 0, nsm);
+  gr.avg = full_grid(pp_avg_ldf_batched<P, true>, PPCfg<P>::NT, 0, nsm);
+  gr.avg_final = full_grid(pp_avg_ldf_batched<P, false>, PPCfg<P>::NT, 0, nsm);
+  gr.sum = full_grid(pp_reduce_batched, 256, 0, nsm);
   gr.sig = full_grid(pp_sigsum_batched<P>, 256, 0, nsm);
   gr.lim = full_grid(pp_limit_batched<P>, PPCfg<P>::NT, 0, nsm);
   gr.seb = full_grid(stage_end_bc_batched<P>, 256, 0, nsm);
@@ -221,24 +223,27 @@ void enqueue_group_try(mhd_batch* b, BatchGroup& g, const BatchGrids& gr, cudaSt
   const int grid_res = gr.res, grid_cmb = gr.cmb, grid_bc = gr.bc, grid_avg = gr.avg, grid_sig = gr.sig,
             grid_lim = gr.lim;
   ctl_batched<<<1, 256, 0, st>>>(in, ninst, CTL_STEP_BEGIN, R, 0);
-  residual2_batched<P><<<grid_res, NT_RES, smem, st>>>(in, g.pref(WK_RES), tot + WK_RES, ninst, 0, 1, ST_RECOMPUTE,
-                                                        0, 0.0, 0.0);
+  residual2_batched<P, RES_UT><<<grid_res, NT_RES, smem, st>>>(in, g.pref(WK_RES), tot + WK_RES, ninst, 0, 1,
+                                                               ST_RECOMPUTE, 0, 0.0, 0.0);
   ctl_batched<<<1, 256, 0, st>>>(in, ninst, CTL_DT_STAGE1, R, 1);  // dt, and the pseudo-time of stage 1
   for (int s = 1; s <= R; ++s) {
     const int fin = (s == R);
     // stage 1: loop 1 forms the stage state and its ghost ring; SSP-RK(2,2)/(3,3): later stages
-    // come from the previous residual
-    if (s > 1 && R > 3)
+    // come from the previous residual, with their loop 1
+    if (s > 1 && R > 3) {
       combine_batched<EB><<<grid_cmb, 256, 0, st>>>(in, g.pref(WK_CMB), tot + WK_CMB, ninst, s, ST_RUN);
-    if (s > 1) bc_batched<P><<<grid_bc, 256, 0, st>>>(in, g.pref(WK_BC), tot + WK_BC, ninst, s, ST_RUN);
-    if (fin)
-      pp_avg_ldf_batched<P, true><<<gr.avg_final, PPCfg<P>::NT, 0, st>>>(in, g.pref(WK_AVG), tot + WK_AVG, ninst, s, ST_RUN,
-                                                                  s == 1);
-    else
-      pp_avg_ldf_batched<P, false><<<grid_avg, PPCfg<P>::NT, 0, st>>>(in, g.pref(WK_AVG), tot + WK_AVG, ninst, s, ST_RUN,
+      bc_batched<P><<<grid_bc, 256, 0, st>>>(in, g.pref(WK_BC), tot + WK_BC, ninst, s, ST_RUN);
+    }
+    if (s == 1 || R > 3) {
+      if (fin)
+        pp_avg_ldf_batched<P, false><<<gr.avg_final, PPCfg<P>::NT, 0, st>>>(in, g.pref(WK_AVG), tot + WK_AVG, ninst, s, ST_RUN,
+                                                                     s == 1);
+      else
+        pp_avg_ldf_batched<P, true><<<grid_avg, PPCfg<P>::NT, 0, st>>>(in, g.pref(WK_AVG), tot + WK_AVG, ninst, s, ST_RUN,
                                                                 s == 1);
+    }
     if (fin) {
-      pp_reduce_batched<<<b->nsm, 256, 0, st>>>(in, ninst, fin, ST_RUN);
+      pp_reduce_batched<<<gr.sum, 256, 0, st>>>(in, g.pref(WK_SUM), tot + WK_SUM, ninst, ST_RUN);
       pp_sigsum_batched<P><<<grid_sig, 256, 0, st>>>(in, g.pref(WK_SIG), tot + WK_SIG, ninst, s, fin, ST_RUN);
     }
     if (fin) pp_limit_batched<P><<<grid_lim, PPCfg<P>::NT, 0, st>>>(in, g.pref(WK_LIM), tot + WK_LIM, ninst, s, fin, ST_RUN);
@@ -249,8 +254,12 @@ void enqueue_group_try(mhd_batch* b, BatchGroup& g, const BatchGrids& gr, cudaSt
     const int nxt = (!fin && (R == 2 || R == 3)) ? s + 1 : 0;
     const double ca = nxt == 0 ? 0.0 : (R == 2 ? 0.5 : (nxt == 2 ? 0.75 : 1.0 / 3.0));
     const double cb = nxt == 0 ? 0.0 : (R == 2 ? 0.5 : (nxt == 2 ? 0.25 : 2.0 / 3.0));
-    residual2_batched<P><<<grid_res, NT_RES, smem, st>>>(in, g.pref(WK_RES), tot + WK_RES, ninst, s, (s % R) + 1,
-                                                          ST_RUN, nxt, ca, cb);
+    if (nxt)
+      residual2_batched<P, RES_POST><<<gr.res_post, NT_RES, smem, st>>>(in, g.pref(WK_RES), tot + WK_RES, ninst, s, (s % R) + 1,
+                                                                    ST_RUN, nxt, ca, cb);
+    else
+      residual2_batched<P, RES_UT><<<grid_res, NT_RES, smem, st>>>(in, g.pref(WK_RES), tot + WK_RES, ninst, s, (s % R) + 1,
+                                                                  ST_RUN, 0, 0.0, 0.0);
   }
   ctl_batched<<<1, 256, 0, st>>>(in, ninst, CTL_STEP_END, R, 0);
 }

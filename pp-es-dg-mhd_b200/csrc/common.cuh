@@ -72,7 +72,8 @@ struct Ctrl {
   int num_negcell_last;
   int pp_relimit;
   int pending_dtlim; // a residual wrote dt_lim_bits that is not yet decoded
-  int pad_[2];
+  unsigned sum_ticket;  // CTAs done with the global-average sum (pp_reduce_kernel); zero between launches
+  int pad_;
   long long log_seq; // records written to the driver log so far (LogEntry)
 };
 
@@ -169,9 +170,7 @@ struct InstDesc {
   LogEntry* log;   // driver log ring (nullptr: none)
   int log_cap;
   int use_oedg, use_ldf, ent_offset, R;
-  int nblk_avg;    // pp_avg_ldf chunks of this instance (partial sums)
   int nseg_limit;  // pp_limit segments of this instance (entropy partials)
-  int pad_;
 };
 
 // Batched kernels see a group's work of one kind as the concatenation of every member's items;

@@ -128,14 +128,14 @@ template <int P>
 dim3 pp_grid_limit(const mhd_gpu* h) { return dim3((h->nx + PPCfg<P>::TEL - 1) / PPCfg<P>::TEL, h->ny); }
 
 // CTAs of pp_avg_ldf_kernel<P> the device holds at once (its grid walks the chunks)
-template <int P, bool NEEDG>
+template <int P, bool LIMIT>
 int pp_resident_ctas(int dev) {
   static int cached[kMaxDevices];
   if (dev < 0 || dev >= kMaxDevices) return 1;
   if (!cached[dev]) {
     int nsm = 0, per_sm = 0;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pp_avg_ldf_kernel<P, NEEDG>, PPCfg<P>::NT, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pp_avg_ldf_kernel<P, LIMIT>, PPCfg<P>::NT, 0);
     cached[dev] = std::max(1, nsm) * std::max(1, per_sm);
   }
   return cached[dev];
@@ -225,12 +225,21 @@ int init_device_tables(int dev) {
       rows[p].iqw[k] = tabs[p].iqw[k];
     }
   CK(cudaMemcpyToSymbol(d_rows, rows, sizeof(rows)));
-  CK(cudaFuncSetAttribute(residual2_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
-  CK(cudaFuncSetAttribute(residual2_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
-  CK(cudaFuncSetAttribute(residual2_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
-  CK(cudaFuncSetAttribute(residual2_batched<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
-  CK(cudaFuncSetAttribute(residual2_batched<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
-  CK(cudaFuncSetAttribute(residual2_batched<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_kernel<1, RES_UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_kernel<1, RES_COMBINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_kernel<1, RES_POST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_kernel<2, RES_UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_kernel<2, RES_COMBINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_kernel<2, RES_POST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_kernel<3, RES_UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_kernel<3, RES_COMBINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_kernel<3, RES_POST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_batched<1, RES_UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_batched<1, RES_POST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_batched<2, RES_UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_batched<2, RES_POST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_batched<3, RES_UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_batched<3, RES_POST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
   CK(cudaFuncSetAttribute(residual2_persistent<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
   CK(cudaFuncSetAttribute(residual2_persistent<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
   CK(cudaFuncSetAttribute(residual2_persistent<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
@@ -286,11 +295,13 @@ void launch_bc(mhd_gpu* h, double* u, int gate) {
 
 // ug: the array whose ghost ring the boundary halos come from (nullptr: u's own)
 template <int P>
-void launch_residual(mhd_gpu* h, const double* u, double* ut, int gate, StageCombine sc = StageCombine{},
-                     const double* ug = nullptr) {
+void launch_residual(mhd_gpu* h, const double* u, double* ut, int gate, int mode = RES_UT,
+                     const StagePost& sp = StagePost{}, const double* ug = nullptr) {
   using L = Res2Layout<P>;
   dim3 grid((h->nx + L::TX - 1) / L::TX, (h->ny + L::TY - 1) / L::TY);
-  launch_next(h->stream, early_launch(h), grid, L::NT, L::BYTES, residual2_kernel<P>, u, ug ? ug : u, ut, h->geo, h->ctrl, gate, sc);
+  launch_next(h->stream, early_launch(h), grid, L::NT, L::BYTES, 
+              mode == RES_POST ? residual2_kernel<P, RES_POST> : mode == RES_COMBINE ? residual2_kernel<P, RES_COMBINE> : residual2_kernel<P, RES_UT>,
+              u, ug ? ug : u, ut, h->geo, h->ctrl, gate, sp);
 }
 
 // the re-try residual of a try (gate ST_RECOMPUTE, usually closed): a persistent grid of the CTAs
@@ -335,27 +346,24 @@ template <int P>
 // entsum_later (time-step pipeline): the entropy sum is left to the stage-end launch
 // accept_only (with accept_dst): the limiter writes its result to accept_dst only, leaving slot's
 // interior as loop 1 left it
+// loop1_done (time-step pipeline): the previous residual did loop 1 of this stage (StagePost), and loop 3
+// where it is fused
 void launch_post(mhd_gpu* h, int slot, int apply_oedg, int apply_ldf, const double* dt_ptr, double oedg_dt,
                  int ent_offset, int comput_ent, double* accept_dst, int gate, int fuse = 0,
-                 Stage1Src s1 = Stage1Src{}, bool entsum_later = false, int accept_only = 0) {
-  const int nb1 = pp_nblk_avg<P>(h);
+                 Stage1Src s1 = Stage1Src{}, bool entsum_later = false, int accept_only = 0, bool loop1_done = false) {
   const int limit_in_loop1 = fuse && !apply_oedg && !comput_ent && !accept_dst;
-  if (apply_oedg) {
-    const int grid1 = std::min(nb1, pp_resident_ctas<P, true>(h->device));
-    launch_next(h->stream, early_launch(h), grid1, PPCfg<P>::NT, 0, pp_avg_ldf_kernel<P, true>, h->u[slot],
-                h->u_avg, h->geo, h->ctrl, gate, apply_ldf, 1, ent_offset, h->partial, h->cell_ent_DG, h->cell_ent_FV, h->cell_ent_nan, limit_in_loop1,
-                nb1, s1);
-  } else {
-    const int grid1 = std::min(nb1, pp_resident_ctas<P, false>(h->device));
-    launch_next(h->stream, early_launch(h), grid1, PPCfg<P>::NT, 0, pp_avg_ldf_kernel<P, false>, h->u[slot],
-                h->u_avg, h->geo, h->ctrl, gate, apply_ldf, 0, ent_offset, h->partial, h->cell_ent_DG, h->cell_ent_FV, h->cell_ent_nan, limit_in_loop1,
-                nb1, s1);
+  if (!loop1_done) {
+    const int nb1 = pp_nblk_avg<P>(h);
+    const int grid1 = std::min(nb1, limit_in_loop1 ? pp_resident_ctas<P, true>(h->device) : pp_resident_ctas<P, false>(h->device));
+    launch_next(h->stream, early_launch(h), grid1, PPCfg<P>::NT, 0, limit_in_loop1 ? pp_avg_ldf_kernel<P, true> : pp_avg_ldf_kernel<P, false>,
+                h->u[slot], h->u_avg, h->geo, h->ctrl, gate, apply_ldf, ent_offset, h->cell_ent_DG, h->cell_ent_FV,
+                h->cell_ent_nan, nb1, s1);
   }
   if (limit_in_loop1) return;
-  if (apply_oedg) {  // the global sums (one CTA) and the face indicators are independent: fork/join
+  if (apply_oedg) {  // the global sums and the face indicators are independent: fork/join
     cudaEventRecord(h->ev_fork, h->stream);
     cudaStreamWaitEvent(h->side_stream, h->ev_fork, 0);
-    pp_reduce_kernel<<<1, 256, 0, h->side_stream>>>(h->partial, nb1, h->ctrl, gate);
+    pp_reduce_kernel<<<pp_sum_chunks(h->nx, h->ny), 256, 0, h->side_stream>>>(h->u_avg, h->geo, h->partial, h->ctrl, gate);
     cudaEventRecord(h->ev_join, h->side_stream);
     const dim3 gs((h->nx + SigCfg<P>::TX - 1) / SigCfg<P>::TX, (h->ny + SigCfg<P>::TY - 1) / SigCfg<P>::TY);
     launch_next(h->stream, early_launch(h), gs, 256, 0, pp_sigsum_kernel<P>, h->u[slot], h->geo, h->ctrl, gate, h->sig_x, h->sig_y);
@@ -442,50 +450,56 @@ void fill_status(const mhd_gpu* h, mhd_gpu_status* st) {
   st->pad_ = 0;
 }
 
-// one try of a time step (drive.f90:93-300), recorded into the capturing stream
-// the combination of stage `stage` (SSP-RK(2,2) stage 2, SSP-RK(3,3) stages 2 and 3; the
-// coefficients of combine_value) folded into the previous residual; none otherwise
-StageCombine next_stage_combine(const mhd_gpu* h, int stage) {
-  StageCombine sc{};
-  if (h->R == 2 && stage == 2) {
-    sc = StageCombine{h->u[0], h->u[2], 0.5, 0.5, &h->ctrl->dt};
-  } else if (h->R == 3 && (stage == 2 || stage == 3)) {
-    sc = StageCombine{h->u[0], h->u[stage], stage == 2 ? 0.75 : 1.0 / 3.0, stage == 2 ? 0.25 : 2.0 / 3.0, &h->ctrl->dt};
-  }
-  return sc;
+// stage `stage` (> 1) out of the previous residual, SSP-RK(2,2) and (3,3): the coefficients of combine_value
+StagePost next_stage_post(const mhd_gpu* h, int stage) {
+  const double ca = h->R == 2 ? 0.5 : (stage == 2 ? 0.75 : 1.0 / 3.0), cb = h->R == 2 ? 0.5 : (stage == 2 ? 0.25 : 2.0 / 3.0);
+  return StagePost{h->u[0], h->u[stage], ca, cb, &h->ctrl->dt, h->u_avg, h->cell_ent_DG, h->cell_ent_FV, h->cell_ent_nan,
+                   h->use_ldf, h->ent_offset, stage == h->R};
 }
 
+// Whether loop 1 of the stages after the first runs in the previous residual (RES_POST) or, with a boundary fill
+// before it, as launches of its own.  Folded a step is faster at every size.  Orszag-Tang, SSP-RK(3,3), launches ->
+// folded (us a step): p = 1, 16^2 65 -> 59, 128^2 89 -> 81, 512^2 500 -> 484; p = 2, 64^2 80 -> 75, 300^2 427 -> 409;
+// p = 3, 100^2 123 -> 117, 180^2 243 -> 243; vortex 512^2 p = 3 1607 -> 1539.  Below 1024 nodes, where
+// it is 2-4 us, a try keeps one launch per procedure, the sequence that step_graph_kernels is known by.
+bool fold_post(const mhd_gpu* h) { return (long long)h->nx * h->ny * h->nn >= 1024; }
+
+// one try of a time step (drive.f90:93-300), recorded into the capturing stream
 template <int P>
 void enqueue_try(mhd_gpu* h) {
   const int R = h->R;
   ctl_step_begin<<<1, 1, 0, h->stream>>>(h->ctrl);
   launch_residual_retry<P>(h, h->u[0], h->ut[1]);
   launch_next(h->stream, early_launch(h), 1, 1, 0, ctl_dt_stage1, h->ctrl, R);  // dt, and the pseudo-time of stage 1
-  // SSP-RK(2,2) and (3,3): stages after the first take their combination from the previous
-  // stage's residual (next_stage_combine); SSP-RK(1,1) and (5,4) keep the separate combine
+  // SSP-RK(2,2) and (3,3): stages after the first take their combination from the previous stage's
+  // residual, with loop 1 (fold_post) or without; SSP-RK(1,1) and (5,4) keep the separate combine
+  const int mode = R != 2 && R != 3 ? RES_UT : fold_post(h) ? RES_POST : RES_COMBINE;
   constexpr int EB = 8 * (P + 1) * (P + 1);
   const long long nghost = 2LL * (h->nx + h->ny) * EB;
   const int nseg = (int)(pp_grid_limit<P>(h).x * pp_grid_limit<P>(h).y);
   for (int s = 1; s <= R; ++s) {
     const int fin = (s == R);
     // stage 1: loop 1 forms the stage state and its ghost ring (Stage1Src)
-    if (s > 1 && R > 3) launch_combine<P>(h, s, &h->ctrl->dt, 0.0, ST_RUN);
-    if (s > 1) launch_bc<P>(h, h->u[s], ST_RUN);
+    const bool posted = s > 1 && mode == RES_POST;
+    if (s > 1 && mode == RES_UT) launch_combine<P>(h, s, &h->ctrl->dt, 0.0, ST_RUN);
+    if (s > 1 && !posted) launch_bc<P>(h, h->u[s], ST_RUN);
     const Stage1Src s1 = s == 1 ? Stage1Src{h->u[0], h->ut[1], &h->ctrl->dt, stage1_coef(R)} : Stage1Src{};
     // the final stage's limiter writes the accepted interior to u_con only (drive.f90:304-311); the
     // stage array's ghost ring is then filled from u_con, and the next step's stage-1 residual reads
     // u_con's interior with that ring.  u_con keeps its own ghost ring, which only the re-try
     // residual reads (drive.f90:104 takes u_con as it is).
     launch_post<P>(h, s, h->use_oedg && fin, h->use_ldf, &h->ctrl->dt, 0.0, h->ent_offset, fin,
-                   fin ? h->u[0] : nullptr, ST_RUN, 1, s1, /*entsum_later=*/true, /*accept_only=*/fin);
+                   fin ? h->u[0] : nullptr, ST_RUN, 1, s1, /*entsum_later=*/true, /*accept_only=*/fin, posted);
     const double* cur = fin ? h->u[0] : h->u[s];  // the stage result's interior
     // entropy sum (final stage), stage-end decision, next stage's pseudo-time and the ghost ring
     launch_next(h->stream, early_launch(h), grid1d(nghost, 256), 256, 0, stage_end_bc_kernel<P>,
                 cur, h->u[s], h->geo, h->ctrl, R, s, fin ? 0 : s + 1, fin ? h->ent_partial : nullptr, nseg, h->log,
                 h->log_cap);
     if (h->diag) launch_diag<P>(h, cur, ST_RUN);
-    launch_residual<P>(h, cur, h->ut[(s % R) + 1], ST_RUN, fin ? StageCombine{} : next_stage_combine(h, s + 1),
-                       h->u[s]);
+    if (fin || mode == RES_UT)
+      launch_residual<P>(h, cur, h->ut[(s % R) + 1], ST_RUN, RES_UT, StagePost{}, h->u[s]);
+    else
+      launch_residual<P>(h, cur, nullptr, ST_RUN, mode, next_stage_post(h, s + 1), h->u[s]);
   }
   launch_next(h->stream, early_launch(h), 1, 1, 0, ctl_step_end, h->ctrl, R, h->log, h->log_cap);
 }
@@ -1187,17 +1201,17 @@ extern "C" int mhd_gpu_semidiscretize_noalloc(int p, int nx, int ny, double hx, 
   switch (p) {
     case 1: {
       using L = Res2Layout<1>;
-      residual2_kernel<1><<<dim3((nx + L::TX - 1) / L::TX, (ny + L::TY - 1) / L::TY), L::NT, L::BYTES, s>>>(u, u, ut, g, ctrl, GATE_ALWAYS, StageCombine{});
+      residual2_kernel<1, RES_UT><<<dim3((nx + L::TX - 1) / L::TX, (ny + L::TY - 1) / L::TY), L::NT, L::BYTES, s>>>(u, u, ut, g, ctrl, GATE_ALWAYS, StagePost{});
       break;
     }
     case 2: {
       using L = Res2Layout<2>;
-      residual2_kernel<2><<<dim3((nx + L::TX - 1) / L::TX, (ny + L::TY - 1) / L::TY), L::NT, L::BYTES, s>>>(u, u, ut, g, ctrl, GATE_ALWAYS, StageCombine{});
+      residual2_kernel<2, RES_UT><<<dim3((nx + L::TX - 1) / L::TX, (ny + L::TY - 1) / L::TY), L::NT, L::BYTES, s>>>(u, u, ut, g, ctrl, GATE_ALWAYS, StagePost{});
       break;
     }
     default: {
       using L = Res2Layout<3>;
-      residual2_kernel<3><<<dim3((nx + L::TX - 1) / L::TX, (ny + L::TY - 1) / L::TY), L::NT, L::BYTES, s>>>(u, u, ut, g, ctrl, GATE_ALWAYS, StageCombine{});
+      residual2_kernel<3, RES_UT><<<dim3((nx + L::TX - 1) / L::TX, (ny + L::TY - 1) / L::TY), L::NT, L::BYTES, s>>>(u, u, ut, g, ctrl, GATE_ALWAYS, StagePost{});
       break;
     }
   }

@@ -332,13 +332,60 @@ __device__ __forceinline__ double limit_group(double* x, const double* avg, bool
 }
 
 // ---------------------------------------------------------------------------------------------
-// loop 1 for one chunk of TE consecutive element blocks of the ghosted grid (one contiguous run of
-// memory).  s_A = the LDF table in shared memory (load_ldf); s_red = CTA
-// scratch of TE * 8 doubles for the chunk sums, which a caller either alternates between two such
-// buffers from chunk to chunk or protects with a barrier after the call (one barrier per chunk
-// here, between the writes of s_red and the reads).
+// LDF projection of one element's (Bx - avg, By - avg), in place: (bx, by) = this lane's node.  It works
+// on the sums and differences of mirror nodes (tables.h, ldf_table): butterflies along x and y, this
+// lane's output place from at most 2 M^2 input places through the group's row, butterflies back.  gb = the
+// group's first lane, nd = this lane holds one of its nodes (the other lanes take part with their own
+// value as partner), row = the group's 2 NN doubles, A = the table (shared or global memory).
 //
-// limit = 1 fuses loop 3 for a stage without OEDG and without the entropy sum: the interior
+// In loop 1 the shared-memory pipe is the bound, and the dense operator (2n^2 products an output) read
+// its rows from there: 400^2 without / with the OEDG sums, p = 3: 92 -> 75 / 90 -> 61 us, p = 2: 77 -> 70 /
+// 70 -> 61 us; p = 1, 500^2: 38.5 -> 37.7 us.
+// ---------------------------------------------------------------------------------------------
+template <int P>
+__device__ __forceinline__ void ldf_project(double& bx, double& by, int gb, int node, bool nd, double* row,
+                                            const double2* __restrict__ A) {
+  constexpr int N = P + 1, NN = N * N, M = (N + 1) / 2;
+  const int lane = threadIdx.x & 31, k = node % N, l = node / N;
+  const int mx = nd ? gb + (N - 1 - k) + N * l : lane, my = nd ? gb + k + N * (N - 1 - l) : lane;
+  const double sx = 2 * k < N - 1 ? 1.0 : (2 * k == N - 1 ? 0.0 : -1.0);
+  const double sy = 2 * l < N - 1 ? 1.0 : (2 * l == N - 1 ? 0.0 : -1.0);
+  bx = __fma_rn(sx, __shfl_sync(FULL_MASK, bx, mx), bx);
+  by = __fma_rn(sx, __shfl_sync(FULL_MASK, by, mx), by);
+  bx = __fma_rn(sy, __shfl_sync(FULL_MASK, bx, my), bx);
+  by = __fma_rn(sy, __shfl_sync(FULL_MASK, by, my), by);
+  double2* in = reinterpret_cast<double2*>(row);
+  if (nd) in[node] = make_double2(bx, by);
+  __syncwarp();
+  double ox = 0.0, oy = 0.0;
+  if (nd) {
+    const double2* w = A + node;
+    const bool px = 2 * k > N - 1, py = 2 * l > N - 1;  // the parity of this lane's place
+#pragma unroll
+    for (int jy = 0; jy < M; ++jy)
+#pragma unroll
+      for (int jx = 0; jx < M; ++jx) {
+        const int s = jx + M * jy;
+        const double2 c = w[s * NN], f = in[(px ? N - 1 - jx : jx) + N * (py ? N - 1 - jy : jy)];
+        ox = __fma_rn(c.x, f.x, ox);
+        oy = __fma_rn(c.y, f.y, oy);
+        const double2 d = w[(s + M * M) * NN], h = in[(px ? jx : N - 1 - jx) + N * (py ? jy : N - 1 - jy)];
+        ox = __fma_rn(d.x, h.y, ox);
+        oy = __fma_rn(d.y, h.x, oy);
+      }
+  }
+  __syncwarp();  // the row may be rewritten
+  ox = __fma_rn(-sy, __shfl_sync(FULL_MASK, ox, my), ox);
+  oy = __fma_rn(-sy, __shfl_sync(FULL_MASK, oy, my), oy);
+  bx = __fma_rn(-sx, __shfl_sync(FULL_MASK, ox, mx), ox);
+  by = __fma_rn(-sx, __shfl_sync(FULL_MASK, oy, mx), oy);
+}
+
+// ---------------------------------------------------------------------------------------------
+// loop 1 for one chunk of TE consecutive element blocks of the ghosted grid (one contiguous run of
+// memory).  s_A = the LDF table in shared memory (load_ldf).
+//
+// LIMIT fuses loop 3 for a stage without OEDG and without the entropy sum: the interior
 // elements are limited in registers before the one write-back.  The reference skips loop 3
 // altogether when any element has an inadmissible average (neg_avg); here other CTAs may already
 // have limited their elements by then.  That is only allowed where the stage result is discarded
@@ -432,13 +479,12 @@ __device__ __forceinline__ void pp_prefetch(const double* __restrict__ u, const 
   cp_async_commit();
 }
 
-template <int P, bool NEEDG, bool PF>
+template <int P, bool LIMIT, bool PF>
 __device__ __forceinline__ void pp_avg_ldf_chunk(double* __restrict__ u, double* __restrict__ u_avg, const Geo& g,
-                                                 Ctrl* ctrl, long long chunk, GridRC cpos, int apply_ldf, int need_global,
-                                                 int ent_offset, double* __restrict__ partial_out,  // 8 doubles
+                                                 Ctrl* ctrl, long long chunk, GridRC cpos, int apply_ldf, int ent_offset,
                                                  double* __restrict__ cell_ent_DG, double* __restrict__ cell_ent_FV,
-                                                 unsigned char* __restrict__ cell_ent_nan, int limit,
-                                                 const double* s_A, double* s_ldf, double* s_red, int* s_cnt,
+                                                 unsigned char* __restrict__ cell_ent_nan,
+                                                 const double* s_A, double* s_ldf, int* s_cnt,
                                                  const Stage1Src& s1,
                                                  double* bu, double* bk, long long next_chunk, GridRC npos) {
   using C = PPCfg<P>;
@@ -531,13 +577,6 @@ __device__ __forceinline__ void pp_avg_ldf_chunk(double* __restrict__ u, double*
 #pragma unroll
     for (int v0 = 0; v0 < 8; v0 += GS)
       if (node + v0 < 8) u_avg[e * 8 + node + v0] = mine[v0 / GS];
-  if (NEEDG && need_global) {
-    // chunk sum of (hx*hy)*avg over interior elements in element order (DG_solver.f90:227-229)
-    if (el < TE)
-#pragma unroll
-      for (int v0 = 0; v0 < 8; v0 += GS)
-        if (node + v0 < 8) s_red[el * 8 + node + v0] = inner ? (g.hx * g.hy) * mine[v0 / GS] : 0.0;
-  }
   // cell entropies for the entropy-offset limiter (DG_solver.f90:195-224)
   if (ent_offset) {
     const double pq = act ? node_prs(x, gamma) : 0.0;
@@ -551,54 +590,16 @@ __device__ __forceinline__ void pp_avg_ldf_chunk(double* __restrict__ u, double*
       cell_ent_nan[e] = okall > 0.5 ? 0 : 1;
     }
   }
-  // LDF projection of (Bx - avg, By - avg), on the sums and differences of mirror nodes (tables.h,
-  // ldf_table): butterflies along x and y, this lane's output place from at most 2 M^2 input places
-  // through the group's row, butterflies back.  The shared-memory pipe bounds this kernel, and the
-  // dense operator (2n^2 products an output) read its rows from there: 400^2 without / with the OEDG
-  // sums, p = 3: 92 -> 75 / 90 -> 61 us, p = 2: 77 -> 70 / 70 -> 61 us; p = 1, 500^2: 38.5 -> 37.7 us.
   if (apply_ldf) {
-    constexpr int M = (N + 1) / 2;
-    const int gb = lane - node;  // the group's first lane
-    const int mx = nd ? gb + (N - 1 - k) + N * l : lane, my = nd ? gb + k + N * (N - 1 - l) : lane;
-    const double sx = 2 * k < N - 1 ? 1.0 : (2 * k == N - 1 ? 0.0 : -1.0);
-    const double sy = 2 * l < N - 1 ? 1.0 : (2 * l == N - 1 ? 0.0 : -1.0);
-    double bx = x[4] - avg[4], by = x[5] - avg[5];
-    bx = __fma_rn(sx, __shfl_sync(FULL_MASK, bx, mx), bx);
-    by = __fma_rn(sx, __shfl_sync(FULL_MASK, by, mx), by);
-    bx = __fma_rn(sy, __shfl_sync(FULL_MASK, bx, my), bx);
-    by = __fma_rn(sy, __shfl_sync(FULL_MASK, by, my), by);
-    double2* in = reinterpret_cast<double2*>(row);
-    if (nd) in[node] = make_double2(bx, by);
-    __syncwarp();
-    double ox = 0.0, oy = 0.0;
-    if (nd) {
-      const double2* w = reinterpret_cast<const double2*>(s_A) + node;
-      const bool px = 2 * k > N - 1, py = 2 * l > N - 1;  // the parity of this lane's place
-#pragma unroll
-      for (int jy = 0; jy < M; ++jy)
-#pragma unroll
-        for (int jx = 0; jx < M; ++jx) {
-          const int s = jx + M * jy;
-          const double2 c = w[s * NN], f = in[(px ? N - 1 - jx : jx) + N * (py ? N - 1 - jy : jy)];
-          ox = __fma_rn(c.x, f.x, ox);
-          oy = __fma_rn(c.y, f.y, oy);
-          const double2 d = w[(s + M * M) * NN], h = in[(px ? jx : N - 1 - jx) + N * (py ? jy : N - 1 - jy)];
-          ox = __fma_rn(d.x, h.y, ox);
-          oy = __fma_rn(d.y, h.x, oy);
-        }
-    }
-    __syncwarp();  // the row is rewritten by the next chunk
-    ox = __fma_rn(-sy, __shfl_sync(FULL_MASK, ox, my), ox);
-    oy = __fma_rn(-sy, __shfl_sync(FULL_MASK, oy, my), oy);
-    ox = __fma_rn(-sx, __shfl_sync(FULL_MASK, ox, mx), ox);
-    oy = __fma_rn(-sx, __shfl_sync(FULL_MASK, oy, mx), oy);
+    double fx = x[4] - avg[4], fy = x[5] - avg[5];
+    ldf_project<P>(fx, fy, lane - node, node, nd, row, reinterpret_cast<const double2*>(s_A));
     if (valid) {
-      x[4] = ox + avg[4];
-      x[5] = oy + avg[5];
+      x[4] = fx + avg[4];
+      x[5] = fy + avg[5];
     }
   }
   bool neg = false, scaled = false;
-  if (!NEEDG && limit) {  // (the OEDG form is never fused: its damping comes first)
+  if constexpr (LIMIT) {
     __syncwarp();  // the group's lane 0 wrote the cell entropies limit_group reads
     limit_group<P>(x, avg, inner && nd, inner && node == 0, node, e, g, ctrl, ent_offset, 0, cell_ent_DG, cell_ent_FV,
                    cell_ent_nan, &neg, &scaled);
@@ -618,15 +619,6 @@ __device__ __forceinline__ void pp_avg_ldf_chunk(double* __restrict__ u, double*
       u[e * EB + 5 * NN + node] = x[5];
     }
   }
-  if (NEEDG && need_global) {
-    __syncthreads();
-    if (tid < 8) {
-      double sacc = 0.0;
-#pragma unroll 4
-      for (int q = 0; q < ne; ++q) sacc = sacc + s_red[q * 8 + tid];
-      partial_out[tid] = sacc;
-    }
-  }
 }
 
 
@@ -636,18 +628,15 @@ __device__ __forceinline__ void load_ldf(const double* __restrict__ A, double* s
 }
 
 // one CTA walks chunks blockIdx.x, blockIdx.x + gridDim.x, ... (the LDF operator is loaded once).
-// NEEDG: the OEDG form (need_global), with the per-chunk partial sums of the averages.
-template <int P, bool NEEDG>
+template <int P, bool LIMIT>
 __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB)
     pp_avg_ldf_kernel(double* __restrict__ u, double* __restrict__ u_avg, Geo g, Ctrl* ctrl,
-                      int gate, int apply_ldf, int need_global, int ent_offset,
-                      double* __restrict__ partial_sum,  // [chunks][8]
+                      int gate, int apply_ldf, int ent_offset,
                       double* __restrict__ cell_ent_DG, double* __restrict__ cell_ent_FV,
-                      unsigned char* __restrict__ cell_ent_nan, int limit, int nchunks, Stage1Src s1) {
+                      unsigned char* __restrict__ cell_ent_nan, int nchunks, Stage1Src s1) {
   using C = PPCfg<P>;
   __shared__ __align__(16) double s_A[ldf_table_doubles(P)];
   __shared__ __align__(16) double s_ldf[C::TE * (C::N2 + 2)];
-  __shared__ double s_red[2 * C::TE * 8];  // chunk sums, two buffers used in turn
   __shared__ __align__(16) double s_pf[(C::NT / 32) * 2 * C::G * C::EB];  // per warp: u (or u_con), k1
   __shared__ int s_cnt;
   if (threadIdx.x == 0) s_cnt = 0;
@@ -664,10 +653,7 @@ __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB)
   const GridRC stride = grid_rc((long long)gridDim.x * C::TE, NXG);
   GridRC pos = grid_rc((long long)blockIdx.x * C::TE, NXG);
   if (blockIdx.x < nchunks) pp_prefetch<P>(u, g, blockIdx.x, pos, s1, bu, bk);
-  // the chunk sums of consecutive chunks go to alternate halves of s_red: the barrier of chunk
-  // k + 1 orders the reads of chunk k before the writes of chunk k + 2
-  int half = 0;
-  for (int c = blockIdx.x; c < nchunks; c += gridDim.x, half ^= 1) {
+  for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
     cp_async_wait_all();
     __syncwarp();
     const long long nxt = c + gridDim.x < nchunks ? (long long)c + gridDim.x : -1;
@@ -676,19 +662,17 @@ __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB)
       npos.i -= NXG;
       ++npos.j;
     }
-    pp_avg_ldf_chunk<P, NEEDG, true>(u, u_avg, g, ctrl, c, pos, apply_ldf, need_global, ent_offset,
-                                     partial_sum + (long long)c * 8, cell_ent_DG, cell_ent_FV, cell_ent_nan, limit,
-                                     s_A, s_ldf, s_red + half * C::TE * 8, &s_cnt, s1, bu, bk, nxt, npos);
+    pp_avg_ldf_chunk<P, LIMIT, true>(u, u_avg, g, ctrl, c, pos, apply_ldf, ent_offset, cell_ent_DG, cell_ent_FV,
+                                     cell_ent_nan, s_A, s_ldf, &s_cnt, s1, bu, bk, nxt, npos);
     pos = npos;
   }
   __syncthreads();
   if (threadIdx.x == 0 && s_cnt) atomicAdd(&ctrl->num_negcell, s_cnt);
 }
 
-// many instances: items = every member's chunks; slot = the stage state; `final` selects the
-// final-stage form (OEDG global reductions for instances that use OEDG); the other stages fuse
-// loop 3 (limit)
-template <int P, bool FINAL>
+// many instances: items = every member's chunks; slot = the stage state; LIMIT: loop 3 fused (every
+// stage but the final one)
+template <int P, bool LIMIT>
 __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB > 3 ? 3 : PPCfg<P>::MINB)
     pp_avg_ldf_batched(const InstDesc* __restrict__ insts, const int* __restrict__ pref,
                        const int* __restrict__ nwork, const int* __restrict__ ninst, int slot, int gate,
@@ -696,7 +680,6 @@ __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB > 3 ? 3 : PPCfg<P
   using C = PPCfg<P>;
   __shared__ __align__(16) double s_A[ldf_table_doubles(P)];
   __shared__ __align__(16) double s_ldf[C::TE * (C::N2 + 2)];
-  __shared__ double s_red[C::TE * 8];  // chunk sums (the loop's barriers protect it)
   __shared__ int s_cnt;
   __shared__ SharedWalk s_walk;  // the walker's state, out of the registers the chunk needs
   if (threadIdx.x == 0) s_walk.start(pref, *ninst, *nwork);
@@ -717,10 +700,9 @@ __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB > 3 ? 3 : PPCfg<P
     if (threadIdx.x == 0) s_walk.advance(pref);
     if (open) {
       const Stage1Src s1 = stage1 ? Stage1Src{d.u[0], d.ut[1], &d.ctrl->dt, stage1_coef(d.R)} : Stage1Src{};
-      pp_avg_ldf_chunk<P, FINAL, false>(d.u[slot], d.u_avg, d.g, d.ctrl, chunk,
-                                        grid_rc((long long)chunk * C::TE, d.g.nx + 2), d.use_ldf, FINAL && d.use_oedg,
-                                        d.ent_offset, d.partial + (long long)chunk * 8, d.cell_ent_DG, d.cell_ent_FV,
-                                        d.cell_ent_nan, !FINAL, s_A, s_ldf, s_red, &s_cnt, s1,
+      pp_avg_ldf_chunk<P, LIMIT, false>(d.u[slot], d.u_avg, d.g, d.ctrl, chunk,
+                                        grid_rc((long long)chunk * C::TE, d.g.nx + 2), d.use_ldf, d.ent_offset,
+                                        d.cell_ent_DG, d.cell_ent_FV, d.cell_ent_nan, s_A, s_ldf, &s_cnt, s1,
                                         nullptr, nullptr, -1, GridRC{0, 0});
     }
     __syncthreads();  // the item is done; the walker has advanced
@@ -729,41 +711,74 @@ __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB > 3 ? 3 : PPCfg<P
 }
 
 // ---------------------------------------------------------------------------------------------
-// global average (fixed-order sum of block partials).  One CTA.
+// Global average (DG_solver.f90:227-229,282-286): the sum of (hx*hy)*avg over the interior elements, in a
+// fixed order.  An item is SUM_CHUNK consecutive elements of u_avg; the CTA that finishes the last item
+// of an instance adds up the items' partial sums.  Thread 8r + v takes variable v of every 32nd element.
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ void pp_reduce_body(const double* __restrict__ partial, int nblk, Ctrl* ctrl) {
-  __shared__ double s[8][256];
+constexpr int SUM_CHUNK = 1024;
+__host__ __device__ inline int pp_sum_chunks(int nx, int ny) {
+  return (int)(((long long)(nx + 2) * (ny + 2) + SUM_CHUNK - 1) / SUM_CHUNK);
+}
+
+// sum over the CTA's 32 rows of threads; threads 0..7 return the eight totals
+__device__ __forceinline__ double pp_sum_rows(double acc, double* s) {
   const int tid = threadIdx.x;
-  double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int b = tid; b < nblk; b += 256)
-#pragma unroll
-    for (int v = 0; v < 8; ++v) acc[v] = acc[v] + partial[b * 8 + v];
-#pragma unroll
-  for (int v = 0; v < 8; ++v) s[v][tid] = acc[v];
+  s[tid] = acc;
   __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (tid < w)
 #pragma unroll
-      for (int v = 0; v < 8; ++v) s[v][tid] = s[v][tid] + s[v][tid + w];
+  for (int w = 128; w >= 8; w >>= 1) {
+    if (tid < w) s[tid] = s[tid] + s[tid + w];
     __syncthreads();
   }
-  if (tid < 8) ctrl->u_avg_global[tid] = s[tid][0];
+  return s[tid & 7];
 }
 
-__global__ void __launch_bounds__(256) pp_reduce_kernel(const double* __restrict__ partial, int nblk,
+__device__ __forceinline__ void pp_sum_chunk(const double* __restrict__ u_avg, const Geo& g, int chunk, double* partial,
+                                             Ctrl* ctrl) {
+  __shared__ double s[256];
+  __shared__ bool s_last;
+  const int tid = threadIdx.x, v = tid & 7, nx = g.nx, ny = g.ny, nchunk = pp_sum_chunks(nx, ny);
+  const long long total = (long long)(nx + 2) * (ny + 2);
+  const long long e0 = (long long)chunk * SUM_CHUNK + (tid >> 3);
+  GridRC at = grid_rc(e0, nx + 2);
+  const double h2 = g.hx * g.hy;
+  double acc = 0.0;
+#pragma unroll 8
+  for (int q = 0; q < SUM_CHUNK / 32; ++q) {
+    const long long e = e0 + 32 * q;
+    if (e < total && at.i >= 1 && at.i <= nx && at.j >= 1 && at.j <= ny) acc = __dadd_rn(acc, __dmul_rn(h2, u_avg[e * 8 + v]));
+    at = grid_adv(at, 32, nx + 2);
+  }
+  acc = pp_sum_rows(acc, s);
+  if (tid < 8) partial[chunk * 8 + tid] = acc;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(&ctrl->sum_ticket, 1u) == (unsigned)nchunk - 1u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  acc = 0.0;
+  for (int b = tid >> 3; b < nchunk; b += 32) acc = __dadd_rn(acc, __ldcg(partial + b * 8 + v));
+  acc = pp_sum_rows(acc, s);
+  if (tid < 8) ctrl->u_avg_global[tid] = acc;
+  if (tid == 0) ctrl->sum_ticket = 0u;
+}
+
+__global__ void __launch_bounds__(256) pp_reduce_kernel(const double* __restrict__ u_avg, Geo g, double* partial,
                                                         Ctrl* ctrl, int gate) {
   if (!gate_open(ctrl, gate)) return;
-  pp_reduce_body(partial, nblk, ctrl);
+  pp_sum_chunk(u_avg, g, blockIdx.x, partial, ctrl);
 }
 
-// many instances: CTA per instance (persistent over the instance list)
-__global__ void __launch_bounds__(256) pp_reduce_batched(const InstDesc* __restrict__ insts,
-                                                         const int* __restrict__ ninst, int final, int gate) {
-  const int n = *ninst;
-  for (int i = blockIdx.x; i < n; i += gridDim.x) {
-    const InstDesc& d = insts[i];
-    if (!gate_open(d.ctrl, gate) || !(d.use_oedg && final)) continue;
-    pp_reduce_body(d.partial, d.nblk_avg, d.ctrl);
+// many instances: items = the chunks of every member (the final stage of those that use OEDG)
+__global__ void __launch_bounds__(256) pp_reduce_batched(const InstDesc* __restrict__ insts, const int* __restrict__ pref,
+                                                         const int* __restrict__ nwork, const int* __restrict__ ninst,
+                                                         int gate) {
+  const int nw = *nwork, n = *ninst;
+  for (BatchWalk it(pref, n, nw); it.more(); it.next()) {
+    const InstDesc& d = insts[it.m];
+    if (!gate_open(d.ctrl, gate) || !d.use_oedg) continue;
+    pp_sum_chunk(d.u_avg, d.g, it.local(), d.partial, d.ctrl);
     __syncthreads();
   }
 }

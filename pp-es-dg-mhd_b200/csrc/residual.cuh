@@ -6,21 +6,29 @@
 // Sums are formed in a fixed order, so the kernel is deterministic.
 #pragma once
 #include "common.cuh"
+#include "misc.cuh"
+#include "post.cuh"
 
 namespace mhd {
 
 // swap_xy (DG_solver.f90:1556-1568) as a variable permutation: 1 <-> 2, 4 <-> 5
 __host__ __device__ constexpr int swap_xy_var(int v) { return v == 1 ? 2 : v == 2 ? 1 : v == 4 ? 5 : v == 5 ? 4 : v; }
 
-// The next stage's SSP-RK combination folded into the residual (drive.f90:185-241 for SSP-RK3,
-// :148-183 for SSP-RK(2,2)): out = ca*u0 + cb*(u + dt*L(u)), rounded exactly as combine_value
-// forms it, written to the interior of the next stage's state instead of storing L(u).  Only
-// where that combination uses no other stage's L (u0 == nullptr: plain residual into ut).
-struct StageCombine {
+// What a residual leaves behind.  RES_UT: L(u), in ut.  RES_COMBINE, where the next stage's SSP-RK
+// combination uses no other stage's L (drive.f90:185-241 for SSP-RK3, :148-183 for SSP-RK(2,2)): in place of
+// L(u) that combination, out = ca*u0 + cb*(u + dt*L(u)), rounded exactly as combine_value forms it.
+// RES_POST: in addition loop 1 of the next stage's post-process (averages, admissibility, LDF projection,
+// cell entropies), with loop 3 where the stage is not the final one (see post.cuh, stage_post below).
+enum ResMode : int { RES_UT = 0, RES_COMBINE = 1, RES_POST = 2 };
+struct StagePost {
   const double* u0;     // u_con (ghosted layout)
   double* out;          // the next stage's state (ghosted layout)
   double ca, cb;
   const double* dt;     // the try's dt (device control block)
+  double* u_avg;        // from here on: RES_POST
+  double *cell_ent_DG, *cell_ent_FV;
+  unsigned char* cell_ent_nan;
+  int use_ldf, ent_offset, final;
 };
 
 // =============================================================================================
@@ -112,6 +120,7 @@ struct Res2Layout {
   static constexpr int O_NB = EY * SX * ES, O_NODE = O_NB;
   static constexpr int NB = 2 * EX * ES > 32 * NS ? 2 * EX * ES : 32 * NS;
   static constexpr int O_BAR = O_NB + NB, O_FACE = O_BAR + 2, WARP = O_FACE + NF * FS;
+  static_assert(NF * FS >= G * (2 * NN + 2) + ((NN & (NN - 1)) ? G * 8 * NN : 0), "stage_post's scratch fits the face records");
   static_assert(NCOPY <= 32 && (EB * 8) % 16 == 0 && (ES * 8) % 16 == 0, "one copy per lane, 16-byte blocks");
   static constexpr size_t BYTES = sizeof(double) * NW * WARP;
   static_assert((BYTES + 1024) * MINB <= 228 * 1024, "the CTAs of an SM fit its shared memory");
@@ -180,16 +189,125 @@ struct TileOut {
 __device__ __forceinline__ void st2(double* p, double a, double b) { *reinterpret_cast<double2*>(p) = make_double2(a, b); }
 __device__ __forceinline__ double2 ld2(const double* p) { return *reinterpret_cast<const double2*>(p); }
 
+// The next stage's element of this lane's group, from its combined node values x (ie, je: the element,
+// act: this lane holds one of its nodes, base: the group's first lane).  Where the element is the source of ghost
+// elements, those are formed first, as the boundary fill would from the values before the projection.
+// scratch: shared memory of the warp, free of use.  What a failing average leaves behind does not
+// matter: the try is abandoned then.
+//
+// In place of a boundary fill and loop 1 as launches of their own for every stage after the first: the
+// state is neither written before the projection nor read again, and the averages cost a lane no
+// more than its own node's sums.
+template <int P>
+__device__ __forceinline__ void stage_post(const double* x, const StagePost& sp, const Geo& g, Ctrl* ctrl, int ie,
+                                           int je, bool rim, bool act, int grp, int base, int node, double* scratch) {
+  using L = Res2Layout<P>;
+  constexpr int N = L::N, NN = L::NN, EB = L::EB, G = L::G;
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, k = node % N, l = node / N;
+  const bool nd = grp < G;  // (the lanes past the groups mirror the first)
+  const DegConst& dc = c_deg[P];
+  const double w = 0.25 * dc.qw[k] * dc.qw[l];
+  double* row = scratch + (nd ? grp : 0) * (2 * NN + 2);
+  // the left, right, bottom and top ghost of the element, where it is their source; then itself
+#pragma unroll 1
+  for (int side = rim ? 0 : 4; side <= 4; ++side) {
+    const int ti = side == 0 ? 0 : side == 1 ? g.nx + 1 : ie, tj = side == 2 ? 0 : side == 3 ? g.ny + 1 : je;
+    const bool ghost = side < 4;
+    bool mine = act;
+    double y[8];
+    if (ghost) {
+      const BcSrc b = bc_source<P>(g, ti, tj, 0, node);
+      const int si = b.fixed ? min(max(ti, 1), g.nx) : b.si, sj = b.fixed ? min(max(tj, 1), g.ny) : b.sj;
+      mine = act && si == ie && sj == je;
+      if (!__any_sync(FULL, mine)) continue;
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        const double t = __shfl_sync(FULL, x[v], base + b.sq);
+        y[v] = b.fixed ? g.bc_state[v] : (bc_source<P>(g, ti, tj, v, node).neg ? -t : t);
+      }
+    } else {
+#pragma unroll
+      for (int v = 0; v < 8; ++v) y[v] = x[v];
+    }
+    // cell averages (DG_solver.f90:177-184)
+    double avg[8];
+#pragma unroll
+    for (int v = 0; v < 8; ++v) avg[v] = w * y[v];
+    if constexpr ((NN & (NN - 1)) == 0) {
+      grp_sum8<NN>(avg, row);
+    } else {  // nine lanes: variable q is summed by lane q of the group
+      double* t = scratch + G * (2 * NN + 2) + (nd ? grp : 0) * (8 * NN);
+      if (nd)
+#pragma unroll
+        for (int v = 0; v < 8; ++v) t[v * NN + node] = avg[v];
+      __syncwarp();
+      if (nd && node < 8) {
+        const double* r = t + node * NN;
+        row[node] = (((r[0] + r[8]) + r[4]) + (r[2] + r[6])) + ((r[1] + r[5]) + (r[3] + r[7]));  // as grp_sum8 adds
+      }
+      __syncwarp();
+#pragma unroll
+      for (int v = 0; v < 8; v += 2) {
+        const double2 p = ld2(row + v);
+        avg[v] = p.x;
+        avg[v + 1] = p.y;
+      }
+    }
+    const long long e = (long long)tj * (g.nx + 2) + ti;
+    if (mine) {
+#pragma unroll
+      for (int v0 = 0; v0 < 8; v0 += NN)
+        if (node + v0 < 8) sp.u_avg[e * 8 + node + v0] = row[node + v0];
+    }
+    __syncwarp();  // the row is rewritten next
+    // admissibility of the average (DG_solver.f90:186-193)
+    const double pa = prs_of(avg[0], avg[1], avg[2], avg[3], avg[4], avg[5], avg[6], avg[7], g.gamma);
+    if (mine && node == 0 && (avg[0] < PP_EPS || pa < PP_EPS)) atomicOr(&ctrl->neg_avg, 1);
+    if (!ghost && sp.ent_offset) {  // cell entropies (DG_solver.f90:195-224)
+      const double pq = act ? node_prs(y, g.gamma) : 0.0;
+      const bool okq = !act || (y[0] >= PP_EPS && pq >= PP_EPS);
+      const double okall = grp_min<NN>(okq ? 1.0 : 0.0);
+      const double ce = grp_sum<NN>((act && okall > 0.5) ? 0.25 * g.hx * g.hy * dc.qw[k] * dc.qw[l] * ent_of(y[0], pq, g.gamma, g.igm1) : 0.0);
+      if (act && node == 0) {
+        sp.cell_ent_FV[e] = ent_of(avg[0], pa, g.gamma, g.igm1);
+        sp.cell_ent_DG[e] = okall > 0.5 ? ce : 0.0;
+        sp.cell_ent_nan[e] = okall > 0.5 ? 0 : 1;
+      }
+      __syncwarp();  // limit_group reads them
+    }
+    if (ghost && !sp.final) continue;  // the end of the stage fills its ghosts again
+    if (sp.use_ldf) {
+      double bx = y[4] - avg[4], by = y[5] - avg[5];
+      ldf_project<P>(bx, by, base, node, nd, row, reinterpret_cast<const double2*>(g.ldfA));
+      y[4] = bx + avg[4];
+      y[5] = by + avg[5];
+    }
+    if (!sp.final) {
+      bool neg = false;
+      limit_group<P, NN>(y, avg, act, node == 0, node, e, g, ctrl, sp.ent_offset, 0, sp.cell_ent_DG, sp.cell_ent_FV,
+                         sp.cell_ent_nan, &neg);
+      const unsigned cnt = __popc(__ballot_sync(FULL, neg));
+      if (lane == 0 && cnt) atomicAdd(&ctrl->num_negcell, (int)cnt);
+    }
+    if (mine) {
+      double* o = sp.out + e * EB + node;
+#pragma unroll
+      for (int v = 0; v < 8; ++v) o[v * NN] = y[v];
+    }
+  }
+}
+
 // One item: elements i0 = ix*EX + 1 .., j0 = iy*EY + 1 .. of the mesh (at least one of them inside).
 // wsm = the warp's shared memory (after res2_prologue).  ug = the array whose ghost
 // ring the boundary traces come from (u itself, or the last stage array whose ring was filled from
 // u's interior after the final stage; the interior always comes from u).  `phase` = the parity of the
 // warp's barrier (flipped here).  The whole warp calls it.  Returns false if the wait for the copies
 // ran out (FLAG_DEVICE_WAIT is then set): the warp must stop.
-template <int P>
+template <int P, int MODE>
 __device__ __forceinline__ bool residual_item(const double* __restrict__ u, const double* __restrict__ ug,
                                               const TileOut& to, const Geo& g, int ix, int iy, double* wsm,
-                                              unsigned& phase, const StageCombine& sc) {
+                                              unsigned& phase, const StagePost& sp) {
   using L = Res2Layout<P>;
   constexpr int N = L::N, NN = L::NN, EB = L::EB, EX = L::EX, EY = L::EY, NFX = L::NFX, NF = L::NF;
   constexpr int ES = L::ES, SX = L::SX;
@@ -448,19 +566,10 @@ __device__ __forceinline__ bool residual_item(const double* __restrict__ u, cons
 #pragma unroll
     for (int v = 1; v < 8; ++v) acc[v] = dfma(src, gp[v], acc[v]);
   }
-  if (act) {
-    if (sc.u0) {  // the next stage's state instead of L(u)
-      const long long e = ((long long)(j0 + gr) * (nx + 2) + (i0 + gc)) * EB + node;
-      const double dt = *sc.dt;
+  if (MODE == RES_UT && act) {
+    double* o = to.ut + ((long long)(j0 + gr - 1) * nx + (i0 + gc - 1)) * EB + node;
 #pragma unroll
-      for (int v = 0; v < 8; ++v)
-        sc.out[e + v * NN] = __dadd_rn(__dmul_rn(sc.ca, __ldg(sc.u0 + e + v * NN)),
-                                       __dmul_rn(sc.cb, __dadd_rn(un[v * NN], __dmul_rn(dt, acc[v]))));
-    } else {
-      double* o = to.ut + ((long long)(j0 + gr - 1) * nx + (i0 + gc - 1)) * EB + node;
-#pragma unroll
-      for (int v = 0; v < 8; ++v) o[v * NN] = acc[v];
-    }
+    for (int v = 0; v < 8; ++v) o[v * NN] = acc[v];
   }
   // dt_lim of an element: the largest node speed and interface speed per direction.  The exact
   // node speeds and maxima are only formed where the item could lower dt_lim: the largest bounds of
@@ -470,20 +579,43 @@ __device__ __forceinline__ bool residual_item(const double* __restrict__ u, cons
   const unsigned uy = __reduce_max_sync(FULL, __float_as_uint(__double2float_ru(act ? fmax(fy, sgy) : 0.0)));
   const double bound = (P + 0.5) * ((double)__uint_as_float(ux) * sxh + (double)__uint_as_float(uy) * syh);
   const double dt_now = __longlong_as_double((long long)__shfl_sync(FULL, dt_bits, 0));  // one value for the warp
-  if (bound * dt_now * (1.0 + 1.0e-12) <= 1.0) return true;
-  const double pf = s_node[lane * L::NS + 9], ir = rcp_nr(pp[0]);
-  const double cs = dmul(dmul(gamma, pf), ir), ss = dfma(bsq, ir, cs), coef = dmul(dmul(4.0, cs), ir);
-  auto speed = [&](double v, double bn) {  // |v| + the fast speed along the direction of bn (DG_solver.f90:784-787)
-    const double disc = at_least(dfma(ss, ss, -dmul(coef, dmul(bn, bn))), TINY);
-    return dadd(fabs(v), sqrt_nr(dmul(0.5, at_least(dadd(ss, sqrt_nr(disc)), TINY))));
-  };
-  const double ax = group_max<NN>(act ? fmax(fx, speed(pp[1], pp[4])) : 0.0, gbase);
-  const double ay = group_max<NN>(act ? fmax(fy, speed(pp[2], pp[5])) : 0.0, gbase);
-  double my_dt = 1.0e300;
-  if (act && node == 0) my_dt = 1.0 / dmul(P + 0.5, dfma(ax, sxh, dmul(ay, syh)));
+  if (!(bound * dt_now * (1.0 + 1.0e-12) <= 1.0)) {
+    const double pf = s_node[lane * L::NS + 9], ir = rcp_nr(pp[0]);
+    const double cs = dmul(dmul(gamma, pf), ir), ss = dfma(bsq, ir, cs), coef = dmul(dmul(4.0, cs), ir);
+    auto speed = [&](double v, double bn) {  // |v| + the fast speed along the direction of bn (DG_solver.f90:784-787)
+      const double disc = at_least(dfma(ss, ss, -dmul(coef, dmul(bn, bn))), TINY);
+      return dadd(fabs(v), sqrt_nr(dmul(0.5, at_least(dadd(ss, sqrt_nr(disc)), TINY))));
+    };
+    const double ax = group_max<NN>(act ? fmax(fx, speed(pp[1], pp[4])) : 0.0, gbase);
+    const double ay = group_max<NN>(act ? fmax(fy, speed(pp[2], pp[5])) : 0.0, gbase);
+    double my_dt = 1.0e300;
+    if (act && node == 0) my_dt = 1.0 / dmul(P + 0.5, dfma(ax, sxh, dmul(ay, syh)));
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) my_dt = fmin(my_dt, __shfl_xor_sync(FULL, my_dt, o));
-  if (lane == 0) atomicMin(&to.ctrl->dt_lim_bits, (unsigned long long)__double_as_longlong(my_dt));
+    for (int o = 16; o > 0; o >>= 1) my_dt = fmin(my_dt, __shfl_xor_sync(FULL, my_dt, o));
+    if (lane == 0) atomicMin(&to.ctrl->dt_lim_bits, (unsigned long long)__double_as_longlong(my_dt));
+  }
+  if constexpr (MODE != RES_UT) {  // the next stage
+    const int ie = i0 + gc, je = j0 + gr;
+    const long long at = ((long long)je * (nx + 2) + ie) * EB + node;
+    double x[8];
+#pragma unroll
+    for (int v = 0; v < 8; ++v) x[v] = 0.0;
+    if (act) {
+      const double dt = *sp.dt;
+#pragma unroll
+      for (int v = 0; v < 8; ++v)
+        x[v] = __dadd_rn(__dmul_rn(sp.ca, __ldg(sp.u0 + at + v * NN)), __dmul_rn(sp.cb, __dadd_rn(un[v * NN], __dmul_rn(dt, acc[v]))));
+    }
+    if constexpr (MODE == RES_COMBINE) {
+      if (act)
+#pragma unroll
+        for (int v = 0; v < 8; ++v) sp.out[at + v * NN] = x[v];
+    } else {
+      __syncwarp();  // the face records are read: their place is scratch from here on
+      const bool rim = i0 == 1 || j0 == 1 || i0 + EX > nx || j0 + EY > ny;  // an element on the boundary
+      stage_post<P>(x, sp, g, to.ctrl, ie, je, rim, act, grp, gbase, node, wsm + L::O_FACE);
+    }
+  }
   return true;
 }
 
@@ -494,10 +626,10 @@ template <int P>
 __host__ __device__ inline int res2_item_rows(int ny) { return (ny + Res2Layout<P>::EY - 1) / Res2Layout<P>::EY; }
 
 // single instance: one CTA per TX x TY block of elements (ug: the ghost-ring source, see residual_item)
-template <int P>
+template <int P, int MODE>
 __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
     residual2_kernel(const double* __restrict__ u, const double* __restrict__ ug, double* __restrict__ ut, Geo g,
-                     Ctrl* ctrl, int gate, StageCombine sc) {
+                     Ctrl* ctrl, int gate, StagePost sp) {
   using L = Res2Layout<P>;
   extern __shared__ __align__(16) double sm[];
   const int warp = threadIdx.x >> 5;
@@ -507,7 +639,7 @@ __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
   grid_begin();
   if (!gate_open(ctrl, gate) || ix * L::EX >= g.nx || iy * L::EY >= g.ny) return;
   unsigned phase = 0;
-  residual_item<P>(u, ug, TileOut{ut, ctrl}, g, ix, iy, wsm, phase, sc);
+  residual_item<P, MODE>(u, ug, TileOut{ut, ctrl}, g, ix, iy, wsm, phase, sp);
 }
 
 // single instance, persistent: the grid's warps take the items in turn (row-major, ncol per row).
@@ -526,16 +658,16 @@ __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
   res2_prologue<P>(wsm);
   unsigned phase = 0;
   for (int t = blockIdx.x * L::NW + warp; t < nitems; t += gridDim.x * L::NW)
-    if (!residual_item<P>(u, u, TileOut{ut, ctrl}, g, t % ncol, t / ncol, wsm, phase, StageCombine{}))
+    if (!residual_item<P, RES_UT>(u, u, TileOut{ut, ctrl}, g, t % ncol, t / ncol, wsm, phase, StagePost{}))
       return;
 }
 
 // many instances of degree P: each warp of a persistent grid walks its share of every member's items
 // (row-major per member); the state is slot `src`, the result goes to ut[dst], or (next_stage > 0)
-// the combination of stage next_stage goes to slot next_stage.  The item's arithmetic is fully
+// stage next_stage goes to slot next_stage (RES_POST).  The item's arithmetic is fully
 // rounded as written (explicit fused multiply-adds, see common.cuh), so a member is bitwise equal to
 // its solo run although this is a different kernel.
-template <int P>
+template <int P, int MODE>
 __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
     residual2_batched(const InstDesc* __restrict__ insts, const int* __restrict__ pref,
                       const int* __restrict__ nwork, const int* __restrict__ ninst, int src, int dst, int gate,
@@ -547,7 +679,7 @@ __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
   struct WarpArgs {
     SharedWalk walk;
     Geo g;
-    StageCombine sc;
+    StagePost sp;
     TileOut to;
   };
   __shared__ WarpArgs s_args[L::NW];
@@ -565,7 +697,9 @@ __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
     if (lane == 0) {
       if (open) {
         a.g = d.g;
-        a.sc = next_stage > 0 ? StageCombine{d.u[0], d.u[next_stage], ca, cb, &d.ctrl->dt} : StageCombine{};
+        if constexpr (MODE == RES_POST)
+          a.sp = StagePost{d.u[0], d.u[next_stage], ca, cb, &d.ctrl->dt, d.u_avg, d.cell_ent_DG, d.cell_ent_FV,
+                           d.cell_ent_nan, d.use_ldf, d.ent_offset, next_stage == d.R};
         a.to = TileOut{d.ut[dst], d.ctrl};
       }
       a.walk.advance(pref);
@@ -575,7 +709,7 @@ __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
       const int ncol = res2_item_cols<P>(a.g.nx);
       // the state after the final stage: u_con's interior with the last stage array's ghost ring
       const int srci = (src == d.R) ? 0 : src;
-      if (!residual_item<P>(d.u[srci], d.u[src], a.to, a.g, local % ncol, local / ncol, wsm, phase, a.sc))
+      if (!residual_item<P, MODE>(d.u[srci], d.u[src], a.to, a.g, local % ncol, local / ncol, wsm, phase, a.sp))
         return;
     }
   }
