@@ -3,7 +3,7 @@
 // A batch holds existing handles (each already through mhd_gpu_solve_begin).  Members are grouped
 // by (degree p, RK stages R).  Per group the batch keeps a device table of InstDesc entries and one
 // flattened work list per kernel kind: residual tiles, average/LDF chunks, OEDG indicator item
-// blocks, limiter row segments, combination blocks and ghost blocks, each entry (instance, a, b).
+// blocks, limiter row segments and ghost blocks, each entry (instance, a, b).
 // One SSP-RK try of every member is one CUDA graph: per group the batched kernels of the try
 // sequence (the same kernel bodies as the single-instance path, so each member's arithmetic is
 // identical alone and in the batch), groups on parallel branches.  The kernels are persistent
@@ -15,7 +15,7 @@
 
 namespace {
 
-enum WorkKind { WK_RES = 0, WK_AVG, WK_SUM, WK_SIG, WK_LIM, WK_CMB, WK_BC, WK_COUNT };
+enum WorkKind { WK_RES = 0, WK_AVG, WK_SUM, WK_SIG, WK_LIM, WK_BC, WK_COUNT };
 
 // One group's device table, one allocation, uploaded with one copy:
 //   InstDesc insts[cap] | int total[WK_COUNT] | int ninst | int pref[WK_COUNT][cap + 1]
@@ -105,7 +105,6 @@ void member_work(const mhd_gpu* h, long long* cnt, InstDesc& d) {
   constexpr int TEL = PPCfg<P>::TEL;  // the limiter's row segments
   d.nseg_limit = (int)(((nx + TEL - 1) / TEL) * ny);
   cnt[WK_LIM] = d.nseg_limit;
-  cnt[WK_CMB] = (nx * ny * EB + 255) / 256;
   cnt[WK_BC] = (2 * (nx + ny) * EB + 255) / 256;
 }
 
@@ -190,18 +189,16 @@ int full_grid(K kernel, int threads, size_t smem, int nsm) {
 }
 
 struct BatchGrids {
-  int res, res_post, cmb, bc, avg, avg_final, sum, sig, lim, seb;
+  int res, res_post, res_post54, avg, avg_final, sum, sig, lim, seb;
 };
 
 // queried before a capture begins (the occupancy calculator is host-only work)
 template <int P>
 BatchGrids batch_grids(int nsm) {
-  constexpr int EB = 8 * (P + 1) * (P + 1);
   BatchGrids gr;
   gr.res = full_grid(residual2_batched<P, RES_UT>, Res2Layout<P>::NT, Res2Layout<P>::BYTES, nsm);
   gr.res_post = full_grid(residual2_batched<P, RES_POST>, Res2Layout<P>::NT, Res2Layout<P>::BYTES, nsm);
-  gr.cmb = full_grid(combine_batched<EB>, 256, 0, nsm);
-  gr.bc = full_grid(bc_batched<P>, 256, 0, nsm);
+  gr.res_post54 = full_grid(residual2_batched<P, RES_POST54>, Res2Layout<P>::NT, Res2Layout<P>::BYTES, nsm);
   gr.avg = full_grid(pp_avg_ldf_batched<P, true>, PPCfg<P>::NT, 0, nsm);
   gr.avg_final = full_grid(pp_avg_ldf_batched<P, false>, PPCfg<P>::NT, 0, nsm);
   gr.sum = full_grid(pp_reduce_batched, 256, 0, nsm);
@@ -213,34 +210,26 @@ BatchGrids batch_grids(int nsm) {
 
 template <int P>
 void enqueue_group_try(mhd_batch* b, BatchGroup& g, const BatchGrids& gr, cudaStream_t st) {
-  constexpr int EB = 8 * (P + 1) * (P + 1);
   const int R = g.R;
   const int* tot = g.total();
   const int* ninst = g.ninst();
   InstDesc* in = g.insts();
   const size_t smem = Res2Layout<P>::BYTES;
   constexpr int NT_RES = Res2Layout<P>::NT;
-  const int grid_res = gr.res, grid_cmb = gr.cmb, grid_bc = gr.bc, grid_avg = gr.avg, grid_sig = gr.sig,
-            grid_lim = gr.lim;
+  const int grid_res = gr.res, grid_avg = gr.avg, grid_sig = gr.sig, grid_lim = gr.lim;
   ctl_batched<<<1, 256, 0, st>>>(in, ninst, CTL_STEP_BEGIN, R, 0);
   residual2_batched<P, RES_UT><<<grid_res, NT_RES, smem, st>>>(in, g.pref(WK_RES), tot + WK_RES, ninst, 0, 1,
-                                                               ST_RECOMPUTE, 0, 0.0, 0.0);
+                                                               ST_RECOMPUTE);
   ctl_batched<<<1, 256, 0, st>>>(in, ninst, CTL_DT_STAGE1, R, 1);  // dt, and the pseudo-time of stage 1
   for (int s = 1; s <= R; ++s) {
     const int fin = (s == R);
-    // stage 1: loop 1 forms the stage state and its ghost ring; SSP-RK(2,2)/(3,3): later stages
-    // come from the previous residual, with their loop 1
-    if (s > 1 && R > 3) {
-      combine_batched<EB><<<grid_cmb, 256, 0, st>>>(in, g.pref(WK_CMB), tot + WK_CMB, ninst, s, ST_RUN);
-      bc_batched<P><<<grid_bc, 256, 0, st>>>(in, g.pref(WK_BC), tot + WK_BC, ninst, s, ST_RUN);
-    }
-    if (s == 1 || R > 3) {
+    // stage 1: loop 1 forms the stage state and its ghost ring; later stages come from the previous
+    // residual, through loop 1 (fold_post)
+    if (s == 1) {
       if (fin)
-        pp_avg_ldf_batched<P, false><<<gr.avg_final, PPCfg<P>::NT, 0, st>>>(in, g.pref(WK_AVG), tot + WK_AVG, ninst, s, ST_RUN,
-                                                                     s == 1);
+        pp_avg_ldf_batched<P, false><<<gr.avg_final, PPCfg<P>::NT, 0, st>>>(in, g.pref(WK_AVG), tot + WK_AVG, ninst, ST_RUN);
       else
-        pp_avg_ldf_batched<P, true><<<grid_avg, PPCfg<P>::NT, 0, st>>>(in, g.pref(WK_AVG), tot + WK_AVG, ninst, s, ST_RUN,
-                                                                s == 1);
+        pp_avg_ldf_batched<P, true><<<grid_avg, PPCfg<P>::NT, 0, st>>>(in, g.pref(WK_AVG), tot + WK_AVG, ninst, ST_RUN);
     }
     if (fin) {
       pp_reduce_batched<<<gr.sum, 256, 0, st>>>(in, g.pref(WK_SUM), tot + WK_SUM, ninst, ST_RUN);
@@ -250,16 +239,12 @@ void enqueue_group_try(mhd_batch* b, BatchGroup& g, const BatchGrids& gr, cudaSt
     // entropy sum (final stage), stage-end decision, next stage's pseudo-time and the ghost rings
     stage_end_bc_batched<P><<<gr.seb, 256, 0, st>>>(in, g.pref(WK_BC), tot + WK_BC, ninst, s, R, fin ? 0 : s + 1,
                                                      fin);
-    // the coefficients of combine_value for SSP-RK(2,2) stage 2 and SSP-RK(3,3) stages 2, 3
-    const int nxt = (!fin && (R == 2 || R == 3)) ? s + 1 : 0;
-    const double ca = nxt == 0 ? 0.0 : (R == 2 ? 0.5 : (nxt == 2 ? 0.75 : 1.0 / 3.0));
-    const double cb = nxt == 0 ? 0.0 : (R == 2 ? 0.5 : (nxt == 2 ? 0.25 : 2.0 / 3.0));
-    if (nxt)
-      residual2_batched<P, RES_POST><<<gr.res_post, NT_RES, smem, st>>>(in, g.pref(WK_RES), tot + WK_RES, ninst, s, (s % R) + 1,
-                                                                    ST_RUN, nxt, ca, cb);
+    if (!fin && R > 3)
+      residual2_batched<P, RES_POST54><<<gr.res_post54, NT_RES, smem, st>>>(in, g.pref(WK_RES), tot + WK_RES, ninst, s, s + 1, ST_RUN);
+    else if (!fin)
+      residual2_batched<P, RES_POST><<<gr.res_post, NT_RES, smem, st>>>(in, g.pref(WK_RES), tot + WK_RES, ninst, s, s + 1, ST_RUN);
     else
-      residual2_batched<P, RES_UT><<<grid_res, NT_RES, smem, st>>>(in, g.pref(WK_RES), tot + WK_RES, ninst, s, (s % R) + 1,
-                                                                  ST_RUN, 0, 0.0, 0.0);
+      residual2_batched<P, RES_UT><<<grid_res, NT_RES, smem, st>>>(in, g.pref(WK_RES), tot + WK_RES, ninst, s, 1, ST_RUN);
   }
   ctl_batched<<<1, 256, 0, st>>>(in, ninst, CTL_STEP_END, R, 0);
 }

@@ -228,18 +228,24 @@ int init_device_tables(int dev) {
   CK(cudaFuncSetAttribute(residual2_kernel<1, RES_UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
   CK(cudaFuncSetAttribute(residual2_kernel<1, RES_COMBINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
   CK(cudaFuncSetAttribute(residual2_kernel<1, RES_POST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_kernel<1, RES_POST54>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
   CK(cudaFuncSetAttribute(residual2_kernel<2, RES_UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
   CK(cudaFuncSetAttribute(residual2_kernel<2, RES_COMBINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
   CK(cudaFuncSetAttribute(residual2_kernel<2, RES_POST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_kernel<2, RES_POST54>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
   CK(cudaFuncSetAttribute(residual2_kernel<3, RES_UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
   CK(cudaFuncSetAttribute(residual2_kernel<3, RES_COMBINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
   CK(cudaFuncSetAttribute(residual2_kernel<3, RES_POST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_kernel<3, RES_POST54>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
   CK(cudaFuncSetAttribute(residual2_batched<1, RES_UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
   CK(cudaFuncSetAttribute(residual2_batched<1, RES_POST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_batched<1, RES_POST54>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
   CK(cudaFuncSetAttribute(residual2_batched<2, RES_UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
   CK(cudaFuncSetAttribute(residual2_batched<2, RES_POST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_batched<2, RES_POST54>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
   CK(cudaFuncSetAttribute(residual2_batched<3, RES_UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
   CK(cudaFuncSetAttribute(residual2_batched<3, RES_POST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
+  CK(cudaFuncSetAttribute(residual2_batched<3, RES_POST54>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
   CK(cudaFuncSetAttribute(residual2_persistent<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<1>::BYTES));
   CK(cudaFuncSetAttribute(residual2_persistent<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<2>::BYTES));
   CK(cudaFuncSetAttribute(residual2_persistent<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Res2Layout<3>::BYTES));
@@ -300,7 +306,7 @@ void launch_residual(mhd_gpu* h, const double* u, double* ut, int gate, int mode
   using L = Res2Layout<P>;
   dim3 grid((h->nx + L::TX - 1) / L::TX, (h->ny + L::TY - 1) / L::TY);
   launch_next(h->stream, early_launch(h), grid, L::NT, L::BYTES, 
-              mode == RES_POST ? residual2_kernel<P, RES_POST> : mode == RES_COMBINE ? residual2_kernel<P, RES_COMBINE> : residual2_kernel<P, RES_UT>,
+              mode == RES_POST54 ? residual2_kernel<P, RES_POST54> : mode == RES_POST ? residual2_kernel<P, RES_POST> : mode == RES_COMBINE ? residual2_kernel<P, RES_COMBINE> : residual2_kernel<P, RES_UT>,
               u, ug ? ug : u, ut, h->geo, h->ctrl, gate, sp);
 }
 
@@ -450,17 +456,25 @@ void fill_status(const mhd_gpu* h, mhd_gpu_status* st) {
   st->pad_ = 0;
 }
 
-// stage `stage` (> 1) out of the previous residual, SSP-RK(2,2) and (3,3): the coefficients of combine_value
+// stage `stage` (> 1) out of the previous residual
 StagePost next_stage_post(const mhd_gpu* h, int stage) {
-  const double ca = h->R == 2 ? 0.5 : (stage == 2 ? 0.75 : 1.0 / 3.0), cb = h->R == 2 ? 0.5 : (stage == 2 ? 0.25 : 2.0 / 3.0);
-  return StagePost{h->u[0], h->u[stage], ca, cb, &h->ctrl->dt, h->u_avg, h->cell_ent_DG, h->cell_ent_FV, h->cell_ent_nan,
-                   h->use_ldf, h->ent_offset, stage == h->R};
+  StagePost sp{};
+  stage_scheme(sp, h->R, stage, h->u, h->ut);
+  sp.dt = &h->ctrl->dt;
+  sp.u_avg = h->u_avg;
+  sp.cell_ent_DG = h->cell_ent_DG;
+  sp.cell_ent_FV = h->cell_ent_FV;
+  sp.cell_ent_nan = h->cell_ent_nan;
+  sp.use_ldf = h->use_ldf;
+  sp.ent_offset = h->ent_offset;
+  return sp;
 }
 
 // Whether loop 1 of the stages after the first runs in the previous residual (RES_POST) or, with a boundary fill
 // before it, as launches of its own.  Folded a step is faster at every size.  Orszag-Tang, SSP-RK(3,3), launches ->
 // folded (us a step): p = 1, 16^2 65 -> 59, 128^2 89 -> 81, 512^2 500 -> 484; p = 2, 64^2 80 -> 75, 300^2 427 -> 409;
-// p = 3, 100^2 123 -> 117, 180^2 243 -> 243; vortex 512^2 p = 3 1607 -> 1539.  Below 1024 nodes, where
+// p = 3, 100^2 123 -> 117, 180^2 243 -> 243; vortex 512^2 p = 3 1607 -> 1539; SSP-RK(5,4), whose combination
+// was a launch too: p = 1, 64^2 110 -> 92; p = 2, 203x190 377 -> 311, 400^2 1306 -> 1053.  Below 1024 nodes, where
 // it is 2-4 us, a try keeps one launch per procedure, the sequence that step_graph_kernels is known by.
 bool fold_post(const mhd_gpu* h) { return (long long)h->nx * h->ny * h->nn >= 1024; }
 
@@ -471,16 +485,16 @@ void enqueue_try(mhd_gpu* h) {
   ctl_step_begin<<<1, 1, 0, h->stream>>>(h->ctrl);
   launch_residual_retry<P>(h, h->u[0], h->ut[1]);
   launch_next(h->stream, early_launch(h), 1, 1, 0, ctl_dt_stage1, h->ctrl, R);  // dt, and the pseudo-time of stage 1
-  // SSP-RK(2,2) and (3,3): stages after the first take their combination from the previous stage's
-  // residual, with loop 1 (fold_post) or without; SSP-RK(1,1) and (5,4) keep the separate combine
-  const int mode = R != 2 && R != 3 ? RES_UT : fold_post(h) ? RES_POST : RES_COMBINE;
+  // stages after the first come from the previous stage's residual, through loop 1 (fold_post), or take their
+  // combination from it (SSP-RK(2,2), (3,3)) or from a launch of its own (SSP-RK(5,4))
+  const int mode = fold_post(h) ? (R > 3 ? RES_POST54 : RES_POST) : R == 2 || R == 3 ? RES_COMBINE : RES_UT;
   constexpr int EB = 8 * (P + 1) * (P + 1);
   const long long nghost = 2LL * (h->nx + h->ny) * EB;
   const int nseg = (int)(pp_grid_limit<P>(h).x * pp_grid_limit<P>(h).y);
   for (int s = 1; s <= R; ++s) {
     const int fin = (s == R);
     // stage 1: loop 1 forms the stage state and its ghost ring (Stage1Src)
-    const bool posted = s > 1 && mode == RES_POST;
+    const bool posted = s > 1 && mode >= RES_POST;
     if (s > 1 && mode == RES_UT) launch_combine<P>(h, s, &h->ctrl->dt, 0.0, ST_RUN);
     if (s > 1 && !posted) launch_bc<P>(h, h->u[s], ST_RUN);
     const Stage1Src s1 = s == 1 ? Stage1Src{h->u[0], h->ut[1], &h->ctrl->dt, stage1_coef(R)} : Stage1Src{};

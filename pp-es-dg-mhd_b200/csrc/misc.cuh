@@ -88,20 +88,6 @@ __global__ void __launch_bounds__(256) bc_kernel(double* __restrict__ u, Geo g, 
   bc_value<P>(u, u, g, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// many instances: items = every member's blocks of 256 ghost values
-template <int P>
-__global__ void __launch_bounds__(256) bc_batched(const InstDesc* __restrict__ insts, const int* __restrict__ pref,
-                                                  const int* __restrict__ nwork, const int* __restrict__ ninst,
-                                                  int slot, int gate) {
-  const int nw = *nwork, n = *ninst;
-  for (BatchWalk it(pref, n, nw); it.more(); it.next()) {
-    const int m = it.m, chunk = it.local();
-    const InstDesc& d = insts[m];
-    if (!gate_open(d.ctrl, gate)) continue;
-    bc_value<P>(d.u[slot], d.u[slot], d.g, (long long)chunk * 256 + threadIdx.x);
-  }
-}
-
 // SSP-RK stage update (drive.f90:130-275) on interior elements, rounded exactly as written
 // (explicit _rn intrinsics: no fused multiply-add contraction).
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
@@ -162,21 +148,6 @@ __global__ void __launch_bounds__(256)
   const double dt = dt_ptr ? *dt_ptr : dt_arg;
   combine_value<EB>(u0, r1, r2, r3, r4, k1, k2, k3, k4, k5, out, nx, ny, R, stage, dt,
                     (long long)blockIdx.x * blockDim.x + threadIdx.x);
-}
-
-// many instances: items = every member's blocks of 256 values; dt from each member's control block
-template <int EB>
-__global__ void __launch_bounds__(256) combine_batched(const InstDesc* __restrict__ insts, const int* __restrict__ pref,
-                                                       const int* __restrict__ nwork, const int* __restrict__ ninst,
-                                                       int stage, int gate) {
-  const int nw = *nwork, n = *ninst;
-  for (BatchWalk it(pref, n, nw); it.more(); it.next()) {
-    const int m = it.m, chunk = it.local();
-    const InstDesc& d = insts[m];
-    if (!gate_open(d.ctrl, gate)) continue;
-    combine_value<EB>(d.u[0], d.u[1], d.u[2], d.u[3], d.u[4], d.ut[1], d.ut[2], d.ut[3], d.ut[4], d.ut[5],
-                      d.u[stage], d.g.nx, d.g.ny, d.R, stage, d.ctrl->dt, (long long)chunk * 256 + threadIdx.x);
-  }
 }
 
 // Fortran layout (8, n, n, E) <-> element-blocked layout [E][8][n*n].  E = element count.

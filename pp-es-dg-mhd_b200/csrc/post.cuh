@@ -670,13 +670,12 @@ __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB)
   if (threadIdx.x == 0 && s_cnt) atomicAdd(&ctrl->num_negcell, s_cnt);
 }
 
-// many instances: items = every member's chunks; slot = the stage state; LIMIT: loop 3 fused (every
-// stage but the final one)
+// many instances, stage 1: items = every member's chunks; LIMIT: loop 3 fused (unless the stage is the
+// final one)
 template <int P, bool LIMIT>
 __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB > 3 ? 3 : PPCfg<P>::MINB)
     pp_avg_ldf_batched(const InstDesc* __restrict__ insts, const int* __restrict__ pref,
-                       const int* __restrict__ nwork, const int* __restrict__ ninst, int slot, int gate,
-                       int stage1) {
+                       const int* __restrict__ nwork, const int* __restrict__ ninst, int gate) {
   using C = PPCfg<P>;
   __shared__ __align__(16) double s_A[ldf_table_doubles(P)];
   __shared__ __align__(16) double s_ldf[C::TE * (C::N2 + 2)];
@@ -699,8 +698,8 @@ __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB > 3 ? 3 : PPCfg<P
     __syncthreads();  // every thread has read the walker; s_A and s_cnt are in place
     if (threadIdx.x == 0) s_walk.advance(pref);
     if (open) {
-      const Stage1Src s1 = stage1 ? Stage1Src{d.u[0], d.ut[1], &d.ctrl->dt, stage1_coef(d.R)} : Stage1Src{};
-      pp_avg_ldf_chunk<P, LIMIT, false>(d.u[slot], d.u_avg, d.g, d.ctrl, chunk,
+      const Stage1Src s1{d.u[0], d.ut[1], &d.ctrl->dt, stage1_coef(d.R)};
+      pp_avg_ldf_chunk<P, LIMIT, false>(d.u[1], d.u_avg, d.g, d.ctrl, chunk,
                                         grid_rc((long long)chunk * C::TE, d.g.nx + 2), d.use_ldf, d.ent_offset,
                                         d.cell_ent_DG, d.cell_ent_FV, d.cell_ent_nan, s_A, s_ldf, &s_cnt, s1,
                                         nullptr, nullptr, -1, GridRC{0, 0});

@@ -14,22 +14,73 @@ namespace mhd {
 // swap_xy (DG_solver.f90:1556-1568) as a variable permutation: 1 <-> 2, 4 <-> 5
 __host__ __device__ constexpr int swap_xy_var(int v) { return v == 1 ? 2 : v == 2 ? 1 : v == 4 ? 5 : v == 5 ? 4 : v; }
 
-// What a residual leaves behind.  RES_UT: L(u), in ut.  RES_COMBINE, where the next stage's SSP-RK
-// combination uses no other stage's L (drive.f90:185-241 for SSP-RK3, :148-183 for SSP-RK(2,2)): in place of
-// L(u) that combination, out = ca*u0 + cb*(u + dt*L(u)), rounded exactly as combine_value forms it.
-// RES_POST: in addition loop 1 of the next stage's post-process (averages, admissibility, LDF projection,
-// cell entropies), with loop 3 where the stage is not the final one (see post.cuh, stage_post below).
-enum ResMode : int { RES_UT = 0, RES_COMBINE = 1, RES_POST = 2 };
+// What a residual leaves behind.  RES_UT: L(u), in ut.  RES_COMBINE, SSP-RK(2,2) and (3,3): in place of
+// L(u) the next stage's SSP-RK combination (drive.f90:185-241, :148-183), rounded exactly as combine_value
+// forms it.  RES_POST, and RES_POST54 for SSP-RK(5,4): in addition loop 1 of the next stage's post-process (averages,
+// admissibility, LDF projection, cell entropies), with loop 3 where the stage is not the final one (see
+// post.cuh, stage_post below).  (One kernel for both kinds of scheme costs SSP-RK(3,3) 0.5-1.5 %.)
+enum ResMode : int { RES_UT = 0, RES_COMBINE = 1, RES_POST = 2, RES_POST54 = 3 };
 struct StagePost {
   const double* u0;     // u_con (ghosted layout)
   double* out;          // the next stage's state (ghosted layout)
-  double ca, cb;
+  double ca, cb;        // stage_value's coefficients
   const double* dt;     // the try's dt (device control block)
   double* u_avg;        // from here on: RES_POST
   double *cell_ent_DG, *cell_ent_FV;
   unsigned char* cell_ent_nan;
   int use_ldf, ent_offset, final;
+  int stage;            // the stage formed; from here on: RES_POST54
+  double cc;            // SSP-RK(5,4): the coefficient of dt*L(u)
+  const double *r2, *r3;  // stage 5: the states of stages 2 and 3 (ghosted layout)
+  double* k4;             // stages 4 and 5: L of stage 3 (interior layout), written by the first, read by the second
 };
+
+// stage s > 1 of an R-stage scheme from the previous stage's residual (the coefficients of combine_value);
+// u, ut: the instance's arrays.
+__host__ __device__ inline void stage_scheme(StagePost& sp, int R, int s, double* const* u, double* const* ut) {
+  sp.u0 = u[0];
+  sp.out = u[s];
+  sp.final = s == R;
+  sp.stage = s;
+  if (R == 2) {
+    sp.ca = sp.cb = 0.5;
+  } else if (R == 3) {
+    sp.ca = s == 2 ? 0.75 : 1.0 / 3.0;
+    sp.cb = s == 2 ? 0.25 : 2.0 / 3.0;
+  } else {
+    sp.ca = s == 2 ? 0.444370493651235 : s == 3 ? 0.620101851488403 : s == 4 ? 0.178079954393132 : 0.386708617503269;
+    sp.cb = s == 2 ? 0.555629506348765 : s == 3 ? 0.379898148511597 : s == 4 ? 0.821920045606868 : 0.0;
+    sp.cc = s == 2 ? 0.368410593050371 : s == 3 ? 0.251891774271694 : s == 4 ? 0.544974750228521 : 0.226007483236906;
+    sp.r2 = u[2];
+    sp.r3 = u[3];
+    sp.k4 = ut[4];
+  }
+}
+
+// A node of the next stage, rounded as combine_value rounds it: x = its eight values, NN apart in memory; u = the
+// current stage's state there, k = its L; at, ki: the node's place in the ghosted and in the interior layout.
+template <int NN, int MODE>
+__device__ __forceinline__ void stage_node(double* x, const StagePost& sp, double dt, const double* u, const double* k,
+                                           long long at, long long ki) {
+  if constexpr (MODE != RES_POST54) {
+#pragma unroll
+    for (int v = 0; v < 8; ++v) x[v] = add(mul(sp.ca, __ldg(sp.u0 + at + v * NN)), mul(sp.cb, add(u[v * NN], mul(dt, k[v]))));
+  } else if (sp.stage < 5) {
+    const double cdt = mul(sp.cc, dt);
+    if (sp.stage == 4)
+#pragma unroll
+      for (int v = 0; v < 8; ++v) sp.k4[ki + v * NN] = k[v];
+#pragma unroll
+    for (int v = 0; v < 8; ++v)
+      x[v] = add(add(mul(sp.ca, __ldg(sp.u0 + at + v * NN)), mul(sp.cb, u[v * NN])), mul(cdt, k[v]));
+  } else {
+    const double cdt = mul(sp.cc, dt), c4 = mul(0.063692468666290, dt);
+#pragma unroll
+    for (int v = 0; v < 8; ++v)
+      x[v] = add(add(add(add(mul(0.517231671970585, __ldg(sp.r2 + at + v * NN)), mul(0.096059710526147, __ldg(sp.r3 + at + v * NN))),
+                         mul(c4, __ldg(sp.k4 + ki + v * NN))), mul(sp.ca, u[v * NN])), mul(cdt, k[v]));
+  }
+}
 
 // =============================================================================================
 // One warp per item, one lane per node.
@@ -596,15 +647,13 @@ __device__ __forceinline__ bool residual_item(const double* __restrict__ u, cons
   }
   if constexpr (MODE != RES_UT) {  // the next stage
     const int ie = i0 + gc, je = j0 + gr;
-    const long long at = ((long long)je * (nx + 2) + ie) * EB + node;
+    const long long at = ((long long)je * (nx + 2) + ie) * EB + node, ki = ((long long)(je - 1) * nx + (ie - 1)) * EB + node;
     double x[8];
 #pragma unroll
     for (int v = 0; v < 8; ++v) x[v] = 0.0;
     if (act) {
       const double dt = *sp.dt;
-#pragma unroll
-      for (int v = 0; v < 8; ++v)
-        x[v] = __dadd_rn(__dmul_rn(sp.ca, __ldg(sp.u0 + at + v * NN)), __dmul_rn(sp.cb, __dadd_rn(un[v * NN], __dmul_rn(dt, acc[v]))));
+      stage_node<NN, MODE>(x, sp, dt, un, acc, at, ki);
     }
     if constexpr (MODE == RES_COMBINE) {
       if (act)
@@ -663,15 +712,14 @@ __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
 }
 
 // many instances of degree P: each warp of a persistent grid walks its share of every member's items
-// (row-major per member); the state is slot `src`, the result goes to ut[dst], or (next_stage > 0)
-// stage next_stage goes to slot next_stage (RES_POST).  The item's arithmetic is fully
+// (row-major per member); the state is slot `src`, the result goes to ut[dst], or stage
+// dst to slot dst (RES_POST).  The item's arithmetic is fully
 // rounded as written (explicit fused multiply-adds, see common.cuh), so a member is bitwise equal to
 // its solo run although this is a different kernel.
 template <int P, int MODE>
 __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
     residual2_batched(const InstDesc* __restrict__ insts, const int* __restrict__ pref,
-                      const int* __restrict__ nwork, const int* __restrict__ ninst, int src, int dst, int gate,
-                      int next_stage, double ca, double cb) {
+                      const int* __restrict__ nwork, const int* __restrict__ ninst, int src, int dst, int gate) {
   using L = Res2Layout<P>;
   extern __shared__ __align__(16) double sm[];
   // per warp: the walker and the member's geometry, stage combination and outputs, read where they
@@ -697,9 +745,17 @@ __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
     if (lane == 0) {
       if (open) {
         a.g = d.g;
-        if constexpr (MODE == RES_POST)
-          a.sp = StagePost{d.u[0], d.u[next_stage], ca, cb, &d.ctrl->dt, d.u_avg, d.cell_ent_DG, d.cell_ent_FV,
-                           d.cell_ent_nan, d.use_ldf, d.ent_offset, next_stage == d.R};
+        if constexpr (MODE >= RES_POST)
+        {
+          stage_scheme(a.sp, d.R, dst, d.u, d.ut);
+          a.sp.dt = &d.ctrl->dt;
+          a.sp.u_avg = d.u_avg;
+          a.sp.cell_ent_DG = d.cell_ent_DG;
+          a.sp.cell_ent_FV = d.cell_ent_FV;
+          a.sp.cell_ent_nan = d.cell_ent_nan;
+          a.sp.use_ldf = d.use_ldf;
+          a.sp.ent_offset = d.ent_offset;
+        }
         a.to = TileOut{d.ut[dst], d.ctrl};
       }
       a.walk.advance(pref);
