@@ -141,9 +141,11 @@ int pp_resident_ctas(int dev) {
   return cached[dev];
 }
 
-// Page-locked slots, each the size of a control block, for what a call reads back and waits for: such a copy is
-// one DMA, a pageable one is staged by the driver (a residual with its dt_lim, 33 x 31, p = 1: 34.3 -> 32.4 us).  One
-// fixed array per process, made with the first device's tables; who finds no slot free uses pageable
+// Page-locked slots, each the size of a control block, for what a call reads back and waits for.  A last small
+// kernel writes it there (publish_kernel), started while the one before it still runs: a copy costs a
+// switch to the copy engine and back.  Copy -> kernel (us): residual with its dt_lim, 33 x 31, p = 1: 33.5 -> 24.3; one
+// step of Orszag-Tang 64^2, p = 2: 101.7 -> 96.3; step from separate calls, 160 x 144, p = 3: 399 -> 374.
+// One fixed array per process, made with the first device's tables; who finds no slot free copies to pageable
 // memory.  Slots are taken and given back under a lock, by instances (for life) and by single calls.
 class HostSlots {
  public:
@@ -165,6 +167,10 @@ class HostSlots {
     free_.pop_back();
     return slots_ + i;
   }
+  bool owns(const Ctrl* c) {
+    std::lock_guard<std::mutex> lk(m_);
+    return slots_ && c >= slots_ && c < slots_ + kSlots;
+  }
   bool give(Ctrl* c) {  // false: not a slot
     std::lock_guard<std::mutex> lk(m_);
     if (!slots_ || c < slots_ || c >= slots_ + kSlots) return false;
@@ -185,7 +191,13 @@ int read_double(const unsigned long long* src, double* out, cudaStream_t st) {
   unsigned long long local = 0;
   Ctrl* slot = g_host_slots.take();
   unsigned long long* bits = slot ? &slot->dt_lim_bits : &local;
-  cudaError_t e = cudaMemcpyAsync(bits, src, sizeof(*bits), cudaMemcpyDeviceToHost, st);
+  cudaError_t e;
+  if (slot) {
+    launch_next(st, true, 1, 32, 0, publish_kernel, src, bits, 1, nullptr);
+    e = cudaGetLastError();
+  } else {
+    e = cudaMemcpyAsync(bits, src, sizeof(*bits), cudaMemcpyDeviceToHost, st);
+  }
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e == cudaSuccess) std::memcpy(out, bits, sizeof(*out));
   if (slot) g_host_slots.give(slot);
@@ -407,8 +419,16 @@ void launch_diag(mhd_gpu* h, const double* u, int gate) {
     }                                       \
   } while (0)
 
-int read_ctrl(mhd_gpu* h) {
-  CK(cudaMemcpyAsync(h->ctrl_host, h->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->stream));
+// the control block to its host mirror, and wait; lift: the step budget ends
+int read_ctrl(mhd_gpu* h, bool lift = false) {
+  if (g_host_slots.owns(h->ctrl_host)) {
+    launch_next(h->stream, true, 1, 32, 0, publish_kernel, reinterpret_cast<unsigned long long*>(h->ctrl),
+                reinterpret_cast<unsigned long long*>(h->ctrl_host), (int)(sizeof(Ctrl) / 8), lift ? h->ctrl : nullptr);
+    CK(cudaGetLastError());
+  } else {
+    if (lift) ctl_step_budget<<<1, 1, 0, h->stream>>>(h->ctrl, -1);
+    CK(cudaMemcpyAsync(h->ctrl_host, h->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->stream));
+  }
   CK(cudaStreamSynchronize(h->stream));
   return MHD_OK;
 }
@@ -1043,7 +1063,8 @@ int mhd_gpu_advance(mhd_gpu_t* h, long long max_steps, int check_every, mhd_gpu_
   }
   // The step budget lives on the device and is set and lifted by kernels around each round of tries, so
   // that a round waits for the device once, when it reads the status (before: a read, two writes of the
-  // budget and three waits a call; one step of Orszag-Tang 64^2, p = 2: 117 -> 102 us).
+  // budget and three waits a call; one step of Orszag-Tang 64^2, p = 2: 117 -> 102 us).  The last one is
+  // the kernel that reads the status (read_ctrl).
   const Ctrl* c = h->ctrl_host;
   long long left = (max_steps > 0) ? max_steps : NO_STEP_LIMIT;
   do {
@@ -1052,9 +1073,8 @@ int mhd_gpu_advance(mhd_gpu_t* h, long long max_steps, int check_every, mhd_gpu_
     const int batch = (int)std::min<long long>(left, check_every);
     ctl_step_budget<<<1, 1, 0, h->stream>>>(h->ctrl, left);
     for (int b = 0; b < batch; ++b) CK(cudaGraphLaunch(h->step_exec, h->stream));
-    ctl_step_budget<<<1, 1, 0, h->stream>>>(h->ctrl, -1);
     CK(cudaGetLastError());
-    rc = read_ctrl(h);
+    rc = read_ctrl(h, /*lift=*/true);
     if (rc) return rc;
     rc = drain_log(h);
     if (rc) return rc;

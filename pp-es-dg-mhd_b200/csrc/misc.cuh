@@ -392,6 +392,15 @@ __global__ void ctl_step_budget(Ctrl* c, long long more) {
   c->step_limit = (c->done || c->flags) ? c->steps : (more > NO_STEP_LIMIT - c->steps ? NO_STEP_LIMIT : c->steps + more);
 }
 
+// What a call reads back, written by the device into its page-locked slot (`words` 8-byte words).
+// lift: the control block whose step budget ends with this.  One warp.
+__global__ void publish_kernel(const unsigned long long* src, unsigned long long* host, int words, Ctrl* lift) {
+  grid_begin();
+  if (lift && threadIdx.x == 0) lift->step_limit = NO_STEP_LIMIT;
+  __syncwarp();
+  for (int i = threadIdx.x; i < words; i += 32) host[i] = src[i];
+}
+
 __global__ void ctl_step_end(Ctrl* c, int R, LogEntry* log, int log_cap) {
   grid_begin();
   ctl_step_end_body(c, R, log, log_cap);
