@@ -2,10 +2,10 @@
 //
 //   pp_avg_ldf_kernel   loop 1 (DG_solver.f90:161-277): cell averages of every interior and
 //                       non-corner ghost element, admissibility of the average, the LDF projection
-//                       of (Bx,By) as one dense nodal operator, and (for OEDG) per-chunk partial
-//                       sums of the average.  In the time-step pipeline a stage without OEDG also
-//                       runs loop 3 here (fused).
-//   pp_reduce_kernel    the global average sum in a fixed order (DG_solver.f90:282-286).
+//                       of (Bx,By) as one dense nodal operator.  In the time-step pipeline a stage
+//                       without OEDG also runs loop 3 here (fused), and the stages after the first
+//                       mostly run loops 1 and 3 in the previous residual (stage_post, residual.cuh).
+//   pp_reduce_kernel    the global average sum in a fixed order (DG_solver.f90:227-229,282-286).
 //   pp_sigsum_kernel    the OEDG face jump indicators OEDG_sigsum_x/y (DG_solver.f90:295-422), and
 //                       the max and min of the post-LDF interior node values (read from the tile
 //                       it stages anyway).
@@ -25,9 +25,9 @@
 // 8 variables in registers.  Loads and stores of a variable are then 8*NN-byte runs per group
 // (coalesced), per-element sums, minima and maxima are reductions inside the group (butterflies for
 // power-of-two groups, a fold plus a butterfly for the 9-lane groups; every lane ends with the same
-// value), and no CTA-wide barrier sits between the steps of one element.  A CTA of NT threads handles a chunk of TE = (NT/32) * (32/GS) consecutive
-// elements; per-chunk partial sums are formed in element order.  The single-instance loop-1
-// kernel is a persistent grid over the chunks in which each warp copies its elements of the next
+// value), and no CTA-wide barrier sits between the steps of one element.  A CTA of NT threads handles
+// a chunk of TE = (NT/32) * (32/GS) consecutive elements.  The single-instance loop-1 kernel is a
+// persistent grid over the chunks in which each warp copies its elements of the next
 // chunk into shared memory (cp.async) while it works on the current one.  In the first stage of
 // a time step loop 1 also forms the stage state from u_con and k1 (Stage1Src).  The indicator
 // kernel stages each tile of elements in shared memory with cp.async, row by row.
@@ -713,6 +713,7 @@ __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB > 3 ? 3 : PPCfg<P
 // Global average (DG_solver.f90:227-229,282-286): the sum of (hx*hy)*avg over the interior elements, in a
 // fixed order.  An item is SUM_CHUNK consecutive elements of u_avg; the CTA that finishes the last item
 // of an instance adds up the items' partial sums.  Thread 8r + v takes variable v of every 32nd element.
+// Bound by latency (512^2: 258 CTAs, 17 MB out of L2); alone it runs beside the face indicators.
 // ---------------------------------------------------------------------------------------------
 constexpr int SUM_CHUNK = 1024;
 __host__ __device__ inline int pp_sum_chunks(int nx, int ny) {

@@ -106,7 +106,8 @@ __device__ __forceinline__ void stage_node(double* x, const StagePost& sp, doubl
 //               pair (each such pair has exactly one endpoint of each kind)
 //   4. the interface fluxes from their records, the Godunov-Powell terms, dt_lim, the store.
 // What bounds it, by counters at p = 3: issue slots (59 %), the shared-memory pipe (64 %, p = 2 78 %)
-// and the FP64 pipe (53 %) are all half taken by 16 warps per SM (126 registers); leaving out the flux
+// and the FP64 pipe (55 %) are all half taken by 16 warps per SM (126 registers).  A warp waits 1.7 cycles an
+// instruction for its own FP64 results, 1.1 for the copies, 0.8 for its turn; leaving out the flux
 // arithmetic saves only 10 %, and at 18-20 warps (96 registers) the spills cost more than the warps
 // bring.  Before it a CTA owned a tile and shared its interface fluxes between two barriers: 400 x 400,
 // p = 3 214 us -> 173 us, p = 2 blast 140 -> 121, 700 x 700 p = 1 201 -> 155; the interface fluxes cost
@@ -247,8 +248,11 @@ __device__ __forceinline__ double2 ld2(const double* p) { return *reinterpret_ca
 // matter: the try is abandoned then.
 //
 // In place of a boundary fill and loop 1 as launches of their own for every stage after the first: the
-// state is neither written before the projection nor read again, and the averages cost a lane no
-// more than its own node's sums.
+// state is neither written before the projection nor read again.  400^2, p = 3, one stage (us): residual
+// with its combination 176 + fill 3 + loop 1 61-75 -> 240-250 and 330 MB less traffic; on small meshes two
+// launches less a stage (fold_post, mhd_gpu.cu).  Staging u_con's blocks with the others by bulk copies gains 1.3 % of
+// a step where the state exceeds L2 and costs 1-2 % elsewhere and 4 % of a batch; fetching them to L2
+// ahead gains nothing.
 template <int P>
 __device__ __forceinline__ void stage_post(const double* x, const StagePost& sp, const Geo& g, Ctrl* ctrl, int ie,
                                            int je, bool rim, bool act, int grp, int base, int node, double* scratch) {
