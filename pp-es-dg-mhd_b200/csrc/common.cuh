@@ -129,10 +129,12 @@ __host__ __device__ constexpr int ldf_table_doubles(int p) {
   return 2 * (p + 1) * (p + 1) * 2 * ((p + 2) / 2) * ((p + 2) / 2);
 }
 
-// Launch of a kernel of a chain, each of which waits by grid_begin.  `early`: its CTAs may start while
-// its predecessor in the stream still runs.
+// Launch of a kernel of a chain, each of which waits by grid_begin: its CTAs may start while its predecessor in
+// the stream still runs, so that the end of one kernel hides the start of the next.  Plain -> early (us a step): p = 1, 48^2
+// (a run of 0.25 time units) 9.3 -> 8.5 ms, 512^2 486 -> 475; p = 2, 400^2 blast 691 -> 683; p = 3, 200^2
+// 338 -> 332, 512^2 vortex 1506 -> 1494.  Nearest to a loss: p = 3, 250^2 413 -> 414.
 template <typename... K, typename... A>
-void launch_next(cudaStream_t st, bool early, dim3 grid, int block, size_t smem, void (*kernel)(K...), A... args) {
+void launch_next(cudaStream_t st, dim3 grid, int block, size_t smem, void (*kernel)(K...), A... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -142,7 +144,7 @@ void launch_next(cudaStream_t st, bool early, dim3 grid, int block, size_t smem,
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
-  cfg.numAttrs = early ? 1 : 0;
+  cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
 }
 

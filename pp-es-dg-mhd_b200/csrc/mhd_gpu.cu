@@ -193,7 +193,7 @@ int read_double(const unsigned long long* src, double* out, cudaStream_t st) {
   unsigned long long* bits = slot ? &slot->dt_lim_bits : &local;
   cudaError_t e;
   if (slot) {
-    launch_next(st, true, 1, 32, 0, publish_kernel, src, bits, 1, nullptr);
+    launch_next(st, 1, 32, 0, publish_kernel, src, bits, 1, nullptr);
     e = cudaGetLastError();
   } else {
     e = cudaMemcpyAsync(bits, src, sizeof(*bits), cudaMemcpyDeviceToHost, st);
@@ -296,19 +296,11 @@ int enter(const mhd_gpu* h) {
 }
 
 // ---- launchers ---------------------------------------------------------------------------
-// Kernels of a small state are over in a few microseconds each, a large part of which is the start of their
-// CTAs: there each kernel is launched while its predecessor runs.  On a large state the early CTAs take
-// slots and shared memory from the predecessor's last wave instead.  A step of Orszag-Tang, SSP-RK(3,3),
-// without -> with (us): p = 1, 256^2 (0.26 million nodes): 218 -> 205; p = 3, 140^2 (0.31): 219 -> 210; p = 3,
-// 200^2 (0.64): 338 -> 332; p = 2, 320^2 (0.92): 526 -> 528; p = 1, 512^2 (1.05): 539 -> 547; p = 2, 400^2 (1.44):
-// 749 -> 774.
-bool early_launch(const mhd_gpu* h) { return (long long)h->nx * h->ny * h->nn <= 3LL << 18; }
-
 template <int P>
 void launch_bc(mhd_gpu* h, double* u, int gate) {
   constexpr int EB = 8 * (P + 1) * (P + 1);
   const long long n = 2LL * (h->nx + h->ny) * EB;
-  launch_next(h->stream, early_launch(h), grid1d(n, 256), 256, 0, bc_kernel<P>, u, h->geo, h->ctrl, gate);
+  launch_next(h->stream, grid1d(n, 256), 256, 0, bc_kernel<P>, u, h->geo, h->ctrl, gate);
 }
 
 // ug: the array whose ghost ring the boundary halos come from (nullptr: u's own)
@@ -317,7 +309,7 @@ void launch_residual(mhd_gpu* h, const double* u, double* ut, int gate, int mode
                      const StagePost& sp = StagePost{}, const double* ug = nullptr) {
   using L = Res2Layout<P>;
   dim3 grid((h->nx + L::TX - 1) / L::TX, (h->ny + L::TY - 1) / L::TY);
-  launch_next(h->stream, early_launch(h), grid, L::NT, L::BYTES, 
+  launch_next(h->stream, grid, L::NT, L::BYTES, 
               mode == RES_POST54 ? residual2_kernel<P, RES_POST54> : mode == RES_POST ? residual2_kernel<P, RES_POST> : mode == RES_COMBINE ? residual2_kernel<P, RES_COMBINE> : residual2_kernel<P, RES_UT>,
               u, ug ? ug : u, ut, h->geo, h->ctrl, gate, sp);
 }
@@ -341,7 +333,7 @@ template <int P>
 void launch_residual_retry(mhd_gpu* h, const double* u, double* ut) {
   using L = Res2Layout<P>;
   const int ncol = res2_item_cols<P>(h->nx), nitems = ncol * res2_item_rows<P>(h->ny);
-  launch_next(h->stream, early_launch(h), std::min(grid1d(nitems, L::NW), res_resident_ctas<P>(h->device)), L::NT, L::BYTES,
+  launch_next(h->stream, std::min(grid1d(nitems, L::NW), res_resident_ctas<P>(h->device)), L::NT, L::BYTES,
               residual2_persistent<P>, u, ut, h->geo, h->ctrl, ST_RECOMPUTE, ncol, nitems);
 }
 
@@ -349,7 +341,7 @@ template <int P>
 void launch_combine(mhd_gpu* h, int stage, const double* dt_ptr, double dt, int gate) {
   constexpr int EB = 8 * (P + 1) * (P + 1);
   const long long n = (long long)h->nx * h->ny * EB;
-  launch_next(h->stream, early_launch(h), grid1d(n, 256), 256, 0, combine_kernel<EB>,
+  launch_next(h->stream, grid1d(n, 256), 256, 0, combine_kernel<EB>,
               h->u[0], h->u[1], h->R >= 2 ? h->u[2] : nullptr, h->R >= 3 ? h->u[3] : nullptr, h->R >= 4 ? h->u[4] : nullptr,
               h->ut[1], h->R >= 2 ? h->ut[2] : nullptr, h->R >= 3 ? h->ut[3] : nullptr, h->R >= 4 ? h->ut[4] : nullptr,
               h->R >= 5 ? h->ut[5] : nullptr, h->u[stage], h->nx, h->ny, h->R, stage, dt_ptr, dt, h->ctrl, gate);
@@ -373,7 +365,7 @@ void launch_post(mhd_gpu* h, int slot, int apply_oedg, int apply_ldf, const doub
   if (!loop1_done) {
     const int nb1 = pp_nblk_avg<P>(h);
     const int grid1 = std::min(nb1, limit_in_loop1 ? pp_resident_ctas<P, true>(h->device) : pp_resident_ctas<P, false>(h->device));
-    launch_next(h->stream, early_launch(h), grid1, PPCfg<P>::NT, 0, limit_in_loop1 ? pp_avg_ldf_kernel<P, true> : pp_avg_ldf_kernel<P, false>,
+    launch_next(h->stream, grid1, PPCfg<P>::NT, 0, limit_in_loop1 ? pp_avg_ldf_kernel<P, true> : pp_avg_ldf_kernel<P, false>,
                 h->u[slot], h->u_avg, h->geo, h->ctrl, gate, apply_ldf, ent_offset, h->cell_ent_DG, h->cell_ent_FV,
                 h->cell_ent_nan, nb1, s1);
   }
@@ -384,7 +376,7 @@ void launch_post(mhd_gpu* h, int slot, int apply_oedg, int apply_ldf, const doub
     pp_reduce_kernel<<<pp_sum_chunks(h->nx, h->ny), 256, 0, h->side_stream>>>(h->u_avg, h->geo, h->partial, h->ctrl, gate);
     cudaEventRecord(h->ev_join, h->side_stream);
     const dim3 gs((h->nx + SigCfg<P>::TX - 1) / SigCfg<P>::TX, (h->ny + SigCfg<P>::TY - 1) / SigCfg<P>::TY);
-    launch_next(h->stream, early_launch(h), gs, 256, 0, pp_sigsum_kernel<P>, h->u[slot], h->geo, h->ctrl, gate, h->sig_x, h->sig_y);
+    launch_next(h->stream, gs, 256, 0, pp_sigsum_kernel<P>, h->u[slot], h->geo, h->ctrl, gate, h->sig_x, h->sig_y);
     cudaStreamWaitEvent(h->stream, h->ev_join, 0);
   }
   dim3 g3 = pp_grid_limit<P>(h);
@@ -392,12 +384,12 @@ void launch_post(mhd_gpu* h, int slot, int apply_oedg, int apply_ldf, const doub
     if (apply_oedg)  // after the join: a plain launch, which waits for both
       pp_limit_kernel<P><<<g3, PPCfg<P>::NT, 0, h->stream>>>(args...);
     else
-      launch_next(h->stream, early_launch(h), g3, PPCfg<P>::NT, 0, pp_limit_kernel<P>, args...);
+      launch_next(h->stream, g3, PPCfg<P>::NT, 0, pp_limit_kernel<P>, args...);
   };
   limit(h->u[slot], h->u_avg, h->geo, h->ctrl, gate, apply_oedg, dt_ptr, oedg_dt, ent_offset, comput_ent, h->sig_x,
         h->sig_y, h->cell_ent_DG, h->cell_ent_FV, h->cell_ent_nan, h->ent_partial, accept_dst, accept_only);
   if (comput_ent && !entsum_later)
-    launch_next(h->stream, early_launch(h), 1, 256, 0, pp_entsum_kernel, h->ent_partial, (int)(g3.x * g3.y), h->ctrl, gate);
+    launch_next(h->stream, 1, 256, 0, pp_entsum_kernel, h->ent_partial, (int)(g3.x * g3.y), h->ctrl, gate);
 }
 
 // stage diagnostics of state u into the newest log record
@@ -405,7 +397,7 @@ template <int P>
 void launch_diag(mhd_gpu* h, const double* u, int gate) {
   const long long E = (long long)h->nx * h->ny;
   const int nb = (int)std::min<long long>(DIAG_MAX_BLOCKS, std::max<long long>(1, E / 16));
-  launch_next(h->stream, early_launch(h), nb, 256, 0, stage_diag_kernel<P>, u, h->geo, h->ctrl, gate,
+  launch_next(h->stream, nb, 256, 0, stage_diag_kernel<P>, u, h->geo, h->ctrl, gate,
               h->diag_part, reinterpret_cast<unsigned int*>(h->diag_part + DIAG_VALS * DIAG_MAX_BLOCKS), h->log,
               h->log_cap);
 }
@@ -422,7 +414,7 @@ void launch_diag(mhd_gpu* h, const double* u, int gate) {
 // the control block to its host mirror, and wait; lift: the step budget ends
 int read_ctrl(mhd_gpu* h, bool lift = false) {
   if (g_host_slots.owns(h->ctrl_host)) {
-    launch_next(h->stream, true, 1, 32, 0, publish_kernel, reinterpret_cast<unsigned long long*>(h->ctrl),
+    launch_next(h->stream, 1, 32, 0, publish_kernel, reinterpret_cast<unsigned long long*>(h->ctrl),
                 reinterpret_cast<unsigned long long*>(h->ctrl_host), (int)(sizeof(Ctrl) / 8), lift ? h->ctrl : nullptr);
     CK(cudaGetLastError());
   } else {
@@ -504,7 +496,7 @@ void enqueue_try(mhd_gpu* h) {
   const int R = h->R;
   ctl_step_begin<<<1, 1, 0, h->stream>>>(h->ctrl);
   launch_residual_retry<P>(h, h->u[0], h->ut[1]);
-  launch_next(h->stream, early_launch(h), 1, 1, 0, ctl_dt_stage1, h->ctrl, R);  // dt, and the pseudo-time of stage 1
+  launch_next(h->stream, 1, 1, 0, ctl_dt_stage1, h->ctrl, R);  // dt, and the pseudo-time of stage 1
   // stages after the first come from the previous stage's residual, through loop 1 (fold_post), or take their
   // combination from it (SSP-RK(2,2), (3,3)) or from a launch of its own (SSP-RK(5,4))
   const int mode = fold_post(h) ? (R > 3 ? RES_POST54 : RES_POST) : R == 2 || R == 3 ? RES_COMBINE : RES_UT;
@@ -526,7 +518,7 @@ void enqueue_try(mhd_gpu* h) {
                    fin ? h->u[0] : nullptr, ST_RUN, 1, s1, /*entsum_later=*/true, /*accept_only=*/fin, posted);
     const double* cur = fin ? h->u[0] : h->u[s];  // the stage result's interior
     // entropy sum (final stage), stage-end decision, next stage's pseudo-time and the ghost ring
-    launch_next(h->stream, early_launch(h), grid1d(nghost, 256), 256, 0, stage_end_bc_kernel<P>,
+    launch_next(h->stream, grid1d(nghost, 256), 256, 0, stage_end_bc_kernel<P>,
                 cur, h->u[s], h->geo, h->ctrl, R, s, fin ? 0 : s + 1, fin ? h->ent_partial : nullptr, nseg, h->log,
                 h->log_cap);
     if (h->diag) launch_diag<P>(h, cur, ST_RUN);
@@ -535,7 +527,7 @@ void enqueue_try(mhd_gpu* h) {
     else
       launch_residual<P>(h, cur, nullptr, ST_RUN, mode, next_stage_post(h, s + 1), h->u[s]);
   }
-  launch_next(h->stream, early_launch(h), 1, 1, 0, ctl_step_end, h->ctrl, R, h->log, h->log_cap);
+  launch_next(h->stream, 1, 1, 0, ctl_step_end, h->ctrl, R, h->log, h->log_cap);
 }
 
 // kernel nodes of a graph (every launch of the captured try, gated ones included)
