@@ -360,6 +360,18 @@ __device__ __forceinline__ double sqrt_nr(double x) {
   const double h = dmul(x, y), t = dfma(-h, dmul(0.5, y), 0.5);
   return dfma(dmul(h, t), dfma(1.5, t, 1.0), h);
 }
+// The same where an argument may lie outside: 1/0 and 1/inf as the division gives them (a subnormal number
+// counts as zero), sqrt(0) = 0 and sqrt(inf) = inf.
+__device__ __forceinline__ double rcp_any(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = dfma(-x, r, 1.0), q = dfma(r, dfma(e, e, e), r);
+  return q == q ? q : r;
+}
+__device__ __forceinline__ double sqrt_any(double x) {  // x >= 0
+  const double s = sqrt_nr(x);
+  return s == s ? s : x;
+}
 
 // _macro_prs_ (DG_solver.f90:125), its quotient as a product with rcp_nr
 __device__ __forceinline__ double prs_of(double rho, double mx, double my, double mz, double bx,

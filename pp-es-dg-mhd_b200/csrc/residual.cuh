@@ -455,7 +455,7 @@ __device__ __forceinline__ bool residual_item(const double* __restrict__ u, cons
     double w[8];
 #pragma unroll
     for (int v = 0; v < 8; ++v) w[v] = un[v * NN];
-    const double ir = rcp_nr(w[0]);
+    const double ir = rcp_any(w[0]);
     const double vx = dmul(ir, w[1]), vy = dmul(ir, w[2]), vz = dmul(ir, w[3]);
     bsq = dsq3(w[4], w[5], w[6]);
     const double pf = gas_pressure(dsub(gamma, 1.0), ddot3(w[1], vx, w[2], vy, w[3], vz), bsq, w[7]);
@@ -629,17 +629,19 @@ __device__ __forceinline__ bool residual_item(const double* __restrict__ u, cons
   // dt_lim of an element: the largest node speed and interface speed per direction.  The exact
   // node speeds and maxima are only formed where the item could lower dt_lim: the largest bounds of
   // the whole warp, rounded up to single precision, bound every element's dt from below (1e-12 covers
-  // the rounding of the bound and of the exact value; a NaN speed or an empty dt_lim takes the exact path).
-  const unsigned ux = __reduce_max_sync(FULL, __float_as_uint(__double2float_ru(act ? fmax(fx, sgx) : 0.0)));
-  const unsigned uy = __reduce_max_sync(FULL, __float_as_uint(__double2float_ru(act ? fmax(fy, sgy) : 0.0)));
+  // the rounding of the bound and of the exact value).  A node's bound that is NaN, as where its density is negative
+  // or zero, stays NaN here (at_least, not fmax), orders above all others, and like an empty dt_lim takes the
+  // exact path, where only what is NaN itself is left out.
+  const unsigned ux = __reduce_max_sync(FULL, __float_as_uint(__double2float_ru(act ? at_least(fx, sgx) : 0.0)));
+  const unsigned uy = __reduce_max_sync(FULL, __float_as_uint(__double2float_ru(act ? at_least(fy, sgy) : 0.0)));
   const double bound = (P + 0.5) * ((double)__uint_as_float(ux) * sxh + (double)__uint_as_float(uy) * syh);
   const double dt_now = __longlong_as_double((long long)__shfl_sync(FULL, dt_bits, 0));  // one value for the warp
   if (!(bound * dt_now * (1.0 + 1.0e-12) <= 1.0)) {
-    const double pf = s_node[lane * L::NS + 9], ir = rcp_nr(pp[0]);
+    const double pf = s_node[lane * L::NS + 9], ir = rcp_any(pp[0]);
     const double cs = dmul(dmul(gamma, pf), ir), ss = dfma(bsq, ir, cs), coef = dmul(dmul(4.0, cs), ir);
     auto speed = [&](double v, double bn) {  // |v| + the fast speed along the direction of bn (DG_solver.f90:784-787)
       const double disc = at_least(dfma(ss, ss, -dmul(coef, dmul(bn, bn))), TINY);
-      return dadd(fabs(v), sqrt_nr(dmul(0.5, at_least(dadd(ss, sqrt_nr(disc)), TINY))));
+      return dadd(fabs(v), sqrt_any(dmul(0.5, at_least(dadd(ss, sqrt_any(disc)), TINY))));
     };
     const double ax = group_max<NN>(act ? fmax(fx, speed(pp[1], pp[4])) : 0.0, gbase);
     const double ay = group_max<NN>(act ? fmax(fy, speed(pp[2], pp[5])) : 0.0, gbase);
