@@ -533,8 +533,13 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
     if (s != 4) d[s] = dsub(f[1][s], f[0][s]);
   }
   d[4] = 0.0;
-  // Roe's weights with one root, s = sqrt(rho_l rho_r): both quotients over (sqrt rho_l + sqrt rho_r)^2
-  const double s_rho = sqrt_nr(dmul(wl[0], wr[0])), irs = rcp_nr(dfma(2.0, s_rho, rho_s));
+  // Roe's weights with one root, s = sqrt(rho_l rho_r): both quotients over (sqrt rho_l + sqrt rho_r)^2.
+  // A density that is not positive makes them NaN, with them the speeds and so the whole flux, as the
+  // logarithms and roots of each density do in the reference (the product of two negative ones is positive:
+  // it takes the left one's sign).
+  const double rho_p = dmul(wl[0], wr[0]);
+  const double s_rho = sqrt_nr(__hiloint2double(__double2hiint(rho_p) | (__double2hiint(wl[0]) & (int)0x80000000), __double2loint(rho_p)));
+  const double irs = rcp_nr(dfma(2.0, s_rho, rho_s));
   const double vx_roe = dmul(dfma(s_rho, dadd(v[0][0], v[1][0]), dadd(wl[1], wr[1])), irs);
   const double db = sqrt_nr(dfma(dsq3(j[4], j[5], j[6]), irs, TINY));
   const double sl_pp = dsub(dsub(at_most(vx_roe, v[0][0]), cf[0]), db);
@@ -558,8 +563,8 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
   const double al = at_least(dmul(b[0], ia), 0.0);
   const double ar = at_least(dmul(b[1], ia), 0.0);
   const double aa = sqrt_nr(dfma(al, ar, TINY));
-  const double sl = at_most(sl_pp, -dadd(ar, aa));  // (never above zero: ar, aa >= 0)
-  const double sr = at_least(sr_pp, dadd(al, aa));
+  const double sl = at_most(-dadd(ar, aa), sl_pp);  // (never above zero: ar, aa >= 0; NaN where sl_pp is)
+  const double sr = at_least(dadd(al, aa), sr_pp);
   const double idsl = rcp_nr(dsub(sr, sl));
   // (sr fl - sl fr)/(sr - sl) from the side with the larger weight, plus the other weight (at most
   // 1/2) times the difference: equal states give exactly their flux, a supersonic face its upwind one

@@ -618,8 +618,11 @@ __device__ __forceinline__ bool residual_item(const double* __restrict__ u, cons
     }
     const double gp[8] = {0.0, pp[4], pp[5], pp[6], pp[1], pp[2], pp[3],
                           ddot3(pp[4], pp[1], pp[5], pp[2], pp[6], pp[3])};
+    // The terms with a factor of zero that the reference's sum has matter where a value is not finite: the
+    // vector's mass part, and the energy's own flux, in which alone an energy that is NaN is not clamped away.
 #pragma unroll
-    for (int v = 1; v < 8; ++v) acc[v] = dfma(src, gp[v], acc[v]);
+    for (int v = 0; v < 8; ++v) acc[v] = dfma(src, gp[v], acc[v]);
+    acc[7] = dfma(0.0, un[7 * NN], acc[7]);
   }
   if (MODE == RES_UT && act) {
     double* o = to.ut + ((long long)(j0 + gr - 1) * nx + (i0 + gc - 1)) * EB + node;
