@@ -1112,15 +1112,20 @@ __device__ __forceinline__ void pp_limit_segment(const LimitIO& io, const Geo& g
     double sx = 0.0, sy = 0.0;
     if (act) {
       const double rho = at_least(x[0], PP_EPS);
-      const double ir = rcp_nr(rho);
+      const double ir = rcp_any(rho);
       const double vx = ir * x[1], vy = ir * x[2];
       const double ek = 0.5 * ir * (x[1] * x[1] + x[2] * x[2] + x[3] * x[3]);
       const double bx = x[4], by = x[5], bz = x[6];
       const double bsq = bx * bx + by * by + bz * bz;
       const double pf = at_least((gamma - 1.0) * (x[7] - (ek + 0.5 * bsq)), PP_EPS);
       const double cs = gamma * pf * ir, ss = cs + bsq * ir, sqsq = ss * ss, coef = 4.0 * cs * ir;
-      sx = fabs(vx) + sqrt_nr(0.5 * at_least(ss + sqrt_nr(at_least(sqsq - coef * (bx * bx), TINY)), TINY));
-      sy = fabs(vy) + sqrt_nr(0.5 * at_least(ss + sqrt_nr(at_least(sqsq - coef * (by * by), TINY)), TINY));
+      const double dx = at_least(sqsq - coef * (bx * bx), TINY), dy = at_least(sqsq - coef * (by * by), TINY);
+      sx = fabs(vx) + sqrt_nr(0.5 * at_least(ss + sqrt_nr(dx), TINY));
+      sy = fabs(vy) + sqrt_nr(0.5 * at_least(ss + sqrt_nr(dy), TINY));
+      if (!(dx + dy < 1.0e270)) {  // beyond sqrt_nr: an infinite speed damps to the average
+        sx = fabs(vx) + sqrt_any(0.5 * at_least(ss + sqrt_any(dx), TINY));
+        sy = fabs(vy) + sqrt_any(0.5 * at_least(ss + sqrt_any(dy), TINY));
+      }
     }
     const double mx = grp_max_nonneg<GS>(sx), my = grp_max_nonneg<GS>(sy);
     // lane `node` of the group forms delta_v for v = node, node + GS, ... from the element's four faces
@@ -1138,7 +1143,7 @@ __device__ __forceinline__ void pp_limit_segment(const LimitIO& io, const Geo& g
         const double gs = ctrl->u_avg_global[v];
         const double uv = at_least(fmax(ord_dec(ctrl->umax_bits[v]) - gs, gs - ord_dec(ctrl->umin_bits[v])), 0.0);
         if (uv > OEDG_EPS)
-          d = at_least((wx * (sig_x[fxl + v] + sig_x[fxl + 8 + v]) + wy * (sig_y[fyb + v] + sig_y[fyt + v])) * rcp_nr(uv), d);
+          d = at_least((wx * (sig_x[fxl + v] + sig_x[fxl + 8 + v]) + wy * (sig_y[fyb + v] + sig_y[fyt + v])) * rcp_any(uv), d);
       }
     }
     const double dmax = grp_max_nonneg<GS>(d);
