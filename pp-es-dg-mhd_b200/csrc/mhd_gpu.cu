@@ -525,7 +525,7 @@ void enqueue_try(mhd_gpu* h) {
     if (fin || mode == RES_UT)
       launch_residual<P>(h, cur, h->ut[(s % R) + 1], ST_RUN, RES_UT, StagePost{}, h->u[s]);
     else
-      launch_residual<P>(h, cur, nullptr, ST_RUN, mode, next_stage_post(h, s + 1), h->u[s]);
+      launch_residual<P>(h, cur, h->ut[s + 1], ST_RUN, mode, next_stage_post(h, s + 1), h->u[s]);
   }
   launch_next(h->stream, 1, 1, 0, ctl_step_end, h->ctrl, R, h->log, h->log_cap);
 }

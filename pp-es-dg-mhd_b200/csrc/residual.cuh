@@ -16,9 +16,10 @@ __host__ __device__ constexpr int swap_xy_var(int v) { return v == 1 ? 2 : v == 
 
 // What a residual leaves behind.  RES_UT: L(u), in ut.  RES_COMBINE, SSP-RK(2,2) and (3,3): in place of
 // L(u) the next stage's SSP-RK combination (drive.f90:185-241, :148-183), rounded exactly as combine_value
-// forms it.  RES_POST, and RES_POST54 for SSP-RK(5,4): in addition loop 1 of the next stage's post-process (averages,
-// admissibility, LDF projection, cell entropies), with loop 3 where the stage is not the final one (see
-// post.cuh, stage_post below).  (One kernel for both kinds of scheme costs SSP-RK(3,3) 0.5-1.5 %.)
+// forms it.  RES_POST: in addition loop 1 of the next stage's post-process (averages, admissibility, LDF projection,
+// cell entropies), with loop 3 where the stage is not the final one (see post.cuh, stage_post below).
+// RES_POST54, SSP-RK(5,4): the same and L(u), in ut: stage 5 reads that of stage 4, and all are the run's
+// ut_con(:,2..5).  (One kernel for both kinds of scheme costs SSP-RK(3,3) 0.5-1.5 %.)
 enum ResMode : int { RES_UT = 0, RES_COMBINE = 1, RES_POST = 2, RES_POST54 = 3 };
 struct StagePost {
   const double* u0;     // u_con (ghosted layout)
@@ -32,7 +33,7 @@ struct StagePost {
   int stage;            // the stage formed; from here on: RES_POST54
   double cc;            // SSP-RK(5,4): the coefficient of dt*L(u)
   const double *r2, *r3;  // stage 5: the states of stages 2 and 3 (ghosted layout)
-  double* k4;             // stages 4 and 5: L of stage 3 (interior layout), written by the first, read by the second
+  const double* k4;       // stage 5: L of stage 3 (interior layout)
 };
 
 // stage s > 1 of an R-stage scheme from the previous stage's residual (the coefficients of combine_value);
@@ -67,9 +68,6 @@ __device__ __forceinline__ void stage_node(double* x, const StagePost& sp, doubl
     for (int v = 0; v < 8; ++v) x[v] = add(mul(sp.ca, __ldg(sp.u0 + at + v * NN)), mul(sp.cb, add(u[v * NN], mul(dt, k[v]))));
   } else if (sp.stage < 5) {
     const double cdt = mul(sp.cc, dt);
-    if (sp.stage == 4)
-#pragma unroll
-      for (int v = 0; v < 8; ++v) sp.k4[ki + v * NN] = k[v];
 #pragma unroll
     for (int v = 0; v < 8; ++v)
       x[v] = add(add(mul(sp.ca, __ldg(sp.u0 + at + v * NN)), mul(sp.cb, u[v * NN])), mul(cdt, k[v]));
@@ -624,7 +622,7 @@ __device__ __forceinline__ bool residual_item(const double* __restrict__ u, cons
     for (int v = 0; v < 8; ++v) acc[v] = dfma(src, gp[v], acc[v]);
     acc[7] = dfma(0.0, un[7 * NN], acc[7]);
   }
-  if (MODE == RES_UT && act) {
+  if ((MODE == RES_UT || MODE == RES_POST54) && act) {
     double* o = to.ut + ((long long)(j0 + gr - 1) * nx + (i0 + gc - 1)) * EB + node;
 #pragma unroll
     for (int v = 0; v < 8; ++v) o[v * NN] = acc[v];
