@@ -303,13 +303,21 @@ void launch_bc(mhd_gpu* h, double* u, int gate) {
   launch_next(h->stream, grid1d(n, 256), 256, 0, bc_kernel<P>, u, h->geo, h->ctrl, gate);
 }
 
+// one CTA per TX x TY elements; rows of CTAs beyond a grid's 65,535 go on in z (the last layer may reach
+// beyond the mesh)
+template <int P>
+dim3 residual_grid(int nx, int ny) {
+  using L = Res2Layout<P>;
+  const int rows = (ny + L::TY - 1) / L::TY, layers = (rows + 65534) / 65535;
+  return dim3((nx + L::TX - 1) / L::TX, (rows + layers - 1) / layers, layers);
+}
+
 // ug: the array whose ghost ring the boundary halos come from (nullptr: u's own)
 template <int P>
 void launch_residual(mhd_gpu* h, const double* u, double* ut, int gate, int mode = RES_UT,
                      const StagePost& sp = StagePost{}, const double* ug = nullptr) {
   using L = Res2Layout<P>;
-  dim3 grid((h->nx + L::TX - 1) / L::TX, (h->ny + L::TY - 1) / L::TY);
-  launch_next(h->stream, grid, L::NT, L::BYTES, 
+  launch_next(h->stream, residual_grid<P>(h->nx, h->ny), L::NT, L::BYTES,
               mode == RES_POST54 ? residual2_kernel<P, RES_POST54> : mode == RES_POST ? residual2_kernel<P, RES_POST> : mode == RES_COMBINE ? residual2_kernel<P, RES_COMBINE> : residual2_kernel<P, RES_UT>,
               u, ug ? ug : u, ut, h->geo, h->ctrl, gate, sp);
 }
@@ -1227,17 +1235,17 @@ extern "C" int mhd_gpu_semidiscretize_noalloc(int p, int nx, int ny, double hx, 
   switch (p) {
     case 1: {
       using L = Res2Layout<1>;
-      residual2_kernel<1, RES_UT><<<dim3((nx + L::TX - 1) / L::TX, (ny + L::TY - 1) / L::TY), L::NT, L::BYTES, s>>>(u, u, ut, g, ctrl, GATE_ALWAYS, StagePost{});
+      residual2_kernel<1, RES_UT><<<residual_grid<1>(nx, ny), L::NT, L::BYTES, s>>>(u, u, ut, g, ctrl, GATE_ALWAYS, StagePost{});
       break;
     }
     case 2: {
       using L = Res2Layout<2>;
-      residual2_kernel<2, RES_UT><<<dim3((nx + L::TX - 1) / L::TX, (ny + L::TY - 1) / L::TY), L::NT, L::BYTES, s>>>(u, u, ut, g, ctrl, GATE_ALWAYS, StagePost{});
+      residual2_kernel<2, RES_UT><<<residual_grid<2>(nx, ny), L::NT, L::BYTES, s>>>(u, u, ut, g, ctrl, GATE_ALWAYS, StagePost{});
       break;
     }
     default: {
       using L = Res2Layout<3>;
-      residual2_kernel<3, RES_UT><<<dim3((nx + L::TX - 1) / L::TX, (ny + L::TY - 1) / L::TY), L::NT, L::BYTES, s>>>(u, u, ut, g, ctrl, GATE_ALWAYS, StagePost{});
+      residual2_kernel<3, RES_UT><<<residual_grid<3>(nx, ny), L::NT, L::BYTES, s>>>(u, u, ut, g, ctrl, GATE_ALWAYS, StagePost{});
       break;
     }
   }

@@ -681,7 +681,8 @@ __host__ __device__ inline int res2_item_cols(int nx) { return (nx + Res2Layout<
 template <int P>
 __host__ __device__ inline int res2_item_rows(int ny) { return (ny + Res2Layout<P>::EY - 1) / Res2Layout<P>::EY; }
 
-// single instance: one CTA per TX x TY block of elements (ug: the ghost-ring source, see residual_item)
+// single instance: one CTA per TX x TY block of elements, rows counted through y and z (residual_grid; ug: the
+// ghost-ring source, see residual_item)
 template <int P, int MODE>
 __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
     residual2_kernel(const double* __restrict__ u, const double* __restrict__ ug, double* __restrict__ ut, Geo g,
@@ -689,7 +690,7 @@ __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
   using L = Res2Layout<P>;
   extern __shared__ __align__(16) double sm[];
   const int warp = threadIdx.x >> 5;
-  const int ix = blockIdx.x * L::IX + warp % L::IX, iy = blockIdx.y * L::IY + warp / L::IX;
+  const int ix = blockIdx.x * L::IX + warp % L::IX, iy = (blockIdx.z * gridDim.y + blockIdx.y) * L::IY + warp / L::IX;
   double* wsm = sm + warp * L::WARP;
   res2_prologue<P>(wsm);
   grid_begin();
