@@ -242,8 +242,8 @@ __device__ __forceinline__ double2 ld2(const double* p) { return *reinterpret_ca
 // The next stage's element of this lane's group, from its combined node values x (ie, je: the element,
 // act: this lane holds one of its nodes, base: the group's first lane).  Where the element is the source of ghost
 // elements, those are formed first, as the boundary fill would from the values before the projection.
-// scratch: shared memory of the warp, free of use.  What a failing average leaves behind does not
-// matter: the try is abandoned then.
+// scratch: shared memory of the warp, free of use.  An element whose average is inadmissible keeps its combined
+// values, and its average and entropies of the stage before (the try is abandoned then).
 //
 // In place of a boundary fill and loop 1 as launches of their own for every stage after the first: the
 // state is neither written before the projection nor read again.  400^2, p = 3, one stage (us): residual
@@ -308,21 +308,22 @@ __device__ __forceinline__ void stage_post(const double* x, const StagePost& sp,
       }
     }
     const long long e = (long long)tj * (g.nx + 2) + ti;
-    if (mine) {
+    // admissibility of the average (DG_solver.f90:186-193)
+    const double pa = prs_of(avg[0], avg[1], avg[2], avg[3], avg[4], avg[5], avg[6], avg[7], g.gamma);
+    const bool ok = mine && !(avg[0] < PP_EPS || pa < PP_EPS);
+    if (mine && !ok && node == 0) atomicOr(&ctrl->neg_avg, 1);
+    if (ok) {
 #pragma unroll
       for (int v0 = 0; v0 < 8; v0 += NN)
         if (node + v0 < 8) sp.u_avg[e * 8 + node + v0] = row[node + v0];
     }
     __syncwarp();  // the row is rewritten next
-    // admissibility of the average (DG_solver.f90:186-193)
-    const double pa = prs_of(avg[0], avg[1], avg[2], avg[3], avg[4], avg[5], avg[6], avg[7], g.gamma);
-    if (mine && node == 0 && (avg[0] < PP_EPS || pa < PP_EPS)) atomicOr(&ctrl->neg_avg, 1);
     if (!ghost && sp.ent_offset) {  // cell entropies (DG_solver.f90:195-224)
       const double pq = act ? node_prs(y, g.gamma) : 0.0;
       const bool okq = !act || (y[0] >= PP_EPS && pq >= PP_EPS);
       const double okall = grp_min<NN>(okq ? 1.0 : 0.0);
       const double ce = grp_sum<NN>((act && okall > 0.5) ? 0.25 * g.hx * g.hy * dc.qw[k] * dc.qw[l] * ent_of(y[0], pq, g.gamma, g.igm1) : 0.0);
-      if (act && node == 0) {
+      if (ok && node == 0) {
         sp.cell_ent_FV[e] = ent_of(avg[0], pa, g.gamma, g.igm1);
         sp.cell_ent_DG[e] = okall > 0.5 ? ce : 0.0;
         sp.cell_ent_nan[e] = okall > 0.5 ? 0 : 1;
@@ -333,12 +334,14 @@ __device__ __forceinline__ void stage_post(const double* x, const StagePost& sp,
     if (sp.use_ldf) {
       double bx = y[4] - avg[4], by = y[5] - avg[5];
       ldf_project<P>(bx, by, base, node, nd, row, reinterpret_cast<const double2*>(g.ldfA));
-      y[4] = bx + avg[4];
-      y[5] = by + avg[5];
+      if (ok) {
+        y[4] = bx + avg[4];
+        y[5] = by + avg[5];
+      }
     }
     if (!sp.final) {
       bool neg = false;
-      limit_group<P, NN>(y, avg, act, node == 0, node, e, g, ctrl, sp.ent_offset, 0, sp.cell_ent_DG, sp.cell_ent_FV,
+      limit_group<P, NN>(y, avg, ok, node == 0, node, e, g, ctrl, sp.ent_offset, 0, sp.cell_ent_DG, sp.cell_ent_FV,
                          sp.cell_ent_nan, &neg);
       const unsigned cnt = __popc(__ballot_sync(FULL, neg));
       if (lane == 0 && cnt) atomicAdd(&ctrl->num_negcell, (int)cnt);
