@@ -137,11 +137,11 @@ __device__ __forceinline__ void combine_value(
 
 template <int EB>
 __global__ void __launch_bounds__(256)
-    combine_kernel(const double* __restrict__ u0, const double* __restrict__ r1, const double* __restrict__ r2,
-                   const double* __restrict__ r3, const double* __restrict__ r4,
-                   const double* __restrict__ k1, const double* __restrict__ k2, const double* __restrict__ k3,
-                   const double* __restrict__ k4, const double* __restrict__ k5, double* __restrict__ out,
-                   int nx, int ny, int R, int stage, const double* __restrict__ dt_ptr, double dt_arg,
+    combine_kernel(const double* u0, const double* r1, const double* r2,
+                   const double* r3, const double* r4,
+                   const double* k1, const double* k2, const double* k3,
+                   const double* k4, const double* k5, double* __restrict__ out,
+                   int nx, int ny, int R, int stage, const double* dt_ptr, double dt_arg,
                    const Ctrl* ctrl, int gate) {
   grid_begin();
   if (!gate_open(ctrl, gate)) return;

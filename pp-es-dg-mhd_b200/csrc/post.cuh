@@ -1022,7 +1022,7 @@ __device__ __forceinline__ void pp_sigsum_tile(const double* __restrict__ u, con
 
 template <int P>
 __global__ void __launch_bounds__(256, SigCfg<P>::MINB)
-    pp_sigsum_kernel(const double* __restrict__ u, Geo g, Ctrl* ctrl, int gate,
+    pp_sigsum_kernel(const double* u, Geo g, Ctrl* ctrl, int gate,
                      double* __restrict__ sig_x, double* __restrict__ sig_y) {
   grid_begin();
   if (!gate_open(ctrl, gate)) return;
@@ -1178,11 +1178,11 @@ __device__ __forceinline__ void pp_limit_segment(const LimitIO& io, const Geo& g
 
 template <int P>
 __global__ void __launch_bounds__(PPCfg<P>::NT, PPCfg<P>::MINB)
-    pp_limit_kernel(double* __restrict__ u, const double* __restrict__ u_avg, Geo g, Ctrl* ctrl,
-                    int gate, int apply_oedg, const double* __restrict__ dt_ptr, double oedg_dt_arg,
-                    int ent_offset, int comput_ent, const double* __restrict__ sig_x,
-                    const double* __restrict__ sig_y, const double* __restrict__ cell_ent_DG,
-                    const double* __restrict__ cell_ent_FV, const unsigned char* __restrict__ cell_ent_nan,
+    pp_limit_kernel(double* __restrict__ u, const double* u_avg, Geo g, Ctrl* ctrl,
+                    int gate, int apply_oedg, const double* dt_ptr, double oedg_dt_arg,
+                    int ent_offset, int comput_ent, const double* sig_x,
+                    const double* sig_y, const double* cell_ent_DG,
+                    const double* cell_ent_FV, const unsigned char* cell_ent_nan,
                     double* __restrict__ ent_partial, double* __restrict__ accept_dst, int accept_only) {
   grid_begin();
   __shared__ double s_ent[PPCfg<P>::TEL];
@@ -1262,7 +1262,7 @@ __device__ __forceinline__ void pp_entsum_body(const double* __restrict__ partia
 template <int P>
 __global__ void __launch_bounds__(256) stage_end_bc_kernel(const double* src, double* u, Geo g, Ctrl* ctrl, int R,
                                                           int stage, int next_stage,
-                                                          const double* __restrict__ ent_partial, int ent_nblk,
+                                                          const double* ent_partial, int ent_nblk,
                                                           LogEntry* log, int log_cap) {
   grid_begin();
   __shared__ int s_run, s_ent;
@@ -1286,7 +1286,7 @@ __global__ void __launch_bounds__(256) stage_end_bc_kernel(const double* src, do
   if (run) bc_value<P>(src, u, g, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-__global__ void __launch_bounds__(256) pp_entsum_kernel(const double* __restrict__ partial, int nblk,
+__global__ void __launch_bounds__(256) pp_entsum_kernel(const double* partial, int nblk,
                                                         Ctrl* ctrl, int gate) {
   grid_begin();
   if (!gate_open(ctrl, gate)) return;
@@ -1352,7 +1352,7 @@ __device__ __forceinline__ void neu_add(double& s, double& c, double x) {
 }
 
 template <int P>
-__global__ void __launch_bounds__(256) stage_diag_kernel(const double* __restrict__ u, Geo g, Ctrl* ctrl, int gate,
+__global__ void __launch_bounds__(256) stage_diag_kernel(const double* u, Geo g, Ctrl* ctrl, int gate,
                                                         double* __restrict__ part, unsigned int* ticket,
                                                         LogEntry* log, int log_cap) {
   grid_begin();

@@ -688,7 +688,7 @@ __host__ __device__ inline int res2_item_rows(int ny) { return (ny + Res2Layout<
 // ghost-ring source, see residual_item)
 template <int P, int MODE>
 __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
-    residual2_kernel(const double* __restrict__ u, const double* __restrict__ ug, double* __restrict__ ut, Geo g,
+    residual2_kernel(const double* u, const double* ug, double* __restrict__ ut, Geo g,
                      Ctrl* ctrl, int gate, StagePost sp) {
   using L = Res2Layout<P>;
   extern __shared__ __align__(16) double sm[];
@@ -707,7 +707,7 @@ __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
 // CTAs that return at once costs far less than one CTA per block.
 template <int P>
 __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
-    residual2_persistent(const double* __restrict__ u, double* __restrict__ ut, Geo g, Ctrl* ctrl, int gate,
+    residual2_persistent(const double* u, double* __restrict__ ut, Geo g, Ctrl* ctrl, int gate,
                          int ncol, int nitems) {
   grid_begin();
   using L = Res2Layout<P>;
