@@ -111,7 +111,8 @@ int mhd_gpu_gll_tables(int p, double *x, double *w, double *M, double *Minv, dou
  * element of degree p (DG_solver.f90:231-266 with LDF.f90:114-250), folded into one dense nodal
  * operator A of size (2n^2)x(2n^2), n = p+1, column-major:
  *     [Bx;By]_new - avg = A ([Bx;By] - avg),   node index k + n*l, Bx block first.
- * Host-only (no GPU needed); the kernels apply exactly this matrix.  p in 1..6. */
+ * Host-only (no GPU needed); p in 1..6.  The kernels (p <= 3) apply the same operator between the
+ * even and odd parts of the node values, which rounds differently. */
 int mhd_gpu_ldf_operator(int p, double hx, double hy, double *A);
 
 /* ---- state transfer (Fortran layouts) --------------------------------------------------- */
@@ -119,7 +120,10 @@ int mhd_gpu_ldf_operator(int p, double hx, double hy, double *A);
 /* slot 0 = u_con, slot s in 1..rknstg = uRK_con(:,:,:,:,:,s) (DG_solver.f90:12,14) */
 int mhd_gpu_upload_state(mhd_gpu_t *h, int slot, const double *u);
 int mhd_gpu_download_state(mhd_gpu_t *h, int slot, double *u);
-/* ut_con(:,:,:,:,:,stage), stage in 1..rknstg (DG_solver.f90:13) */
+/* ut_con(:,:,:,:,:,stage), stage in 1..rknstg (DG_solver.f90:13).  mhd_gpu_semidiscretize writes the
+ * one it is given.  A run (mhd_gpu_advance, batches, the server) writes ut(1), the derivative of the accepted
+ * state, and with SSP-RK(5,4) the derivatives ut(2..5) of its stages; with SSP-RK(2,2) and (3,3) those go
+ * into the next stage without being stored, and ut(2..) keep what they held. */
 int mhd_gpu_upload_ut(mhd_gpu_t *h, int stage, const double *ut);
 int mhd_gpu_download_ut(mhd_gpu_t *h, int stage, double *ut);
 /* u_avg (DG_solver.f90:11), the input of save_tecbin_finite_volume (io.f90:4) */
@@ -357,8 +361,8 @@ int mhd_server_destroy(mhd_server_t *s);
  * The call allocates nothing: its only scratch (the dt_lim reduction cell and status words) is a
  * 4 KiB static device array inside the library, which every GPU that loads the library holds
  * until the process exits.  All calls share that array and it keeps the last call's contents;
- * the reduction cell is reset at the start of every call, and calls that overlap on the GPU
- * (different streams or host threads at the same time) race on it.
+ * the reduction cell is reset at the start of every call that asks for dt_lim, and calls that overlap
+ * on the GPU (different streams or host threads at the same time) race on it.
  * The first call on a device sets that device up (constant tables, kernel attributes and the
  * address of the static array); make that first call before any stream capture.  That set-up is
  * kept for the life of the process, like every handle's device set-up: the library must not be

@@ -2,7 +2,7 @@
 //
 // A batch holds existing handles (each already through mhd_gpu_solve_begin).  Members are grouped
 // by (degree p, RK stages R).  Per group the batch keeps a device table of InstDesc entries and one
-// flattened work list per kernel kind: residual tiles, average/LDF chunks, OEDG indicator item
+// flattened work list per kernel kind: residual items, average/LDF chunks, OEDG indicator item
 // blocks, limiter row segments and ghost blocks, each entry (instance, a, b).
 // One SSP-RK try of every member is one CUDA graph: per group the batched kernels of the try
 // sequence (the same kernel bodies as the single-instance path, so each member's arithmetic is

@@ -538,7 +538,8 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
   // logarithms and roots of each density do in the reference (the product of two negative ones is positive:
   // it takes the left one's sign).
   const double rho_p = dmul(wl[0], wr[0]);
-  const double s_rho = sqrt_nr(__hiloint2double(__double2hiint(rho_p) | (__double2hiint(wl[0]) & (int)0x80000000), __double2loint(rho_p)));
+  const int sign_l = __double2hiint(wl[0]) & (int)0x80000000;
+  const double s_rho = sqrt_nr(__hiloint2double(__double2hiint(rho_p) | sign_l, __double2loint(rho_p)));
   const double irs = rcp_nr(dfma(2.0, s_rho, rho_s));
   const double vx_roe = dmul(dfma(s_rho, dadd(v[0][0], v[1][0]), dadd(wl[1], wr[1])), irs);
   const double db = sqrt_nr(dfma(dsq3(j[4], j[5], j[6]), irs, TINY));

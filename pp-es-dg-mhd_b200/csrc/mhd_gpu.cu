@@ -317,9 +317,12 @@ template <int P>
 void launch_residual(mhd_gpu* h, const double* u, double* ut, int gate, int mode = RES_UT,
                      const StagePost& sp = StagePost{}, const double* ug = nullptr) {
   using L = Res2Layout<P>;
-  launch_next(h->stream, residual_grid<P>(h->nx, h->ny), L::NT, L::BYTES,
-              mode == RES_POST54 ? residual2_kernel<P, RES_POST54> : mode == RES_POST ? residual2_kernel<P, RES_POST> : mode == RES_COMBINE ? residual2_kernel<P, RES_COMBINE> : residual2_kernel<P, RES_UT>,
-              u, ug ? ug : u, ut, h->geo, h->ctrl, gate, sp);
+  const auto kernel = mode == RES_POST54    ? residual2_kernel<P, RES_POST54>
+                      : mode == RES_POST    ? residual2_kernel<P, RES_POST>
+                      : mode == RES_COMBINE ? residual2_kernel<P, RES_COMBINE>
+                                            : residual2_kernel<P, RES_UT>;
+  launch_next(h->stream, residual_grid<P>(h->nx, h->ny), L::NT, L::BYTES, kernel, u, ug ? ug : u, ut, h->geo, h->ctrl,
+              gate, sp);
 }
 
 // the re-try residual of a try (gate ST_RECOMPUTE, usually closed): a persistent grid of the CTAs
@@ -356,7 +359,6 @@ void launch_combine(mhd_gpu* h, int stage, const double* dt_ptr, double dt, int 
 }
 
 // post_process on slot `slot` (everything but the control-block reset and the host read-back)
-template <int P>
 // fuse = 1 (time-step pipeline only): a stage without OEDG, entropy or acceptance copy runs loops
 // 1 and 3 in one kernel (the stage result is discarded if an average is inadmissible)
 // s1 (time-step pipeline, stage 1 only): loop 1 forms the stage state from u0 and the stage-1
@@ -366,13 +368,15 @@ template <int P>
 // interior as loop 1 left it
 // loop1_done (time-step pipeline): the previous residual did loop 1 of this stage (StagePost), and loop 3
 // where it is fused
+template <int P>
 void launch_post(mhd_gpu* h, int slot, int apply_oedg, int apply_ldf, const double* dt_ptr, double oedg_dt,
                  int ent_offset, int comput_ent, double* accept_dst, int gate, int fuse = 0,
                  Stage1Src s1 = Stage1Src{}, bool entsum_later = false, int accept_only = 0, bool loop1_done = false) {
   const int limit_in_loop1 = fuse && !apply_oedg && !comput_ent && !accept_dst;
   if (!loop1_done) {
     const int nb1 = pp_nblk_avg<P>(h);
-    const int grid1 = std::min(nb1, limit_in_loop1 ? pp_resident_ctas<P, true>(h->device) : pp_resident_ctas<P, false>(h->device));
+    const int grid1 = std::min(nb1, limit_in_loop1 ? pp_resident_ctas<P, true>(h->device)
+                                                   : pp_resident_ctas<P, false>(h->device));
     launch_next(h->stream, grid1, PPCfg<P>::NT, 0, limit_in_loop1 ? pp_avg_ldf_kernel<P, true> : pp_avg_ldf_kernel<P, false>,
                 h->u[slot], h->u_avg, h->geo, h->ctrl, gate, apply_ldf, ent_offset, h->cell_ent_DG, h->cell_ent_FV,
                 h->cell_ent_nan, nb1, s1);
@@ -494,8 +498,9 @@ StagePost next_stage_post(const mhd_gpu* h, int stage) {
 // before it, as launches of its own.  Folded a step is faster at every size.  Orszag-Tang, SSP-RK(3,3), launches ->
 // folded (us a step): p = 1, 16^2 65 -> 59, 128^2 89 -> 81, 512^2 500 -> 484; p = 2, 64^2 80 -> 75, 300^2 427 -> 409;
 // p = 3, 100^2 123 -> 117, 180^2 243 -> 243; vortex 512^2 p = 3 1607 -> 1539; SSP-RK(5,4), whose combination
-// was a launch too: p = 1, 64^2 110 -> 92; p = 2, 203x190 377 -> 311, 400^2 1306 -> 1053.  Below 1024 nodes, where
-// it is 2-4 us, a try keeps one launch per procedure, the sequence that step_graph_kernels is known by.
+// was a launch too: p = 1, 64^2 110 -> 88; p = 2, 203x190 377 -> 318, 400^2 1306 -> 1065.
+// States below 1024 nodes keep the launches, 2-4 us slower, for one reason only: the number of kernels in their
+// try (step_graph_kernels: 18 at SSP-RK(3,3) with OEDG) is part of what callers and tests know.
 bool fold_post(const mhd_gpu* h) { return (long long)h->nx * h->ny * h->nn >= 1024; }
 
 // one try of a time step (drive.f90:93-300), recorded into the capturing stream

@@ -94,8 +94,8 @@ __device__ __forceinline__ void stage_node(double* x, const StagePost& sp, doubl
 //   2. the nodes' primitives, to a record per node in shared memory;
 //   3. the entropy-conservative flux of every node pair of a line, computed once, by one of the
 //      pair's two lanes, from the partner's record; the other lane receives the flux by a shuffle
-//      (the shared-memory pipe carries a shuffled value once, a stored and loaded one twice).  Rounds per degree (k along x, l along y; every round gives each lane exactly
-//      one flux to compute):
+//      (the shared-memory pipe carries a shuffled value once, a stored and loaded one twice).  Rounds per
+//      degree (k along x, l along y; every round gives each lane exactly one flux to compute):
 //        p = 1  one round: lanes with k == l take their x pair, the others their y pair
 //        p = 2  a ring along x (partner k+1 mod 3, received from k+2 mod 3), then the same along y:
 //               the three pairs of a line are the ring's three edges
@@ -449,7 +449,7 @@ __device__ __forceinline__ bool residual_item(const double* __restrict__ u, cons
   const double* un = wsm + ((act ? gr : 0) * SX + (act ? gc : 0) + 1) * ES + node;  // the node's staged state
   const double sxh = g.sxh, syh = g.syh;
   const double sxq = 0.5 * sxh, syq = 0.5 * syh;  // 2 (2/h) / 4: the pair fluxes come as four times the flux
-  // (all arithmetic of the item is exactly rounded as written: dmul/dadd/dsub/dfma of common.cuh, so
+  // (all arithmetic of L(u) is exactly rounded as written: dmul/dadd/dsub/dfma of common.cuh, so
   // that each kernel it is inlined into rounds it the same way: a batch member equals its solo run)
   double sgx, sgy, bsq, pp[8];  // bounds of the wave speeds, |B|^2; pp: (rho, vx, vy, vz, Bx, By, Bz, beta), the EC flux's inputs
   {
@@ -724,9 +724,11 @@ __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
 
 // many instances of degree P: each warp of a persistent grid walks its share of every member's items
 // (row-major per member); the state is slot `src`, the result goes to ut[dst], or stage
-// dst to slot dst (RES_POST).  The item's arithmetic is fully
-// rounded as written (explicit fused multiply-adds, see common.cuh), so a member is bitwise equal to
-// its solo run although this is a different kernel.
+// dst to slot dst (RES_POST).  L(u) and the combination are fully rounded as written (explicit fused
+// multiply-adds, see common.cuh), so a member is bitwise equal to its solo run although this is a different
+// kernel.  Loops 1 and 3 of the stage formed (stage_post) are not: there the equality with the solo kernels and
+// with the launches of their own rests on the compiler contracting the same inlined code alike, and on
+// tests/test_gpu_folded_stages.py and test_gpu_folded_solo.py, which compare the three.
 template <int P, int MODE>
 __global__ void __launch_bounds__(Res2Layout<P>::NT, Res2Layout<P>::MINB)
     residual2_batched(const InstDesc* __restrict__ insts, const int* __restrict__ pref,

@@ -19,9 +19,10 @@ int dpow_rows(int p, double* R0, double* RN);
 // A is (2n^2)x(2n^2) column-major, node index k + n*l, Bx block first.
 int ldf_nodal_operator(int p, double hx, double hy, double* A);
 
-// The same operator as the kernels apply it (p <= 3), between the node values' even and odd parts.  With the GLL nodes symmetric, replace f_k, f_{p-k} by their sum (at k < p-k) and difference (at
-// p-k), in both directions: the operator then couples Bx only with Bx of the same parity in x and y and
-// with By of the opposite parity in both (a reflection maps divergence-free fields to such fields), so
+// The same operator as the kernels apply it (p <= 3), between the node values' even and odd parts.  With the
+// GLL nodes symmetric, replace f_k, f_{p-k} by their sum (at k < p-k) and difference (at p-k), in both
+// directions: the operator then couples Bx only with Bx of the same parity in x and y and with By of the
+// opposite parity in both (a reflection maps divergence-free fields to such fields), so
 // a node needs at most M^2 + M^2 inputs, M = (p+2)/2, instead of 2 (p+1)^2.
 // out[2 (s n^2 + q) + c], q = k + n l: the weight of output c (0: Bx, 1: By) of node q for input slot
 // s < 2 M^2.  Slots s = jx + M jy < M^2 are the same field at node (jx or p - jx, jy or p - jy), the
