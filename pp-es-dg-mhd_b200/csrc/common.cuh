@@ -503,7 +503,6 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
     const double disc = at_least(dfma(ss, ss, -dmul(dmul(dmul(4.0, cs), ir[h]), bn2)), TINY);
     cf[h] = sqrt_nr(dmul(0.5, dadd(ss, sqrt_nr(disc))));
     f[h][0] = w[1];
-    f[h][1] = dfma(v[h][0], w[1], -bn2);  // the pressures follow below
     f[h][2] = dfma(v[h][0], w[2], -dmul(w[5], w[4]));
     f[h][3] = dfma(v[h][0], w[3], -dmul(w[6], w[4]));
     f[h][4] = 0.0;
@@ -513,7 +512,10 @@ __device__ __forceinline__ void espp_hll(const double* wl, const double* wr, dou
   }
   const double pb = at_most(prs[0], prs[1]);
 #pragma unroll
-  for (int h = 0; h < 2; ++h) f[h][1] = dadd(f[h][1], dfma(0.5, bsq[h], dsub(prs[h], pb)));
+  for (int h = 0; h < 2; ++h) {  // rounded as ec_flux4 rounds its p_tot - B_n^2, so that the two cancel where the field is constant
+    const double* w = h ? wr : wl;
+    f[h][1] = dfma(v[h][0], w[1], dfma(-w[4], w[4], dfma(0.5, bsq[h], dsub(prs[h], pb))));
+  }
   const double rho_s = dadd(wl[0], wr[0]);
   double ds;
   {

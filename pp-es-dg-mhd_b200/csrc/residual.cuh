@@ -578,9 +578,9 @@ __device__ __forceinline__ bool residual_item(const double* __restrict__ u, cons
     // local div B (DG_solver.f90:813)
     double dbx = 0.0, dby = 0.0;
 #pragma unroll
-    for (int r = 0; r < N; ++r) {
-      dbx = dfma(Dk(r), r == 0 ? pp[4] : __shfl_sync(FULL, pp[4], along_x(r)), dbx);
-      dby = dfma(Dl(r), r == 0 ? pp[5] : __shfl_sync(FULL, pp[5], along_y(r)), dby);
+    for (int r = 1; r < N; ++r) {  // the rows of D sum to zero: of differences, so that a constant field has none
+      dbx = dfma(Dk(r), dsub(__shfl_sync(FULL, pp[4], along_x(r)), pp[4]), dbx);
+      dby = dfma(Dl(r), dsub(__shfl_sync(FULL, pp[5], along_y(r)), pp[5]), dby);
     }
     // (2/h)/w times the interface flux, + at the first node of a line and - at the last; `src`
     // collects the factor of the Godunov-Powell vector (0, B, v, v.B) (DG_solver.f90:794-799)
